@@ -42,12 +42,13 @@ extern "C" {
 #define KWG_STATUS_DEVICE_TIMEOUT 4 /* price is NaN; a bounded device-side wait expired */
 
 /* ---- numeric modes ------------------------------------------------------------------- */
-#define KWG_FP64 0 /* all stepping in FP64: parity with the reference to <= 1e-10 relative */
+#define KWG_FP64 0 /* FP64 results: parity with the reference to <= 1e-10 relative (stepping in
+                      FP64, or on chip in pairs of FP32 with refined solves) */
 #define KWG_FP32 1 /* FP32 stepping: FP64 setup and interpolation, float-float state and residual */
 
 #define KWG_SOLVER_AUTO 0   /* the autotuned choice for this shape, else a cost model */
 #define KWG_SOLVER_THOMAS 1 /* FP64: thread per option, option-interleaved streaming layout */
-#define KWG_SOLVER_PCR 2    /* warp per option, partitioned solve with warp-shuffle cyclic
+#define KWG_SOLVER_PCR 2    /* on chip, one to four warps per option, partitioned solve with warp-shuffle cyclic
                                reduction, state on chip (FP64: x_dim <= 1024; FP32: <= 2048) */
 
 /* Same field order, types and 56-byte layout as kw::Option (src/Core/kwAsset.h:12-22). */
@@ -73,7 +74,11 @@ typedef struct kwg_fd1d_params {
     double density;    /* FD1D.DENSITY, default 0.25; +INFINITY = uniform grid (the
                           density -> infinity limit of the sinh grid)        */
     int32_t precision; /* KWG_FP64 (default) or KWG_FP32 */
-    int32_t solver;    /* KWG_SOLVER_AUTO (default), _THOMAS or _PCR */
+    int32_t solver;    /* KWG_SOLVER_AUTO (default); _THOMAS: the FP64 streaming solver, one
+                          thread per PDE; _PCR: the on-chip solver, one to four warps per
+                          PDE, x_dim <= 1024.  AUTO takes the on-chip one at theta = 1/2 up
+                          to x_dim 2048 (except many PDEs of 56 nodes or fewer) unless
+                          the autotuner recorded another choice */
     int32_t strict;    /* blocking host calls (kwg_fd1d_price, kwg_fd1d_bs_price,
                           kwg_fd1d_price_uneven): 1 returns an error for the first
                           bad option, like the reference
@@ -189,12 +194,14 @@ int kwg_fd1d_price_uneven(kwg_ctx* ctx, const kwg_option* opts, const int32_t* x
 /* Result of the autotuner: the launch shape it picked and the solve-kernel time of
  * every candidate (-1: not timed or not applicable). */
 typedef struct kwg_tuning {
-    int32_t solver;       /* KWG_SOLVER_THOMAS or KWG_SOLVER_PCR (FP64); KWG_SOLVER_PCR (FP32) */
+    int32_t solver;       /* KWG_SOLVER_THOMAS or KWG_SOLVER_PCR (FP64); KWG_SOLVER_PCR (FP32);
+                             KWG_SOLVER_AUTO: the on-chip FP64 solver on a grid of 1025 to
+                             2048 nodes, which only AUTO selects there */
     int32_t block_warps;  /* warps (32 options each) per block of the streaming FP64 solver */
     int32_t option_warps; /* warps (32 threads each) per option of the FP32 solver */
     int32_t sm_blocks;    /* resident blocks per SM of the streaming FP64 solver (0: as many as fit) */
     double thomas_ms[3];  /* streaming FP64 solver with 1, 2, 4 warps per block */
-    double pcr_ms;        /* FP64 warp-per-PDE solver */
+    double pcr_ms;        /* FP64 on-chip solver (KWG_SOLVER_PCR) */
     double fp32_ms[3];    /* FP32 solver with 1, 2, 4 warps per option (the launch may
                              use fewer: at least 2 nodes per lane, and at least 2 warps
                              for grids of more than 1024 nodes) */

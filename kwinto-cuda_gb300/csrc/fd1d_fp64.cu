@@ -924,6 +924,7 @@ void fd1d_prepare_kernels(int device)
     }
     fd1d_fp32_prepare(device);
     fd1d_pcr64_prepare(device);
+    fd1d_pair64_prepare(device);
     if (prev >= 0 && prev != device) cudaSetDevice(prev);
     g_ready[device].store(true, std::memory_order_release);
 }

@@ -107,9 +107,19 @@ int fd1d_fp32_launch(const PdeBatch& b, const AssetBatch& a, const Fd1dShape& sh
 
 // FP64 warp-per-PDE on-chip solve (x_dim <= 1024).  Same work buffer as FP32.
 int fd1d_pcr64_nodes_per_lane(int x_dim);
+int fd1d_pcr64_rescue(const PdeBatch& b, const Fd1dShape& sh, double* vout, const int32_t* list, int32_t* pde_status,
+                      int* counters, int sms, cudaStream_t stream);
 int fd1d_pcr64_launch(const PdeBatch& b, const AssetBatch& a, const Fd1dShape& sh, double* vout, int32_t* pde_status,
                       int* counters, double* prices, int32_t* status, int device, cudaStream_t stream,
                       const SolveEvents* ev);
+
+// FP64 accuracy on the FP32 units (fd1d_pair64.cu): theta = 1/2, x_dim <= 2048, one to
+// eight warps per PDE.  The work buffer holds the final V of every PDE and the list of the
+// PDEs left to the FP64 kernel (`rescue`, m ints); -1 for shapes it does not take.
+size_t fd1d_pair64_work_bytes(int m, long long nodes);
+int fd1d_pair64_launch(const PdeBatch& b, const AssetBatch& a, const Fd1dShape& sh, double* vout, int32_t* rescue,
+                       int32_t* pde_status, int* counters, double* prices, int32_t* status, int device,
+                       cudaStream_t stream, const SolveEvents* ev);
 
 // Device options (56-byte kw::Option records) -> the SoA arrays of a PdeBatch and
 // an AssetBatch, every option its own PDE, the PDEs grouped by exercise / put-call
@@ -133,6 +143,7 @@ __global__ void fd1d_interp_rows(const PdeBatch b, const AssetBatch a, Fd1dShape
 void fd1d_prepare_kernels(int device);
 void fd1d_fp32_prepare(int device);
 void fd1d_pcr64_prepare(int device);
+void fd1d_pair64_prepare(int device);
 
 // Occupancy-derived persistent grid size (blocks of block_warps warps) for the FP64
 // solve kernel.

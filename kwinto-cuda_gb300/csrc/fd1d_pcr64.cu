@@ -3,8 +3,8 @@
 // Same step as the streaming kernel (fd1d_fp64.cu):  y = T^-1 V (T = theta B),
 // V' = max(y - cV, p) on nodes < N-1 (src/Math/kwFd1d.cpp:61-132), but the 32 lanes
 // of a warp share one PDE, so a batch of m options keeps m warps busy instead of
-// m/32.  This is the variant for small batches, where the thread-per-option kernel
-// cannot fill the GPU; the autotuner picks between them.
+// m/32.  It serves theta != 1/2 on small batches, where the thread-per-option kernel cannot
+// fill the GPU, and the PDEs that the solver on FP32 units (fd1d_pair64.cu) leaves over.
 //
 // Solve of T y = V (N_p = 32 M nodes, lane k owns nodes kM .. kM+M-1; the grid is
 // padded to N_p with decoupled identity rows):
@@ -14,6 +14,8 @@
 //   * separators: a 32-unknown tridiagonal system, parallel cyclic reduction over
 //     the warp (5 shuffle levels).
 // Factors, spikes and the reduction multipliers are computed once per PDE in FP64.
+// With a list (rescue launches) it takes the listed PDEs only: those whose values the
+// FP32-pair solver cannot hold (fd1d_pair64.cu).
 // Per node and step: 6 FP64 operations (forward, backward, two spike terms, scale,
 // update); the reduced system adds ~15 per lane.
 #include <cstdint>
@@ -48,7 +50,7 @@ constexpr size_t pcr64_smem()
 template <int M, bool kHalf, bool kShared>
 __global__ void __launch_bounds__(32) fd1d_solve_fp64_pcr(const PdeBatch b, Fd1dShape sh, double* __restrict__ vout,
                                                           int32_t* __restrict__ pde_status,
-                                                          int* __restrict__ counters)
+                                                          int* __restrict__ counters, const int32_t* __restrict__ list)
 {
     extern __shared__ double qtab[];  // [M][kP64Fields][32], or (kShared) [M][32] + [M][5][2]
     const int k = threadIdx.x & 31;
@@ -68,9 +70,10 @@ __global__ void __launch_bounds__(32) fd1d_solve_fp64_pcr(const PdeBatch b, Fd1d
 
     for (;;) {
         int pde = 0;
-        if (k == 0) pde = atomicAdd(&counters[0], 1);
+        if (k == 0) pde = atomicAdd(&counters[list ? 3 : 0], 1);
         pde = __shfl_sync(kFull64, pde, 0);
-        if (pde >= b.m) break;
+        if (pde >= (list ? counters[2] : b.m)) break;
+        if (list) pde = list[pde];
         const int N = shape_x(sh, pde);
         const int T = shape_t(sh, pde);
 
@@ -271,32 +274,31 @@ __global__ void __launch_bounds__(32) fd1d_solve_fp64_pcr(const PdeBatch b, Fd1d
 
 namespace {
 
-// Resident blocks per SM of fd1d_solve_fp64_pcr<M, *, kShared>, set by fd1d_pcr64_prepare.
-template <int M, bool kShared>
+// Resident blocks per SM of fd1d_solve_fp64_pcr<M, kHalf, kShared>, set by fd1d_pcr64_prepare.
+template <int M, bool kHalf, bool kShared>
 int& per_sm_pcr64()
 {
     static int v = 1;
     return v;
 }
 
-template <int M, bool kShared>
+template <int M, bool kHalf, bool kShared>
 void prepare_pcr64_variant()
 {
     const size_t smem = pcr64_smem<M, kShared>();
-    cudaFuncSetAttribute(fd1d_solve_fp64_pcr<M, true, kShared>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                         (int)smem);
-    cudaFuncSetAttribute(fd1d_solve_fp64_pcr<M, false, kShared>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                         (int)smem);
+    auto kern = fd1d_solve_fp64_pcr<M, kHalf, kShared>;
+    cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     int per_sm = 0;
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fd1d_solve_fp64_pcr<M, true, kShared>, 32, smem);
-    per_sm_pcr64<M, kShared>() = per_sm < 1 ? 1 : per_sm;
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, 32, smem);
+    per_sm_pcr64<M, kHalf, kShared>() = per_sm < 1 ? 1 : per_sm;
 }
 
 template <int M>
 void prepare_pcr64()
 {
-    prepare_pcr64_variant<M, false>();
-    prepare_pcr64_variant<M, true>();
+    prepare_pcr64_variant<M, false, false>();
+    prepare_pcr64_variant<M, false, true>();
+    prepare_pcr64_variant<M, true, false>();  // theta = 1/2: listed PDEs only
 }
 
 template <int M, bool kShared>
@@ -305,12 +307,12 @@ int launch_pcr64_variant(const PdeBatch& b, const AssetBatch& a, const Fd1dShape
                          cudaStream_t stream, const SolveEvents* ev)
 {
     const size_t smem = pcr64_smem<M, kShared>();
-    auto kern = sh.c == 1. ? fd1d_solve_fp64_pcr<M, true, kShared> : fd1d_solve_fp64_pcr<M, false, kShared>;
-    const int per_sm = per_sm_pcr64<M, kShared>();
+    auto kern = fd1d_solve_fp64_pcr<M, false, kShared>;  // theta = 1/2 goes to fd1d_pair64.cu
+    const int per_sm = per_sm_pcr64<M, false, kShared>();
     const int blocks = b.m < sms * per_sm ? b.m : sms * per_sm;
     cudaMemsetAsync(counters, 0, 4 * sizeof(int), stream);
     if (ev) cudaEventRecord(ev->start, stream);
-    kern<<<blocks, 32, smem, stream>>>(b, sh, vout, pde_status, counters);
+    kern<<<blocks, 32, smem, stream>>>(b, sh, vout, pde_status, counters, nullptr);
     if (ev) cudaEventRecord(ev->stop, stream);
     int launches = 1;
     if (a.n > 0) {
@@ -331,10 +333,20 @@ int launch_pcr64(const PdeBatch& b, const AssetBatch& a, const Fd1dShape& sh, do
     return launch_pcr64_variant<M, false>(b, a, sh, vout, pde_status, counters, prices, status, sms, stream, ev);
 }
 
+template <int M>
+void launch_rescue(const PdeBatch& b, const Fd1dShape& sh, double* vout, const int32_t* list, int32_t* pde_status,
+                   int* counters, int sms, cudaStream_t stream)
+{
+    const int cap = sms * per_sm_pcr64<M, true, false>();
+    fd1d_solve_fp64_pcr<M, true, false><<<b.m < cap ? b.m : cap, 32, pcr64_smem<M, false>(), stream>>>(
+        b, sh, vout, pde_status, counters, list);
+}
+
 }  // namespace
 
 void fd1d_pcr64_prepare(int)
 {
+    prepare_pcr64_variant<64, true, false>();
     prepare_pcr64<2>();
     prepare_pcr64<4>();
     prepare_pcr64<8>();
@@ -347,6 +359,22 @@ int fd1d_pcr64_nodes_per_lane(int x_dim)
     int m = 2;
     while (32 * m < x_dim) m *= 2;
     return m <= 32 ? m : -1;
+}
+
+// The PDEs that fd1d_solve_pair64 left on its list (counters[2] of them, queue
+// counters[3]); up to 2048 nodes.
+int fd1d_pcr64_rescue(const PdeBatch& b, const Fd1dShape& sh, double* vout, const int32_t* list, int32_t* pde_status,
+                      int* counters, int sms, cudaStream_t stream)
+{
+    switch (fd1d_fp32_nodes_per_lane(sh.x_dim)) {
+    case 2: launch_rescue<2>(b, sh, vout, list, pde_status, counters, sms, stream); break;
+    case 4: launch_rescue<4>(b, sh, vout, list, pde_status, counters, sms, stream); break;
+    case 8: launch_rescue<8>(b, sh, vout, list, pde_status, counters, sms, stream); break;
+    case 16: launch_rescue<16>(b, sh, vout, list, pde_status, counters, sms, stream); break;
+    case 32: launch_rescue<32>(b, sh, vout, list, pde_status, counters, sms, stream); break;
+    default: launch_rescue<64>(b, sh, vout, list, pde_status, counters, sms, stream); break;
+    }
+    return 1;
 }
 
 int fd1d_pcr64_launch(const PdeBatch& b, const AssetBatch& a, const Fd1dShape& sh, double* vout, int32_t* pde_status,

@@ -239,19 +239,29 @@ __global__ void selftest_waits(int32_t* __restrict__ out, uint32_t limit)
 
 
 // Launch choices for a batch of m PDEs: the explicit ones in p, else what the
-// autotuner recorded for the shape, else defaults.  FP64 solver default: a cost
-// model -- the thread-per-option kernel runs m/32 warps, the warp-per-option kernel
-// m warps at twice the FP64 work per node-step, so the latter wins while m/32 warps
-// cannot fill the GPU (a few warps per SM).
+// autotuner recorded for the shape, else defaults.  FP64 solver default: the on-chip
+// solver on FP32 units where it takes the shape (theta = 1/2, up to 2048 nodes), except
+// for many PDEs on small grids: it spends the same time on 3 to 64 nodes (one warp's
+// separator solve), the streaming solver 6 FP64 cycles per node once its lanes are full.
+// Measured, 131072 PDEs, 200 steps, uniform: 16/32/48/64 nodes streaming 2.5/4.7/7.0/9.4 ms,
+// on chip 8.4/8.4/8.4/8.1 ms; a lone streaming warp takes ~290 cycles per node, so below
+// ~430 PDEs per node the on-chip solver is ahead again.  Other schemes: a cost model -- the
+// thread-per-option kernel runs m/32 warps, the warp-per-option FP64 kernel m warps at twice
+// the FP64 work per node-step, so the latter wins while m/32 warps cannot fill the GPU.
 kwg_ctx::Tuned choose(kwg_ctx* ctx, const kwg_fd1d_params* p, int m)
 {
     kwg_ctx::Tuned t;
     auto it = ctx->tuned.find(tune_key(p->precision, p->x_dim, p->t_dim, m));
+    const bool pcr_ok = kwg::fd1d_pcr64_nodes_per_lane(p->x_dim) > 0;
     if (it != ctx->tuned.end()) {
         t = it->second;
+        // recorded for theta = 1/2, which the key does not hold
+        if (p->precision == KWG_FP64 && t.solver == KWG_SOLVER_PCR && !pair64_ok(p) && !pcr_ok)
+            t.solver = KWG_SOLVER_THOMAS;
     } else {
-        const bool pcr_ok = kwg::fd1d_pcr64_nodes_per_lane(p->x_dim) > 0;
-        t.solver = (pcr_ok && m < 8192) ? KWG_SOLVER_PCR : KWG_SOLVER_THOMAS;
+        const bool many_small = p->x_dim <= 56 && m > 430 * p->x_dim;
+        const bool on_chip = pair64_ok(p) ? !many_small : pcr_ok && m < 8192;
+        t.solver = on_chip ? KWG_SOLVER_PCR : KWG_SOLVER_THOMAS;
     }
     if (p->precision == KWG_FP32) t.solver = KWG_SOLVER_PCR;
     else if (p->solver != KWG_SOLVER_AUTO) t.solver = p->solver;
@@ -290,7 +300,16 @@ int run_batch(kwg_ctx* ctx, char* io, const IoLayout& L, int m, int n, const kwg
     sh.block_warps = tn.block_warps;
     sh.option_warps = tn.option_warps;
     sh.sm_blocks = tn.sm_blocks;
-    if (p->precision == KWG_FP64 && solver == KWG_SOLVER_PCR) {
+    if (solver == KWG_SOLVER_PCR && pair64_ok(p)) {
+        const long long nodes = (long long)m * sh.x_dim;
+        if (int rc = ensure_device(ctx, &ctx->d_work, &ctx->work_bytes, kwg::fd1d_pair64_work_bytes(m, nodes))) return rc;
+        double* v = (double*)ctx->d_work;
+        const int n_launch = kwg::fd1d_pair64_launch(b, a, sh, v, (int32_t*)(v + nodes), (int32_t*)(io + L.pde_status),
+                                                     ctx->d_counter, prices, status, ctx->device, stream,
+                                                     ctx->next_events());
+        if (n_launch < 0) return set_err(ctx, KWG_ERR_INVALID, "kwg: the on-chip FP64 solver supports x_dim <= 2048");
+        ctx->launches += n_launch;
+    } else if (p->precision == KWG_FP64 && solver == KWG_SOLVER_PCR) {
         const size_t wbytes = kwg::fd1d_fp32_work_bytes(m, sh.x_dim);
         if (int rc = ensure_device(ctx, &ctx->d_work, &ctx->work_bytes, wbytes)) return rc;
         const int n_launch = kwg::fd1d_pcr64_launch(b, a, sh, (double*)ctx->d_work, (int32_t*)(io + L.pde_status),
@@ -660,10 +679,12 @@ int kwg_autotune_ex(kwg_ctx* ctx, const kwg_fd1d_params* p, size_t m, kwg_tuning
     const std::vector<kwg_option> opts = tuning_batch(m);
     std::vector<double> prices(m);
     const bool pcr_ok = kwg::fd1d_pcr64_nodes_per_lane(p->x_dim) > 0;
-    const kwg_ctx::Tuned best = tune(ctx, p, pcr_ok, [&](const kwg_fd1d_params& q) {
+    const uint64_t key = tune_key(p->precision, p->x_dim, p->t_dim, (int)m);
+    ctx->tuned.erase(key);
+    const kwg_ctx::Tuned best = tune(ctx, p, pcr_ok, pair64_ok(p), [&](const kwg_fd1d_params& q) {
         return kwg_fd1d_price(ctx, opts.data(), m, &q, prices.data(), nullptr);
     }, out);
-    ctx->tuned[tune_key(p->precision, p->x_dim, p->t_dim, (int)m)] = best;
+    ctx->tuned[key] = best;
     ctx->err.clear();
     return KWG_OK;
 }

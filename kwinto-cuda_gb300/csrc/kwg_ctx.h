@@ -139,6 +139,12 @@ inline int check_params(kwg_ctx* ctx, const kwg_fd1d_params* p)
     return KWG_OK;
 }
 
+// The FP64 solver on FP32 units takes this grid and scheme (fd1d_pair64.cu).
+inline bool pair64_ok(const kwg_fd1d_params* p)
+{
+    return p->precision == KWG_FP64 && p->theta == 0.5 && kwg::fd1d_fp32_nodes_per_lane(p->x_dim) > 0;
+}
+
 // Autotuner key: precision, grid and the batch size rounded up to a power of two.
 // Uneven batches use x_dim = t_dim = 0.
 inline uint64_t tune_key(int precision, int x_dim, int t_dim, long long m)
@@ -167,9 +173,13 @@ inline double time_solve(kwg_ctx* ctx, F&& call)
 // Times every candidate launch shape on fn(params) and returns the fastest: FP64 --
 // the streaming solver with 1, 2, 4 warps per block (as many blocks per SM as fit),
 // with one 4-warp block per SM (one warp per scheduler), and the warp-per-PDE solver
-// (when pcr_ok); FP32 -- 1, 2, 4 and 8 warps per option.
+// (when pcr_ok); FP32 -- 1, 2, 4 and 8 warps per option.  auto_on_chip: a call with AUTO and
+// no record takes the on-chip FP64 solver although KWG_SOLVER_PCR is refused (grids of 1025
+// to 2048 nodes); it is then timed through AUTO, and reported as KWG_SOLVER_AUTO.  The
+// caller has dropped the shape's earlier record.
 template <typename F>
-inline kwg_ctx::Tuned tune(kwg_ctx* ctx, const kwg_fd1d_params* p, bool pcr_ok, F&& fn, kwg_tuning* out)
+inline kwg_ctx::Tuned tune(kwg_ctx* ctx, const kwg_fd1d_params* p, bool pcr_ok, bool auto_on_chip, F&& fn,
+                           kwg_tuning* out)
 {
     kwg_tuning r = {};
     for (double& v : r.thomas_ms) v = -1.;
@@ -209,6 +219,11 @@ inline kwg_ctx::Tuned tune(kwg_ctx* ctx, const kwg_fd1d_params* p, bool pcr_ok, 
             q.sm_blocks = 0;
             r.pcr_ms = time_solve(ctx, [&] { return fn(q); });
             consider(r.pcr_ms, KWG_SOLVER_PCR, 1, 1, 0);
+        } else if (auto_on_chip) {
+            q.solver = KWG_SOLVER_AUTO;
+            q.block_warps = 0;
+            q.sm_blocks = 0;
+            consider(time_solve(ctx, [&] { return fn(q); }), KWG_SOLVER_PCR, 1, 1, 0);
         }
     } else {
         const int ws[4] = {1, 2, 4, 8};
@@ -219,7 +234,7 @@ inline kwg_ctx::Tuned tune(kwg_ctx* ctx, const kwg_fd1d_params* p, bool pcr_ok, 
             consider(ms, KWG_SOLVER_PCR, 1, ws[i], 0);
         }
     }
-    r.solver = best.solver;
+    r.solver = best.solver == KWG_SOLVER_PCR && auto_on_chip && !pcr_ok ? KWG_SOLVER_AUTO : best.solver;
     r.block_warps = best.block_warps;
     r.option_warps = best.option_warps;
     r.sm_blocks = best.sm_blocks;

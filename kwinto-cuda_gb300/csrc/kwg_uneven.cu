@@ -108,14 +108,15 @@ extern "C" int kwg_fd1d_price_uneven(kwg_ctx* ctx, const kwg_option* opts, const
     // uneven batches of this precision and size, else Thomas with one warp per block
     // (FP64) and one warp per option (FP32)
     kwg_ctx::Tuned tn;
+    if (q.precision == KWG_FP64 && q.solver == KWG_SOLVER_AUTO && pair64_ok(&q)) tn.solver = KWG_SOLVER_PCR;
     {
         const auto it = ctx->tuned.find(tune_key(q.precision, 0, 0, (long long)n));
         if (it != ctx->tuned.end()) {
             tn = it->second;
-            if (q.precision == KWG_FP64 && q.solver == KWG_SOLVER_AUTO &&
-                (tn.solver != KWG_SOLVER_PCR || kwg::fd1d_pcr64_nodes_per_lane(x_max) > 0))
-                q.solver = tn.solver;
         }
+        if (q.precision == KWG_FP64 && q.solver == KWG_SOLVER_AUTO &&
+            (tn.solver != KWG_SOLVER_PCR || pair64_ok(&q) || kwg::fd1d_pcr64_nodes_per_lane(x_max) > 0))
+            q.solver = tn.solver;
         if (q.block_warps || q.sm_blocks) {
             if (q.block_warps) tn.block_warps = q.block_warps;
             tn.sm_blocks = q.sm_blocks;
@@ -123,6 +124,7 @@ extern "C" int kwg_fd1d_price_uneven(kwg_ctx* ctx, const kwg_option* opts, const
         if (q.option_warps) tn.option_warps = q.option_warps;
     }
     const bool pcr = q.precision == KWG_FP32 || q.solver == KWG_SOLVER_PCR;
+    const bool pair = q.solver == KWG_SOLVER_PCR && pair64_ok(&q);
     KWG_CUDA(ctx, cudaSetDevice(ctx->device));
 
     // 1. dedup by (t, r, q, z, e, w, x_dim, t_dim)
@@ -181,7 +183,7 @@ extern "C" int kwg_fd1d_price_uneven(kwg_ctx* ctx, const kwg_option* opts, const
         }
     } else {
         auto mlane = [&](uint32_t pde) {
-            return q.precision == KWG_FP32 ? kwg::fd1d_fp32_nodes_per_lane(xd(pde))
+            return q.precision == KWG_FP32 || pair ? kwg::fd1d_fp32_nodes_per_lane(xd(pde))
                                            : kwg::fd1d_pcr64_nodes_per_lane(xd(pde));
         };
         // nodes per lane ascending, node-steps descending (x_dim <= 2048 here, so
@@ -215,8 +217,9 @@ extern "C" int kwg_fd1d_price_uneven(kwg_ctx* ctx, const kwg_option* opts, const
     // 3. pack inputs into pinned memory
     const UnevenLayout L = uneven_layout(ms, n, tiles.size());
     if (int rc = ensure_host(ctx, &ctx->h_io, &ctx->h_io_bytes, L.total)) return rc;
-    const size_t wbytes = pcr ? (size_t)node_lanes * sizeof(double)
-                              : kwg::fd1d_fp64_work_bytes_nl((int)ms, node_lanes);
+    const size_t wbytes = pair  ? kwg::fd1d_pair64_work_bytes((int)ms, node_lanes)
+                          : pcr ? (size_t)node_lanes * sizeof(double)
+                                : kwg::fd1d_fp64_work_bytes_nl((int)ms, node_lanes);
     // the graph bakes in device addresses: grow buffers before deciding on replay
     if (int rc = ensure_device(ctx, &ctx->d_io, &ctx->io_bytes, L.total)) return rc;
     if (int rc = ensure_device(ctx, &ctx->d_work, &ctx->work_bytes, wbytes)) return rc;
@@ -299,7 +302,11 @@ extern "C" int kwg_fd1d_price_uneven(kwg_ctx* ctx, const kwg_option* opts, const
                 ss.row_off += beg;
                 kwg::AssetBatch none = a;
                 none.n = 0;
-                const int r = q.precision == KWG_FP32
+                double* v = (double*)ctx->d_work;
+                const int r = pair ? kwg::fd1d_pair64_launch(sb, none, ss, v, (int32_t*)(v + node_lanes) + beg,
+                                                             d_pde_status + beg, ctx->d_counter, d_prices, d_status,
+                                                             ctx->device, st, ctx->next_events())
+                              : q.precision == KWG_FP32
                                   ? kwg::fd1d_fp32_launch(sb, none, ss, (double*)ctx->d_work, d_pde_status + beg,
                                                           ctx->d_counter, d_prices, d_status, ctx->device, st,
                                                           ctx->next_events())
@@ -318,7 +325,7 @@ extern "C" int kwg_fd1d_price_uneven(kwg_ctx* ctx, const kwg_option* opts, const
     };
 
     uint64_t sig = 0x5eed;
-    for (uint64_t v : {(uint64_t)q.precision, (uint64_t)pcr, (uint64_t)sh.block_warps, (uint64_t)sh.option_warps,
+    for (uint64_t v : {(uint64_t)q.precision, (uint64_t)pcr, (uint64_t)pair, (uint64_t)sh.block_warps, (uint64_t)sh.option_warps,
                        (uint64_t)sh.sm_blocks,
                        (uint64_t)n, (uint64_t)ms, (uint64_t)tiles.size(),
                        (uint64_t)node_lanes, (uint64_t)(uintptr_t)ctx->d_io, (uint64_t)(uintptr_t)ctx->d_work,
@@ -392,10 +399,14 @@ extern "C" int kwg_autotune_uneven(kwg_ctx* ctx, const kwg_option* opts, const i
     for (size_t i = 0; i < n; ++i) x_max = std::max(x_max, (int)x_dims[i]);
     std::vector<double> prices(n);
     const bool pcr_ok = kwg::fd1d_pcr64_nodes_per_lane(x_max) > 0;
-    const kwg_ctx::Tuned best = tune(ctx, p, pcr_ok, [&](const kwg_fd1d_params& q) {
+    const uint64_t key = tune_key(p->precision, 0, 0, (long long)n);
+    ctx->tuned.erase(key);
+    kwg_fd1d_params widest = *p;
+    widest.x_dim = x_max;
+    const kwg_ctx::Tuned best = tune(ctx, p, pcr_ok, pair64_ok(&widest), [&](const kwg_fd1d_params& q) {
         return kwg_fd1d_price_uneven(ctx, opts, x_dims, t_dims, n, &q, prices.data(), nullptr);
     }, out);
-    ctx->tuned[tune_key(p->precision, 0, 0, (long long)n)] = best;
+    ctx->tuned[key] = best;
     ctx->err.clear();
     return KWG_OK;
 }
