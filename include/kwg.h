@@ -92,9 +92,10 @@ typedef struct kwg_fd1d_params {
                           option as its own PDE, fully asynchronously */
     int32_t block_warps;  /* FP64 streaming solver: warps (32 options each) per thread
                              block, 1, 2 or 4; 0 (default) = tuned or 1 */
-    int32_t option_warps; /* warp-per-PDE FP32 solver: warps (32 threads each) per
-                             option, 1, 2, 4 or 8 (grids of more than 1024 nodes at
-                             least 2; at least 2 nodes per lane); 0 (default) = tuned or 1 */
+    int32_t option_warps; /* FP32 solver: warps (32 threads each) per option, 1, 2, 4 or 8
+                             (8 runs as 4; grids of more than 1024 nodes take at least 2,
+                             grids of 128 nodes or fewer 1); 0 (default) = tuned or by the
+                             batch size */
     int32_t sm_blocks;    /* FP64 streaming solver: resident blocks per SM, 0 (default) =
                              tuned or as many as fit (two 4-warp blocks).  With
                              block_warps 4 and sm_blocks 1 each of an SM's four warp
@@ -202,9 +203,8 @@ typedef struct kwg_tuning {
     int32_t sm_blocks;    /* resident blocks per SM of the streaming FP64 solver (0: as many as fit) */
     double thomas_ms[3];  /* streaming FP64 solver with 1, 2, 4 warps per block */
     double pcr_ms;        /* FP64 on-chip solver (KWG_SOLVER_PCR) */
-    double fp32_ms[3];    /* FP32 solver with 1, 2, 4 warps per option (the launch may
-                             use fewer: at least 2 nodes per lane, and at least 2 warps
-                             for grids of more than 1024 nodes) */
+    double fp32_ms[3];    /* FP32 solver with 1, 2, 4 warps per option (the launch may use
+                             another count: option_warps of kwg_fd1d_params) */
     double spread_ms;     /* streaming FP64 solver, 4 warps per block, one block per SM */
     double fp32_8w_ms;    /* FP32 solver with 8 warps per option (same caveat) */
 } kwg_tuning;

@@ -59,9 +59,9 @@ struct Fd1dShape {
     // lane (no padded nodes), which the warp-per-PDE uniform-grid kernels require
     bool full_lanes = false;
     // resolved launch shapes: warps per block of the streaming FP64 solver (1, 2, 4;
-    // 32 options each) and warps per option of the FP32 solver (1, 2)
+    // 32 options each) and warps per option of the FP32 solver (1, 2, 4)
     int block_warps = 1;
-    int option_warps = 1;
+    int option_warps = 0;  // 0: by the batch size
     int sm_blocks = 0;  // FP64 streaming solver: resident blocks per SM (0: as many as fit)
     int keep_nodes = 0;  // FP64 streaming solver: nodes at each sweep's end stored evict-last in L2 (set by the launch)
     // FP64 streaming solver, uniform batches: tiles [0, twin_tiles) hold 16 twin pairs
@@ -95,10 +95,10 @@ int fd1d_fp64_launch(const PdeBatch& b, const AssetBatch& a, const Fd1dShape& sh
                      int* counters, double* prices, int32_t* status, int solve_blocks, cudaStream_t stream,
                      const SolveEvents* ev);
 
-// FP32 stepping (one, two, four or eight warps per PDE, on chip; sh.option_warps).  Nodes per
-// lane M of the one-warp layout for an x-grid of x_dim nodes (the grid is padded to
-// 32*M with decoupled identity rows; W warps take M/W each); -1 if x_dim > 2048.
-// The work buffer holds the final V of every PDE, [m][x_dim] doubles.
+// FP32 stepping (fd1d_fp32.cu): one, two or four warps per PDE on chip (sh.option_warps).  Nodes
+// per lane M of the one-warp layout for an x-grid of x_dim nodes (the grid is padded to 32*M
+// with decoupled identity rows; W warps take M/W each); -1 if x_dim > 2048.  The work buffer
+// holds the final V of every PDE, [m][x_dim] doubles.
 int fd1d_fp32_nodes_per_lane(int x_dim);
 size_t fd1d_fp32_work_bytes(int m, int x_dim);
 int fd1d_fp32_launch(const PdeBatch& b, const AssetBatch& a, const Fd1dShape& sh, double* vout, int32_t* pde_status,
@@ -114,7 +114,7 @@ int fd1d_pcr64_launch(const PdeBatch& b, const AssetBatch& a, const Fd1dShape& s
                       const SolveEvents* ev);
 
 // FP64 accuracy on the FP32 units (fd1d_pair64.cu): theta = 1/2, x_dim <= 2048, one to
-// eight warps per PDE.  The work buffer holds the final V of every PDE and the list of the
+// four warps per PDE.  The work buffer holds the final V of every PDE and the list of the
 // PDEs left to the FP64 kernel (`rescue`, m ints); -1 for shapes it does not take.
 size_t fd1d_pair64_work_bytes(int m, long long nodes);
 int fd1d_pair64_launch(const PdeBatch& b, const AssetBatch& a, const Fd1dShape& sh, double* vout, int32_t* rescue,

@@ -40,7 +40,7 @@ struct kwg_ctx {
     struct Tuned {
         int solver = KWG_SOLVER_THOMAS;
         int block_warps = 1;
-        int option_warps = 1;
+        int option_warps = 0;  // 0: by the batch size
         int sm_blocks = 0;
     };
     std::map<uint64_t, Tuned> tuned;

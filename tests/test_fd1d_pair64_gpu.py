@@ -1,4 +1,4 @@
-"""The FP64 solver on FP32 units (what KWG_SOLVER_AUTO takes for theta = 1/2 and up to 2048
+"""The on-chip solvers.  FP64 on FP32 units (what KWG_SOLVER_AUTO takes for theta = 1/2 and up to 2048
 nodes): edges of its lane and warp layouts, the warps-per-PDE rule, and the PDEs it leaves
 to the FP64 kernel.  Prices within 1e-10 relative of the oracle (or of the streaming FP64
 solver), 1e-13 K absolute below 1e-3, as the library's other FP64 paths."""
@@ -115,3 +115,21 @@ def test_other_schemes_after_tuning(built):
         assert np.array_equal(p, want) and np.array_equal(st, wst)
     finally:
         c.close()
+
+
+@pytest.mark.parametrize("theta", [0.5, 0.8])
+@pytest.mark.parametrize("n,x_dim,density", [(1, 512, 0.25), (305, 512, 0.25), (700, 500, math.inf), (152, 1024, math.inf),
+                                             (153, 1024, 0.25), (40, 2048, math.inf), (40, 2047, 0.25), (3, 3, 0.25),
+                                             (9, 65, math.inf)])
+def test_fp32_warps_per_pde(ctx, n, x_dim, density, theta):
+    """FP32 stepping with the warp count left to the rule, against the streaming FP64 solver
+    within the FP32 path's 1e-5 (a relative 2e-7 on the 3-node grid, whose prices are large)."""
+    import kwg
+
+    o = mixed(n, seed=n)
+    kw = dict(t_dim=50, x_dim=x_dim, scale=5.0, density=density, theta=theta)
+    rc, p, st = ctx.fd1d_price(o, kwg.params(precision=kwg.FP32, **kw))
+    assert rc == 0 and (st == 0).all()
+    rc, want, _ = ctx.fd1d_price(o, kwg.params(solver=kwg.SOLVER_THOMAS, **kw))
+    assert rc == 0
+    assert np.max(np.abs(p - want) - 2e-7 * np.abs(want)) <= 1e-5
