@@ -61,8 +61,8 @@ __device__ __forceinline__ void two_diff(float2 a, float2 b, float2& s, float2& 
 
 // Keeps the compiler from loading the next phase's tables ahead of time: with one warp per
 // PDE no barrier stands between the phases, and the loads it moved up cost registers (pair
-// arithmetic, M = 32: 255 and 444 bytes of spills without, 218 and none with).  FP32 stepping has
-// the registers to spare and is 3 to 10 % slower with it.
+// arithmetic, M = 32: 255 and 444 bytes of spills without, 218 and none with).  Where registers
+// are to spare the early loads are worth 3 to 10 %.
 template <bool kOn>
 __device__ __forceinline__ void phase_edge()
 {
@@ -147,14 +147,25 @@ __device__ __forceinline__ Split split(double v)
     return r;
 }
 
-// Warps per SM that the registers must leave room for.  Pair arithmetic: more (16 at M = 16,
-// 20 at M = 8, 24 at M = 4) spills a little and is no faster (8192 PDEs of 512 uniform nodes
-// 6.09 ms at 12, 6.12 at 16).  FP32 stepping at M = 32: one warp per PDE 9.63 ms at 8 (8192 PDEs,
-// 1024 uniform nodes, 1024 steps) and 9.77 at 12, two warps 6.38 and 5.33 (4096 of 2048 nodes, 512
-// steps); M = 16: 2.41 ms at 16 and 2.79 at 8 (8192 of 512 nodes).
-constexpr int min_warps(int M, int W, bool pair)
+// Warps per SM that the registers must leave room for, and phase edges.  Pair arithmetic, ms:
+//   M = 16, one warp per PDE, tables per node (shared memory holds ten PDEs): 600 PDEs of 512
+//     nodes 0.67 at 8 without edges, 0.76 at 12 with; 8192 of them 6.57 and 6.82; two and four
+//     warps 7.61 at 10, 7.64 at 12, 8.25 at 8 (8192 of 1024 nodes); uniform 5.84 at 14, 6.00 at 12
+//   M = 8, tables per node: 6.50 at 12 without, 6.73 at 16 with, 7.14 at 16 without (16384 of
+//     256 nodes); uniform 6.17 at 16 with, 6.26 at 12 without
+//   M = 4: 3.55 without edges, 3.73 with (16384 of 128 uniform nodes)
+// FP32 stepping, without edges: M = 32, one warp per PDE 9.63 at 8 (8192 of 1024 uniform nodes, 1024
+// steps) and 9.77 at 12, two warps 6.38 and 5.33 (4096 of 2048 nodes, 512 steps); M = 16 2.41 at 16
+// and 2.79 at 8 (8192 of 512 nodes).
+constexpr int min_warps(int M, int W, bool uni, bool pair)
 {
-    return M == 32 ? (pair || W == 1 ? 8 : 12) : M == 16 ? (pair ? 12 : 16) : 16;
+    if (!pair) return M == 32 ? (W == 1 ? 8 : 12) : 16;
+    if (M == 16) return uni ? (W == 1 ? 14 : 12) : (W == 1 ? 8 : 10);
+    return M == 32 ? 8 : M == 8 && !uni ? 12 : 16;
+}
+__host__ __device__ constexpr bool phase_edges(int M, int W, bool uni, bool pair)
+{
+    return pair && (M == 32 || (M == 16 && (uni || W > 1)) || (M == 8 && uni));
 }
 
 // Shared-memory layout of one PDE group (floats).  P = M / 2 slots, NL = 32 W lanes.
@@ -193,12 +204,12 @@ struct Lay {
 }  // namespace
 
 template <int M, bool kUni, int W, bool kPair>
-__global__ void __launch_bounds__(32 * W, min_warps(M, W, kPair) / W)
+__global__ void __launch_bounds__(32 * W, min_warps(M, W, kUni, kPair) / W)
     fd1d_solve_onchip(const PdeBatch b, Fd1dShape sh, double* __restrict__ vout, int32_t* __restrict__ pde_status,
                       int* __restrict__ counters, int32_t* __restrict__ rescue)
 {
     using Y = Lay<M, kUni, W, kPair>;
-    constexpr bool kEdge = kPair;
+    constexpr bool kEdge = phase_edges(M, W, kUni, kPair);
     constexpr int P = Y::P, NL = Y::NL, kStride = Y::kStride;
     static_assert(M >= 2 && M % 2 == 0, "as many rows above the pivot as below");
     extern __shared__ __align__(16) float tab[];
