@@ -147,25 +147,39 @@ __device__ __forceinline__ Split split(double v)
     return r;
 }
 
-// Warps per SM that the registers must leave room for, and phase edges.  Pair arithmetic, ms:
-//   M = 16, one warp per PDE, tables per node (shared memory holds ten PDEs): 600 PDEs of 512
-//     nodes 0.67 at 8 without edges, 0.76 at 12 with; 8192 of them 6.57 and 6.82; two and four
-//     warps 7.61 at 10, 7.64 at 12, 8.25 at 8 (8192 of 1024 nodes); uniform 5.84 at 14, 6.00 at 12
-//   M = 8, tables per node: 6.50 at 12 without, 6.73 at 16 with, 7.14 at 16 without (16384 of
-//     256 nodes); uniform 6.17 at 16 with, 6.26 at 12 without
-//   M = 4: 3.55 without edges, 3.73 with (16384 of 128 uniform nodes)
-// FP32 stepping, without edges: M = 32, one warp per PDE 9.63 at 8 (8192 of 1024 uniform nodes, 1024
-// steps) and 9.77 at 12, two warps 6.38 and 5.33 (4096 of 2048 nodes, 512 steps); M = 16 2.41 at 16
-// and 2.79 at 8 (8192 of 512 nodes).
-constexpr int min_warps(int M, int W, bool uni, bool pair)
+// A variant's share of the registers: the warps per SM that must fit, phase edges, and how
+// many of the factor tables stay in registers for the whole PDE (the spikes; also 1/d and u;
+// also l -- shared memory otherwise returns them every step, 40 of 56 bytes per slot and lane in
+// FP32 stepping, where it was the busiest unit, 71 %).  Best of 1 to 5 settings each, ms before
+// the tables moved -> now (8192 PDEs of 512 and 1024 nodes, 16384 of 256 and 128, 4096 of 2048;
+// 512 steps, FP32 at 2048 nodes 1024):
+//                          FP32 stepping             pair arithmetic
+//   M = 32 uniform         9.63 (1024 steps)         12.44
+//   M = 16 uniform, W = 1  2.41 -> 2.28              5.84 -> 5.66
+//   M = 16, W = 1          2.94 -> 2.75              6.57 -> 6.41
+//   M = 16, W = 2          7.33 -> 6.90              7.60 -> 7.53 (255 steps)
+//   M = 16, W = 4          18.3 -> 15.5              8.74 -> 7.85 (255 steps)
+//   M = 8 uniform          2.43 -> 2.22              6.16 -> 5.97
+//   M = 8                  2.89 -> 2.52              6.49 -> 6.12
+//   M = 4 uniform          1.54 -> 1.30              3.55 -> 3.55
+// Fewer registers or more warps spill or starve: FP32 M = 32 9.77 at 12 warps, pair M = 16 W = 2
+// 9.58 with all tables, 8.25 at 8 warps.
+struct Budget {
+    int warps, tables;
+    bool edges;
+};
+__host__ __device__ constexpr Budget budget(int M, int W, bool uni, bool pair)
 {
-    if (!pair) return M == 32 ? (W == 1 ? 8 : 12) : 16;
-    if (M == 16) return uni ? (W == 1 ? 14 : 12) : (W == 1 ? 8 : 10);
-    return M == 32 ? 8 : M == 8 && !uni ? 12 : 16;
-}
-__host__ __device__ constexpr bool phase_edges(int M, int W, bool uni, bool pair)
-{
-    return pair && (M == 32 || (M == 16 && (uni || W > 1)) || (M == 8 && uni));
+    if (!pair) {
+        if (M == 32) return {W == 1 ? 8 : 12, 0, false};
+        if (M == 16 && uni) return W == 1 ? Budget{12, 3, false} : Budget{16, 0, false};
+        if (M == 16) return W == 1 ? Budget{12, 1, false} : W == 2 ? Budget{12, 2, false} : Budget{10, 3, false};
+        return W > 1 ? Budget{16, 3, false} : Budget{M == 8 ? 16 : 20, 2, false};  // few PDEs: 128 of 512 nodes 0.25, 0.27 at 20
+    }
+    if (M == 32) return {8, 0, true};
+    if (M == 16 && uni) return W == 1 ? Budget{10, 2, true} : Budget{12, 0, true};
+    if (M == 16) return W == 1 ? Budget{8, 3, false} : W == 2 ? Budget{12, 1, true} : Budget{10, 2, true};
+    return {16, 3, M == 8};
 }
 
 // Shared-memory layout of one PDE group (floats).  P = M / 2 slots, NL = 32 W lanes.
@@ -204,12 +218,13 @@ struct Lay {
 }  // namespace
 
 template <int M, bool kUni, int W, bool kPair>
-__global__ void __launch_bounds__(32 * W, min_warps(M, W, kUni, kPair) / W)
+__global__ void __launch_bounds__(32 * W, budget(M, W, kUni, kPair).warps / W)
     fd1d_solve_onchip(const PdeBatch b, Fd1dShape sh, double* __restrict__ vout, int32_t* __restrict__ pde_status,
                       int* __restrict__ counters, int32_t* __restrict__ rescue)
 {
     using Y = Lay<M, kUni, W, kPair>;
-    constexpr bool kEdge = phase_edges(M, W, kUni, kPair);
+    constexpr bool kEdge = budget(M, W, kUni, kPair).edges;
+    constexpr int kReg = budget(M, W, kUni, kPair).tables;
     constexpr int P = Y::P, NL = Y::NL, kStride = Y::kStride;
     static_assert(M >= 2 && M % 2 == 0, "as many rows above the pivot as below");
     extern __shared__ __align__(16) float tab[];
@@ -695,6 +710,19 @@ __global__ void __launch_bounds__(32 * W, min_warps(M, W, kUni, kPair) / W)
             }
         };
         auto coef_s = [&](int kk) { return kUni && kk > 0 && kk < P - 1 ? cAl : C1t[crow(kk) * NL]; };
+        // factors held in registers for the whole PDE (kReg)
+        constexpr int P1 = kReg >= 3 ? P : 1, P2 = kReg >= 2 ? P : 1, P3 = kReg >= 1 ? P : 1;
+        float2 r1[P1];
+        float4 r2[P2], r3[P3];
+#pragma unroll
+        for (int kk = 0; kk < P1; ++kk) r1[kk] = T1[kk * kStride];
+#pragma unroll
+        for (int kk = 0; kk < P2; ++kk) r2[kk] = T2[kk * kStride];
+#pragma unroll
+        for (int kk = 0; kk < P3; ++kk) r3[kk] = T3[kk * kStride];
+        auto fac1 = [&](int kk) -> float2 { return kReg >= 3 ? r1[kReg >= 3 ? kk : 0] : T1[kk * kStride]; };
+        auto fac2 = [&](int kk) -> float4 { return kReg >= 2 ? r2[kReg >= 2 ? kk : 0] : T2[kk * kStride]; };
+        auto fac3 = [&](int kk) -> float4 { return kReg >= 1 ? r3[kReg >= 1 ? kk : 0] : T3[kk * kStride]; };
         // B x = y in FP32, in place on the slots; s1: x of the next lane's separator, um: x of
         // the previous lane's last node
         auto solve = [&](float2 (&y)[P], int which, float& s1, float& um) {
@@ -702,15 +730,15 @@ __global__ void __launch_bounds__(32 * W, min_warps(M, W, kUni, kPair) / W)
             float2 F = f2(0.f, 0.f);
 #pragma unroll
             for (int kk = P - 1; kk >= 1; --kk) {
-                F = fma2(neg(T1[kk * kStride]), F, y[kk]);
+                F = fma2(neg(fac1(kk)), F, y[kk]);
                 y[kk] = F;
             }
-            const float4 p2 = T2[0], p3 = T3[0];
-            const float yP = fmaf(-p2.w, F.y, fmaf(-T1[0].y, F.x, y[0].y)) * p2.y;
+            const float4 p2 = fac2(0), p3 = fac3(0);
+            const float yP = fmaf(-p2.w, F.y, fmaf(-fac1(0).y, F.x, y[0].y)) * p2.y;
             float2 X = f2(yP, yP);
 #pragma unroll
             for (int kk = 1; kk < P; ++kk) {
-                const float4 q = T2[kk * kStride];
+                const float4 q = fac2(kk);
                 X = fma2(neg(f2(q.z, q.w)), X, mul2(y[kk], f2(q.x, q.y)));
                 y[kk] = X;
             }
@@ -764,7 +792,7 @@ __global__ void __launch_bounds__(32 * W, min_warps(M, W, kUni, kPair) / W)
             const float2 ms = f2(-s, -s), ms1 = f2(-s1, -s1);
 #pragma unroll
             for (int kk = 1; kk < P; ++kk) {
-                const float4 q = T3[kk * kStride];
+                const float4 q = fac3(kk);
                 y[kk] = fma2(ms1, f2(q.z, q.w), fma2(ms, f2(q.x, q.y), y[kk]));
             }
             y[0] = f2(s, fmaf(-s1, p3.w, fmaf(-s, p3.y, yP)));
