@@ -18,15 +18,11 @@ struct GemmArgs {
     const __nv_bfloat16* A;
     const __nv_bfloat16* B;
     int M, N, K, lda, ldb;
-    int k_per_split;                  // K range of one blockIdx.z
     const float* bias;                // [N] or null
-    bool silu;                        // activation applied to out_bf16 / out_bf16_t
-    bool atomic_f32;                  // out_f32 += acc (split-K reduction), no other outputs
+    bool silu;                        // activation applied to out_bf16
     float* out_f32;                   // [M][ldo]
     __nv_bfloat16* out_bf16;          // [M][ldo]
-    __nv_bfloat16* out_bf16_t;        // [N][ldt] (transposed)
-    float* out_dact;                  // [M][ldo]: act'(z)
-    int ldo, ldt;
+    int ldo;
     // out_bf16 row stride; with split_bf16 the value is stored as hi at column n and
     // lo = bf16(a - hi) at column n + N, so the next layer reads a 16-bit mantissa
     int ldb16;
@@ -41,7 +37,8 @@ struct GemmArgs {
 
 size_t gemm_smem_bytes();
 cudaError_t gemm_set_smem_limit();  // on the current device
-cudaError_t gemm_launch(const GemmArgs& g, int splits, cudaStream_t stream);
+cudaError_t gemm_launch(const GemmArgs& g, cudaStream_t stream);
+cudaError_t mlp_grad_set_smem_limit();  // on the current device
 
 // Shared-memory limits of the surrogate kernels on the current device, once per
 // device (bit d of a process-wide mask); every launcher calls it first.
@@ -79,19 +76,18 @@ struct MlpBox {
 // Barone-Adesi-Whaley for American options, Black-Scholes for European ones.
 void mlp_launch_featurize(const kwg_option* opts, int n, const MlpBox& box, float* x, uint8_t* inside, double* base,
                           cudaStream_t st);
-// Feature rows f[idx[r]] (idx null: f[r]) for r < b -> split BF16 rows x [b_pad][64]
-// (rows >= b zero), transposed hi rows xt [64][b_pad] (may be null), targets tb and
-// floors fb (either may be null; a null fl gives no floor).
-void mlp_launch_pack(const float* f, const float* t, const float* fl, const int32_t* idx, int b, int b_pad,
-                     __nv_bfloat16* x, __nv_bfloat16* xt, float* tb, float* fb, cudaStream_t st);
-void mlp_launch_out_grad(const float* y, const float* t, const float* fl, int b, int b_pad, __nv_bfloat16* dy,
-                         __nv_bfloat16* dyt, float* db5, double* loss, cudaStream_t st);
-void mlp_launch_dz(const float* da, const float* dact, int b, int b_pad, __nv_bfloat16* dz, __nv_bfloat16* dzt,
-                   float* db, cudaStream_t st);
-void mlp_launch_adam(float* p, const float* g, float* m, float* v, int n, float lr, float b1, float b2, float eps,
+// Feature rows f[r] for r < b -> split BF16 rows x [b_pad][64] (rows >= b zero).
+void mlp_launch_pack(const float* f, int b, int b_pad, __nv_bfloat16* x, cudaStream_t st);
+// Loss (added to *loss) and gradients (added to g) of one minibatch: rows idx[r] (idx null: r) of
+// features x, targets t and floors fl (may be null), r < b, in one launch (mlp_train.cu).
+cudaError_t mlp_launch_grad(const float* x, const float* t, const float* fl, const int32_t* idx, int b,
+                            const __nv_bfloat16* wb, const float* params, float* g, double* loss, int* error, int sms,
+                            cudaStream_t st);
+// Adam on the FP32 parameters; clears the gradients it has used.
+void mlp_launch_adam(float* p, float* g, float* m, float* v, int n, float lr, float b1, float b2, float eps,
                      float c1, float c2, cudaStream_t st);
-// BF16 forward weights (layout above) and W^T [5][128 in][128 out] for the backward.
-void mlp_launch_refresh(const float* w, __nv_bfloat16* wb, __nv_bfloat16* wt, cudaStream_t st);
+// BF16 forward weights (layout above).
+void mlp_launch_refresh(const float* w, __nv_bfloat16* wb, cudaStream_t st);
 void mlp_launch_price(const kwg_option* opts, const float* y, const double* base, int n, float y_scale,
                       double* prices, cudaStream_t st);
 

@@ -34,20 +34,16 @@ struct kwg_mlp {
     std::string err;
     kwg::MlpBox box;
     float y_scale = 1.f;
-    // parameters (FP32 master), gradients, Adam moments; BF16 forward weights
-    // (K-doubled, mlp.h) and W^T for the backward
+    // parameters (FP32 master), gradients, Adam moments; BF16 forward weights (K-doubled, mlp.h)
     float *p = nullptr, *g = nullptr, *m = nullptr, *v = nullptr;
-    __nv_bfloat16 *wb = nullptr, *wt = nullptr;
+    __nv_bfloat16* wb = nullptr;
     long long adam_t = 0;
-    // batch workspace (capacity `cap` rows)
+    // forward workspace (capacity `cap` rows): split input rows [64], split activations [256],
+    // outputs
     int cap = 0;
-    __nv_bfloat16 *x = nullptr, *xt = nullptr;             // split input rows [64] / transposed hi
-    __nv_bfloat16 *act[3] = {}, *actt[4] = {};              // split activations [256] / transposed hi
-    float* dact[4] = {};                                      // SiLU'(z)
-    float *y = nullptr, *tb = nullptr, *fb = nullptr, *da = nullptr;
-    float* feat = nullptr;                                    // features [cap][5]
-    double* base = nullptr;                                   // analytic base prices [cap]
-    __nv_bfloat16 *dy = nullptr, *dyt = nullptr, *dz = nullptr, *dzt = nullptr;
+    __nv_bfloat16* x = nullptr;
+    __nv_bfloat16* act[3] = {};
+    float* y = nullptr;
     double* loss = nullptr;
     int* error = nullptr;
     // the last training run: mean loss of every epoch, the epoch whose parameters
@@ -76,49 +72,23 @@ int mlp_err(kwg_mlp* h, int code, const std::string& msg)
 
 void free_ws(kwg_mlp* h)
 {
-    void* bufs[] = {h->x, h->xt, h->y, h->tb, h->fb, h->da, h->dy, h->dyt, h->dz, h->dzt, h->feat, h->base};
+    void* bufs[] = {h->x, h->act[0], h->act[1], h->act[2], h->y};
     for (void* b : bufs)
         if (b) cudaFree(b);
-    for (int l = 0; l < 4; ++l) {
-        if (l < 3 && h->act[l]) cudaFree(h->act[l]);
-        if (h->actt[l]) cudaFree(h->actt[l]);
-        if (h->dact[l]) cudaFree(h->dact[l]);
-        if (l < 3) h->act[l] = nullptr;
-        h->actt[l] = nullptr;
-        h->dact[l] = nullptr;
-    }
-    h->x = h->xt = h->dy = h->dyt = h->dz = h->dzt = nullptr;
-    h->y = h->tb = h->fb = h->da = h->feat = nullptr;
-    h->base = nullptr;
+    h->x = h->act[0] = h->act[1] = h->act[2] = nullptr;
+    h->y = nullptr;
     h->cap = 0;
 }
 
-// Workspace for batches of up to `rows` rows (a multiple of 64).
+// Forward workspace for up to `rows` rows (a multiple of 64).
 int ensure_ws(kwg_mlp* h, int rows)
 {
     if (rows <= h->cap) return KWG_OK;
     free_ws(h);
-    const size_t r = (size_t)rows, w = kMlpWidth;
+    const size_t r = (size_t)rows;
     MLP_CUDA(h, cudaMalloc(&h->x, r * kwg::kMlpInK * 2));
-    MLP_CUDA(h, cudaMalloc(&h->xt, r * kwg::kMlpInK * 2));
-    for (int l = 0; l < 4; ++l) {
-        if (l < 3) MLP_CUDA(h, cudaMalloc(&h->act[l], r * kwg::kMlpHidK * 2));
-        MLP_CUDA(h, cudaMalloc(&h->actt[l], r * w * 2));
-        MLP_CUDA(h, cudaMalloc(&h->dact[l], r * w * 4));
-    }
+    for (int l = 0; l < 3; ++l) MLP_CUDA(h, cudaMalloc(&h->act[l], r * kwg::kMlpHidK * 2));
     MLP_CUDA(h, cudaMalloc(&h->y, r * 4));
-    MLP_CUDA(h, cudaMalloc(&h->feat, r * kMlpIn * 4));
-    MLP_CUDA(h, cudaMalloc(&h->base, r * 8));
-    MLP_CUDA(h, cudaMalloc(&h->tb, r * 4));
-    MLP_CUDA(h, cudaMalloc(&h->fb, r * 4));
-    MLP_CUDA(h, cudaMalloc(&h->da, r * w * 4));
-    MLP_CUDA(h, cudaMalloc(&h->dy, r * w * 2));
-    MLP_CUDA(h, cudaMalloc(&h->dyt, r * w * 2));
-    MLP_CUDA(h, cudaMalloc(&h->dz, r * w * 2));
-    MLP_CUDA(h, cudaMalloc(&h->dzt, r * w * 2));
-    // dY has one nonzero column (dY^T one nonzero row): the rest stays zero
-    MLP_CUDA(h, cudaMemset(h->dy, 0, r * w * 2));
-    MLP_CUDA(h, cudaMemset(h->dyt, 0, r * w * 2));
     h->cap = rows;
     return KWG_OK;
 }
@@ -133,21 +103,17 @@ kwg::GemmArgs gemm_args(const __nv_bfloat16* a, const __nv_bfloat16* b, int m, i
     g.K = k;
     g.lda = k;
     g.ldb = k;
-    g.k_per_split = k;
     g.ldo = n;
-    g.ldt = m;
     g.ldb16 = n;
     g.error = error;
     return g;
 }
 
 float* bias_of(float* p, int layer) { return p + kMlpWeights + layer * kMlpWidth; }
-const __nv_bfloat16* wt_of(const __nv_bfloat16* w, int layer) { return w + (size_t)layer * kMlpWidth * kMlpWidth; }
 const __nv_bfloat16* wb_of(const __nv_bfloat16* w, int layer) { return w + (size_t)layer * kwg::kMlpFwdSlot; }
 
-// Forward over rows [0, rows) of h->x.  train: keep transposed hi activations and
-// SiLU' for the backward pass.  Output (the scaled premium) in h->y.
-int forward(kwg_mlp* h, int rows, bool train)
+// Forward over rows [0, rows) of h->x.  Output (the scaled premium) in h->y.
+int forward(kwg_mlp* h, int rows)
 {
     const __nv_bfloat16* in = h->x;
     for (int l = 0; l < 4; ++l) {
@@ -164,50 +130,8 @@ int forward(kwg_mlp* h, int rows, bool train)
             g.head_bias = bias_of(h->p, 4);
             g.out_head = h->y;
         }
-        if (train) {
-            g.out_bf16_t = h->actt[l];
-            g.out_dact = h->dact[l];
-        }
-        MLP_CUDA(h, kwg::gemm_launch(g, 1, h->stream));
+        MLP_CUDA(h, kwg::gemm_launch(g, h->stream));
         if (l < 3) in = h->act[l];
-    }
-    return KWG_OK;
-}
-
-// Backward of the MSE loss over rows [0, b) (b_pad rows in the buffers); gradients
-// accumulate into h->g (zeroed here), the loss into *h->loss.
-int backward(kwg_mlp* h, int b, int b_pad)
-{
-    MLP_CUDA(h, cudaMemsetAsync(h->g, 0, sizeof(float) * kMlpParams, h->stream));
-    // dY^T is [128][b_pad]: only row 0 is written, so clear the rest for this b_pad
-    MLP_CUDA(h, cudaMemsetAsync(h->dyt, 0, (size_t)kMlpWidth * b_pad * 2, h->stream));
-    kwg::mlp_launch_out_grad(h->y, h->tb, h->fb, b, b_pad, h->dy, h->dyt, bias_of(h->g, 4), h->loss, h->stream);
-    const int split = 256;
-    // dW[out][in] += dZ^T A over the batch (A: transposed hi activations, `ins` rows)
-    auto dw = [&](const __nv_bfloat16* dzt, const __nv_bfloat16* xt, int layer, int ins) -> int {
-        kwg::GemmArgs g = gemm_args(dzt, xt, kMlpWidth, ins, b_pad, h->error);
-        g.ldo = kMlpWidth;
-        g.atomic_f32 = true;
-        g.out_f32 = h->g + (size_t)layer * kMlpWidth * kMlpWidth;
-        g.k_per_split = split;
-        MLP_CUDA(h, kwg::gemm_launch(g, (b_pad + split - 1) / split, h->stream));
-        return KWG_OK;
-    };
-    auto dx = [&](const __nv_bfloat16* dzr, int layer) -> int {
-        kwg::GemmArgs g = gemm_args(dzr, wt_of(h->wt, layer), b_pad, kMlpWidth, kMlpWidth, h->error);
-        g.out_f32 = h->da;
-        MLP_CUDA(h, kwg::gemm_launch(g, 1, h->stream));
-        return KWG_OK;
-    };
-    // output layer: dW5 = dY^T act4, dA4 = dY W5
-    if (int rc = dw(h->dyt, h->actt[3], 4, kMlpWidth)) return rc;
-    if (int rc = dx(h->dy, 4)) return rc;
-    for (int l = 3; l >= 0; --l) {
-        kwg::mlp_launch_dz(h->da, h->dact[l], b, b_pad, h->dz, h->dzt, bias_of(h->g, l), h->stream);
-        if (int rc = l == 0 ? dw(h->dzt, h->xt, 0, kwg::kMlpInK) : dw(h->dzt, h->actt[l - 1], l, kMlpWidth))
-            return rc;
-        if (l > 0)
-            if (int rc = dx(h->dz, l)) return rc;
     }
     return KWG_OK;
 }
@@ -316,7 +240,7 @@ int kwg_gemm_bf16(const void* d_a, const void* d_b, float* d_c, int m, int n, in
     kwg::GemmArgs g = gemm_args(static_cast<const __nv_bfloat16*>(d_a), static_cast<const __nv_bfloat16*>(d_b), m, n,
                                 k, nullptr);
     g.out_f32 = d_c;
-    return kwg::gemm_launch(g, 1, (cudaStream_t)stream) == cudaSuccess ? KWG_OK : KWG_ERR_CUDA;
+    return kwg::gemm_launch(g, (cudaStream_t)stream) == cudaSuccess ? KWG_OK : KWG_ERR_CUDA;
 }
 
 kwg_mlp* kwg_mlp_create(int device, uint64_t seed)
@@ -333,7 +257,6 @@ kwg_mlp* kwg_mlp_create(int device, uint64_t seed)
     ok = ok && cudaMalloc(&h->m, sizeof(float) * kMlpParams) == cudaSuccess;
     ok = ok && cudaMalloc(&h->v, sizeof(float) * kMlpParams) == cudaSuccess;
     ok = ok && cudaMalloc(&h->wb, sizeof(__nv_bfloat16) * kwg::kMlpFwdWeights) == cudaSuccess;
-    ok = ok && cudaMalloc(&h->wt, sizeof(__nv_bfloat16) * kMlpWeights) == cudaSuccess;
     ok = ok && cudaMalloc(&h->loss, sizeof(double)) == cudaSuccess;
     ok = ok && cudaMalloc(&h->error, sizeof(int)) == cudaSuccess;
     if (!ok) {
@@ -369,7 +292,7 @@ void kwg_mlp_destroy(kwg_mlp* h)
     cudaSetDevice(h->device);
     if (h->stream) cudaStreamSynchronize(h->stream);
     free_ws(h);
-    void* bufs[] = {h->p, h->g, h->m, h->v, h->wb, h->wt, h->loss, h->error, h->d_arena};
+    void* bufs[] = {h->p, h->g, h->m, h->v, h->wb, h->loss, h->error, h->d_arena};
     for (void* b : bufs)
         if (b) cudaFree(b);
     if (h->h_arena) cudaFreeHost(h->h_arena);
@@ -394,7 +317,7 @@ int kwg_mlp_set_params(kwg_mlp* h, const float* params, const double* box_lo, co
     MLP_CUDA(h, cudaMemsetAsync(h->v, 0, sizeof(float) * kMlpParams, h->stream));
     MLP_CUDA(h, cudaMemsetAsync(h->error, 0, sizeof(int), h->stream));
     h->adam_t = 0;
-    kwg::mlp_launch_refresh(h->p, h->wb, h->wt, h->stream);
+    kwg::mlp_launch_refresh(h->p, h->wb, h->stream);
     MLP_CUDA(h, cudaStreamSynchronize(h->stream));
     return KWG_OK;
 }
@@ -420,8 +343,8 @@ int kwg_mlp_forward(kwg_mlp* h, const float* d_x, int n, float* d_y)
     MLP_CUDA(h, cudaSetDevice(h->device));
     const int rows = (n + 63) / 64 * 64;
     if (int rc = ensure_ws(h, rows)) return rc;
-    kwg::mlp_launch_pack(d_x, nullptr, nullptr, nullptr, n, rows, h->x, nullptr, nullptr, nullptr, h->stream);
-    if (int rc = forward(h, rows, false)) return rc;
+    kwg::mlp_launch_pack(d_x, n, rows, h->x, h->stream);
+    if (int rc = forward(h, rows)) return rc;
     MLP_CUDA(h, cudaMemcpyAsync(d_y, h->y, (size_t)n * 4, cudaMemcpyDeviceToDevice, h->stream));
     return check_error(h);
 }
@@ -432,12 +355,10 @@ int kwg_mlp_gradients(kwg_mlp* h, const float* d_x, const float* d_t, const floa
     if (!h || !d_x || !d_t || !d_grad || n <= 0) return KWG_ERR_INVALID;
     h->err.clear();
     MLP_CUDA(h, cudaSetDevice(h->device));
-    const int rows = (n + 63) / 64 * 64;
-    if (int rc = ensure_ws(h, rows)) return rc;
-    kwg::mlp_launch_pack(d_x, d_t, d_floor, nullptr, n, rows, h->x, h->xt, h->tb, h->fb, h->stream);
+    MLP_CUDA(h, cudaMemsetAsync(h->g, 0, sizeof(float) * kMlpParams, h->stream));
     MLP_CUDA(h, cudaMemsetAsync(h->loss, 0, sizeof(double), h->stream));
-    if (int rc = forward(h, rows, true)) return rc;
-    if (int rc = backward(h, n, rows)) return rc;
+    MLP_CUDA(h, kwg::mlp_launch_grad(d_x, d_t, d_floor, nullptr, n, h->wb, h->p, h->g, h->loss, h->error, h->sms,
+                                     h->stream));
     MLP_CUDA(h, cudaMemcpyAsync(d_grad, h->g, sizeof(float) * kMlpParams, cudaMemcpyDeviceToDevice, h->stream));
     if (loss) MLP_CUDA(h, cudaMemcpyAsync(loss, h->loss, sizeof(double), cudaMemcpyDeviceToHost, h->stream));
     return check_error(h);
@@ -459,8 +380,6 @@ int kwg_mlp_train(kwg_mlp* h, const kwg_option* d_opts, const double* d_prices, 
     if (!h || !d_opts || !d_prices || n <= 0 || epochs <= 0 || batch <= 0 || !(lr > 0.f)) return KWG_ERR_INVALID;
     h->err.clear();
     MLP_CUDA(h, cudaSetDevice(h->device));
-    const int b_pad = (std::min(batch, n) + 63) / 64 * 64;
-    if (int rc = ensure_ws(h, b_pad)) return rc;
     // features, premium targets and exercise-region floors of the whole training set
     float *X = nullptr, *T = nullptr, *F = nullptr, *pbest = nullptr;
     double* base = nullptr;
@@ -517,6 +436,10 @@ int kwg_mlp_train(kwg_mlp* h, const kwg_option* d_opts, const double* d_prices, 
         cleanup();
         return mlp_err(h, KWG_ERR_CUDA, "kwg_mlp_train: parameter snapshot failed");
     }
+    if (cudaMemsetAsync(h->g, 0, sizeof(float) * kMlpParams, h->stream) != cudaSuccess) {
+        cleanup();
+        return mlp_err(h, KWG_ERR_CUDA, "kwg_mlp_train: gradient reset failed");
+    }
     for (int ep = 0; ep < epochs; ++ep) {
         std::shuffle(order.begin(), order.end(), rng);
         if (cudaMemcpyAsync(idx, order.data(), (size_t)n * 4, cudaMemcpyHostToDevice, h->stream) != cudaSuccess ||
@@ -526,13 +449,11 @@ int kwg_mlp_train(kwg_mlp* h, const kwg_option* d_opts, const double* d_prices, 
         }
         for (int s = 0; s < steps_per_epoch; ++s, ++step) {
             const int b = std::min(batch, n - s * batch);
-            const int bp = (b + 63) / 64 * 64;
-            kwg::mlp_launch_pack(X, T, F, idx + (size_t)s * batch, b, bp, h->x, h->xt, h->tb, h->fb, h->stream);
-            int rc = forward(h, bp, true);
-            if (!rc) rc = backward(h, b, bp);
-            if (rc) {
+            const cudaError_t ge = kwg::mlp_launch_grad(X, T, F, idx + (size_t)s * batch, b, h->wb, h->p, h->g, h->loss,
+                                                        h->error, h->sms, h->stream);
+            if (ge != cudaSuccess) {
                 cleanup();
-                return rc;
+                return mlp_err(h, KWG_ERR_CUDA, std::string("kwg_mlp_train: ") + cudaGetErrorString(ge));
             }
             // Adam with a cosine-decayed learning rate (to 1% of lr)
             ++h->adam_t;
@@ -542,7 +463,7 @@ int kwg_mlp_train(kwg_mlp* h, const kwg_option* d_opts, const double* d_prices, 
             kwg::mlp_launch_adam(h->p, h->g, h->m, h->v, kMlpParams, lr_t, b1, b2, 1e-8f,
                                  1.f - std::pow(b1, (float)h->adam_t), 1.f - std::pow(b2, (float)h->adam_t),
                                  h->stream);
-            kwg::mlp_launch_refresh(h->p, h->wb, h->wt, h->stream);
+            kwg::mlp_launch_refresh(h->p, h->wb, h->stream);
         }
         // mean of the epoch's minibatch losses
         double l = 0.;
@@ -565,7 +486,7 @@ int kwg_mlp_train(kwg_mlp* h, const kwg_option* d_opts, const double* d_prices, 
             e = cudaMemcpyAsync(h->p, pbest, sizeof(float) * kMlpParams, cudaMemcpyDeviceToDevice, h->stream);
             if (e == cudaSuccess) e = cudaMemsetAsync(h->m, 0, sizeof(float) * kMlpParams, h->stream);
             if (e == cudaSuccess) e = cudaMemsetAsync(h->v, 0, sizeof(float) * kMlpParams, h->stream);
-            if (e == cudaSuccess) kwg::mlp_launch_refresh(h->p, h->wb, h->wt, h->stream);
+            if (e == cudaSuccess) kwg::mlp_launch_refresh(h->p, h->wb, h->stream);
         }
         if (e != cudaSuccess) {
             cleanup();
@@ -580,7 +501,7 @@ int kwg_mlp_train(kwg_mlp* h, const kwg_option* d_opts, const double* d_prices, 
             cleanup();
             return mlp_err(h, KWG_ERR_CUDA, "kwg_mlp_train: parameter restore failed");
         }
-        kwg::mlp_launch_refresh(h->p, h->wb, h->wt, h->stream);
+        kwg::mlp_launch_refresh(h->p, h->wb, h->stream);
     }
     if (cudaStreamSynchronize(h->stream) != cudaSuccess) {
         cleanup();

@@ -235,6 +235,7 @@ cudaError_t mlp_prepare_device()
     if (done.load() & bit) return cudaSuccess;
     cudaError_t e = cudaFuncSetAttribute(mlp_price_fused, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemBytes);
     if (e == cudaSuccess) e = gemm_set_smem_limit();
+    if (e == cudaSuccess) e = mlp_grad_set_smem_limit();
     if (e == cudaSuccess) done.fetch_or(bit);
     return e;
 }

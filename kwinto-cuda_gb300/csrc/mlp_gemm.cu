@@ -1,16 +1,14 @@
 // mlp_gemm.cu -- BF16 x BF16 -> FP32 GEMM on the tcgen05 tensor cores with a fused
-// epilogue, the building block of the MLP surrogate's forward and backward passes.
+// epilogue, the building block of the MLP surrogate's layer-by-layer forward pass.
 //
 //     acc[M][N] = A[M][K] * B[N][K]^T        (A, B row-major BF16: K contiguous)
 //     z = acc + bias[n]
-//     out_f32[m][n]  = z                      (or atomically += acc, for split-K)
-//     out_bf16[m][n] = act(z),  out_bf16_t[n][m] = act(z)
-//     out_dact[m][n] = act'(z)               (FP32; SiLU derivative for backward)
+//     out_f32[m][n]  = z
+//     out_bf16[m][n] = act(z)
 //     out_head[m]    = head_bias + sum_n head_w[n] act(z)   (FP32, fused 128 -> 1 layer)
 // out_bf16 may hold the activation as a BF16 pair (hi at column n, lo at n + N).
 //
-// One CTA of 128 threads computes one 128 x 128 tile (blockIdx.x over M, .y over N)
-// over the K range of blockIdx.z.  K is staged 64 at a time into shared memory in
+// One CTA of 128 threads computes one 128 x 128 tile (blockIdx.x over M, .y over N).  K is staged 64 at a time into shared memory in
 // the no-swizzle core-matrix layout (tc.cuh); thread 0 issues four 128x128x16 MMAs
 // per stage into a TMEM accumulator of 128 columns and commits to an mbarrier that
 // every thread waits on (bounded) before the stage is refilled.  The epilogue reads
@@ -33,12 +31,6 @@ constexpr uint32_t kStageBBytes = kTileN * kStageK * 2;  // 16 KB
 constexpr uint32_t kTmemCols = 128;
 
 __device__ __forceinline__ float silu(float z) { return z / (1.f + __expf(-z)); }
-__device__ __forceinline__ float dsilu(float z)
-{
-    const float s = 1.f / (1.f + __expf(-z));
-    return s * (1.f + z * (1.f - s));
-}
-
 // Copies a 128 x 64 BF16 block (rows r0.., cols k0..) of a row-major matrix with
 // leading dimension ld into shared memory in core-matrix layout.  Rows >= rows
 // are zero-filled.
@@ -64,8 +56,6 @@ __global__ void __launch_bounds__(128) gemm_bf16_tn(const GemmArgs g)
     uint32_t* tslot = reinterpret_cast<uint32_t*>(gsm + kStageABytes + kStageBBytes + 8);
     const int warp = threadIdx.x / 32, lane = threadIdx.x % 32;
     const int m0 = blockIdx.x * kTileM, n0 = blockIdx.y * kTileN;
-    const int kz0 = blockIdx.z * g.k_per_split;
-    const int kz1 = min(g.K, kz0 + g.k_per_split);
 
     if (warp == 0) {
         tc::tmem_alloc(smem_addr(tslot), kTmemCols);
@@ -83,7 +73,7 @@ __global__ void __launch_bounds__(128) gemm_bf16_tn(const GemmArgs g)
     bool ok = true;
 
     uint32_t phase = 0, last = 0;
-    for (int k0 = kz0; k0 < kz1; k0 += kStageK) {
+    for (int k0 = 0; k0 < g.K; k0 += kStageK) {
         stage_block(sa, g.A, g.lda, m0, g.M, k0);
         stage_block(sb, g.B, g.ldb, n0, g.N, k0);
         tc::fence_proxy_async_smem();
@@ -94,7 +84,7 @@ __global__ void __launch_bounds__(128) gemm_bf16_tn(const GemmArgs g)
             for (int kk = 0; kk < kStageK / 16; ++kk) {
                 const uint64_t ad = tc::smem_desc(smem_addr(sa) + kk * 256, 128, (kStageK / 8) * 128);
                 const uint64_t bd = tc::smem_desc(smem_addr(sb) + kk * 256, 128, (kStageK / 8) * 128);
-                tc::mma_bf16(tmem, ad, bd, idesc, (k0 > kz0) || (kk > 0));
+                tc::mma_bf16(tmem, ad, bd, idesc, (k0 > 0) || (kk > 0));
             }
             tc::commit(smem_addr(mbar));
         }
@@ -106,7 +96,7 @@ __global__ void __launch_bounds__(128) gemm_bf16_tn(const GemmArgs g)
     if (!__syncthreads_and(ok)) mbar_wait(mbar, last);  // let MMAs in flight finish before TMEM is freed
     tc::fence_after_sync();
 
-    if (__syncthreads_and(ok) && kz1 > kz0) {
+    if (__syncthreads_and(ok)) {
         const int row = m0 + warp * 32 + lane;
         float head = 0.f;
         for (int c = 0; c < kTileN; c += 32) {
@@ -118,10 +108,6 @@ __global__ void __launch_bounds__(128) gemm_bf16_tn(const GemmArgs g)
                 const int n = n0 + c + i;
                 if (n >= g.N) continue;
                 const float acc = v[i];
-                if (g.atomic_f32) {
-                    atomicAdd(g.out_f32 + (size_t)row * g.ldo + n, acc);
-                    continue;
-                }
                 const float z = acc + (g.bias ? g.bias[n] : 0.f);
                 if (g.out_f32) g.out_f32[(size_t)row * g.ldo + n] = z;
                 const float a = g.silu ? silu(z) : z;
@@ -130,8 +116,6 @@ __global__ void __launch_bounds__(128) gemm_bf16_tn(const GemmArgs g)
                     g.out_bf16[(size_t)row * g.ldb16 + n] = hi;
                     if (g.split_bf16) g.out_bf16[(size_t)row * g.ldb16 + g.N + n] = __float2bfloat16(a - __bfloat162float(hi));
                 }
-                if (g.out_bf16_t) g.out_bf16_t[(size_t)n * g.ldt + row] = hi;
-                if (g.out_dact) g.out_dact[(size_t)row * g.ldo + n] = g.silu ? dsilu(z) : 1.f;
                 if (g.head_w) head = fmaf(__bfloat162float(g.head_w[n]), a, head);
             }
         }
@@ -153,10 +137,10 @@ cudaError_t gemm_set_smem_limit()
     return cudaFuncSetAttribute(gemm_bf16_tn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)gemm_smem_bytes());
 }
 
-cudaError_t gemm_launch(const GemmArgs& g, int splits, cudaStream_t stream)
+cudaError_t gemm_launch(const GemmArgs& g, cudaStream_t stream)
 {
     if (const cudaError_t e = mlp_prepare_device(); e != cudaSuccess) return e;
-    dim3 grid((g.M + kTileM - 1) / kTileM, (g.N + kTileN - 1) / kTileN, splits);
+    dim3 grid((g.M + kTileM - 1) / kTileM, (g.N + kTileN - 1) / kTileN);
     gemm_bf16_tn<<<grid, 128, gemm_smem_bytes(), stream>>>(g);
     return cudaGetLastError();
 }

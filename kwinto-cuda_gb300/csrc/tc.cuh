@@ -38,6 +38,11 @@ __host__ __device__ constexpr uint32_t idesc_bf16_f32(int m, int n)
     return (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(n >> 3) << 17) | ((uint32_t)(m >> 4) << 24);
 }
 
+// Instruction-descriptor bits: A, B in MN-major form.  The same core matrices (8 x 16 bytes) then hold
+// 8 K-rows of 8 consecutive M or N elements; in the descriptor SBO stays the distance between
+// core matrices adjacent along M or N, LBO the distance between those adjacent along K.
+constexpr uint32_t kMajorMnA = 1u << 15, kMajorMnB = 1u << 16;
+
 // Warp-collective TMEM allocation of `ncols` columns (power of 2, >= 32); the base
 // address is written to shared memory at `dst`.
 __device__ __forceinline__ void tmem_alloc(uint32_t dst_saddr, uint32_t ncols)
