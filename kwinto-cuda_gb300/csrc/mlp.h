@@ -88,8 +88,6 @@ void mlp_launch_adam(float* p, float* g, float* m, float* v, int n, float lr, fl
                      float c1, float c2, cudaStream_t st);
 // BF16 forward weights (layout above).
 void mlp_launch_refresh(const float* w, __nv_bfloat16* wb, cudaStream_t st);
-void mlp_launch_price(const kwg_option* opts, const float* y, const double* base, int n, float y_scale,
-                      double* prices, cudaStream_t st);
 
 // Network prices of n options in one persistent launch (mlp_fused.cu): `sms` CTAs at
 // most, weights resident in shared memory, activations on chip.

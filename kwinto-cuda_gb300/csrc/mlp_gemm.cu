@@ -18,6 +18,7 @@
 #include <cuda_runtime.h>
 
 #include "mlp.h"
+#include "mlp_math.cuh"
 #include "tc.cuh"
 #include "tma.cuh"
 
@@ -30,7 +31,6 @@ constexpr uint32_t kStageABytes = kTileM * kStageK * 2;  // 16 KB
 constexpr uint32_t kStageBBytes = kTileN * kStageK * 2;  // 16 KB
 constexpr uint32_t kTmemCols = 128;
 
-__device__ __forceinline__ float silu(float z) { return z / (1.f + __expf(-z)); }
 // Copies a 128 x 64 BF16 block (rows r0.., cols k0..) of a row-major matrix with
 // leading dimension ld into shared memory in core-matrix layout.  Rows >= rows
 // are zero-filled.
@@ -110,7 +110,7 @@ __global__ void __launch_bounds__(128) gemm_bf16_tn(const GemmArgs g)
                 const float acc = v[i];
                 const float z = acc + (g.bias ? g.bias[n] : 0.f);
                 if (g.out_f32) g.out_f32[(size_t)row * g.ldo + n] = z;
-                const float a = g.silu ? silu(z) : z;
+                const float a = g.silu ? silu_f(z) : z;
                 const __nv_bfloat16 hi = __float2bfloat16(a);
                 if (g.out_bf16) {
                     g.out_bf16[(size_t)row * g.ldb16 + n] = hi;

@@ -21,11 +21,12 @@ __global__ void mlp_featurize(const kwg_option* __restrict__ opts, int n, MlpBox
     const kwg_option o = opts[i];
     float f[kMlpIn];
     bool in = false;
-    features(o, box, f, in);
+    const OptionTerms terms = option_terms(o);
+    features(o, terms, box, f, in);
     if (x)
 #pragma unroll
         for (int c = 0; c < kMlpIn; ++c) x[(size_t)i * kMlpIn + c] = f[c];
-    if (base) base[i] = base_price(o);
+    if (base) base[i] = base_price(o, terms);
     if (inside) inside[i] = in ? 1 : 0;
 }
 
@@ -84,18 +85,6 @@ __global__ void mlp_refresh(const float* __restrict__ w, __nv_bfloat16* __restri
     }
 }
 
-// Surrogate price = max(intrinsic, base + K * premium), premium = y / y_scale, base
-// the analytic price of mlp_featurize.
-__global__ void mlp_price(const kwg_option* __restrict__ opts, const float* __restrict__ y,
-                          const double* __restrict__ base, int n, float y_scale, double* __restrict__ prices)
-{
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    const kwg_option o = opts[i];
-    const double v = base[i] + o.k * (double)(y[i] / y_scale);
-    prices[i] = o.e ? fmax(v, intrinsic(o)) : v;
-}
-
 void mlp_launch_featurize(const kwg_option* opts, int n, const MlpBox& box, float* x, uint8_t* inside, double* base,
                           cudaStream_t st)
 {
@@ -116,12 +105,6 @@ void mlp_launch_adam(float* p, float* g, float* m, float* v, int n, float lr, fl
 void mlp_launch_refresh(const float* w, __nv_bfloat16* wb, cudaStream_t st)
 {
     mlp_refresh<<<dim3(kMlpWidth, kMlpLayers), kMlpWidth, 0, st>>>(w, wb);
-}
-
-void mlp_launch_price(const kwg_option* opts, const float* y, const double* base, int n, float y_scale,
-                      double* prices, cudaStream_t st)
-{
-    mlp_price<<<(n + 127) / 128, 128, 0, st>>>(opts, y, base, n, y_scale, prices);
 }
 
 }  // namespace kwg

@@ -57,7 +57,8 @@ __device__ __forceinline__ uint32_t act_offset(int row, int ch)
 
 __device__ __forceinline__ float dsilu_f(float z)
 {
-    const float s = 1.f / (1.f + __expf(-z));
+    // the reciprocal as in silu_f: no branch, corrected by its exact residual
+    const float d = 1.f + __expf(-z), r = rcp_approx(d), s = z < -87.f ? 0.f : fmaf(fmaf(-d, r, 1.f), r, r);
     return s * (1.f + z * (1.f - s));
 }
 
