@@ -70,6 +70,16 @@ constexpr float kNoFloor = 1e30f;
 struct MlpBox {
     double lo[kMlpIn];
     double hi[kMlpIn];
+    double scale[kMlpIn];  // 2 / (hi - lo)
+
+    void set(const double* l, const double* h)
+    {
+        for (int i = 0; i < kMlpIn; ++i) {
+            lo[i] = l[i];
+            hi[i] = h[i];
+            scale[i] = 2. / (h[i] - l[i]);
+        }
+    }
 };
 
 // Features [n][5] (may be null), in-box flags and analytic base prices (may be null):

@@ -266,8 +266,7 @@ kwg_mlp* kwg_mlp_create(int device, uint64_t seed)
     // training box of the 32768-option workload's distributions, with a margin:
     // K/S in [0.8, 1.2], vol sqrt T in [0.05, 0.85], r T and q T in [0, 0.2]
     const double lo[kMlpIn] = {-0.25, 0.04, 0.0, 0.0, -1.0}, hi[kMlpIn] = {0.20, 0.86, 0.2, 0.2, 1.0};
-    std::memcpy(h->box.lo, lo, sizeof lo);
-    std::memcpy(h->box.hi, hi, sizeof hi);
+    h->box.set(lo, hi);
     // He-uniform weights on the active entries; padded rows/columns stay zero
     std::vector<float> p(kMlpParams, 0.f);
     std::mt19937_64 rng(seed);
@@ -307,10 +306,7 @@ int kwg_mlp_set_params(kwg_mlp* h, const float* params, const double* box_lo, co
     if (!h || !params || !(y_scale > 0.f)) return KWG_ERR_INVALID;
     h->err.clear();
     MLP_CUDA(h, cudaSetDevice(h->device));
-    if (box_lo && box_hi) {
-        std::memcpy(h->box.lo, box_lo, sizeof h->box.lo);
-        std::memcpy(h->box.hi, box_hi, sizeof h->box.hi);
-    }
+    if (box_lo && box_hi) h->box.set(box_lo, box_hi);
     h->y_scale = y_scale;
     MLP_CUDA(h, cudaMemcpyAsync(h->p, params, sizeof(float) * kMlpParams, cudaMemcpyHostToDevice, h->stream));
     MLP_CUDA(h, cudaMemsetAsync(h->m, 0, sizeof(float) * kMlpParams, h->stream));

@@ -5,7 +5,7 @@
 // launches per minibatch, each with 32 or 16 CTAs of 128 threads that staged their operands
 // through registers and wrote activations, SiLU', their transposes and dZ to global memory, one
 // row per thread.  A 4096-row minibatch took 0.79 ms a call; this kernel's 64 CTAs keep
-// everything on chip and only add 82 thousand gradient sums each to global memory: 41 us, 0.071 ms
+// everything on chip and only add 82 thousand gradient sums each to global memory: 0.065 ms
 // a call.  It is bound by the latency of its eight dependent MMA-and-epilogue stages.
 //
 // Channels in lanes.  Every product is formed with the channels along the MMA's M (the TMEM

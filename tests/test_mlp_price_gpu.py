@@ -1,4 +1,4 @@
-"""The surrogate's pricing kernel at the edges of its tile pipeline."""
+"""The surrogate's pricing kernel at the edges of its tile pipeline, and its analytic base price."""
 import numpy as np
 import pytest
 
@@ -48,3 +48,32 @@ def test_tiles_and_slots(net, tiles, rows):
     want = np.where(o["e"] != 0, np.maximum(want, intrinsic), want)
     assert np.max(np.abs(price.cpu().numpy() - want) / o["k"]) <= 1e-12
     assert torch.equal(inside, inside2)
+
+
+@pytest.mark.parametrize("case", ["wide", "small rates", "zero rates", "negative rates", "small vol"])
+def test_base_price_matches_oracle(net, case):
+    """Barone-Adesi-Whaley base price against the FP64 bisection, within 2e-6 of the strike: FP32 carries
+    the root and the premium (16 roundings of 2^-23)."""
+    import mlp_oracle as mo
+    import portfolio
+    import torch
+
+    n, rng = 20000, np.random.default_rng(3)
+    o = portfolio.american_portfolio(n, seed=11)
+    if case == "wide":
+        o["z"], o["t"] = np.exp(rng.uniform(-4, 0.5, n)), np.exp(rng.uniform(-6, 2.5, n))
+        o["r"], o["q"] = rng.uniform(0, 0.15, n), rng.uniform(0, 0.15, n)
+        o["k"] = o["s"] * np.exp(rng.uniform(-2, 2, n))
+    elif case == "small rates":
+        o["r"], o["q"] = np.exp(rng.uniform(-25, -2, n)), np.exp(rng.uniform(-25, -2, n))
+    elif case == "zero rates":
+        o["r"], o["q"] = (np.where(rng.random(n) < 0.3, 0.0, o[f]) for f in ("r", "q"))
+    elif case == "negative rates":
+        o["r"], o["q"] = rng.uniform(-0.05, 0.1, n), rng.uniform(-0.05, 0.1, n)
+    else:
+        o["z"], o["t"] = np.exp(rng.uniform(-12, -4, n)), 1.0
+    d_o = _device(o)
+    base = torch.empty(n, dtype=torch.float64, device="cuda")
+    net.featurize(d_o.data_ptr(), n, 0, 0, base.data_ptr())
+    torch.cuda.synchronize()
+    assert np.max(np.abs(base.cpu().numpy() - mo.baw(o)) / o["k"]) <= 2e-6
