@@ -3,17 +3,24 @@
 //
 // Numerics.  The reference step B V' = E V (src/Math/kwFd1d.cpp:61-132) is taken in
 // delta form,  V' = max(V + d, p)  with  B d = dt A V  (E = B + dt A), so FP32 only
-// ever carries the small increment d.  V and the payoff p are float-float pairs
-// (hi + lo, ~48 significant bits).  The residual dt A V is formed from differences
-// of the pairs, which are exact in FP32, with the operator written as
-//     dt A V_j = c1 S_j + c2 (V_{j+1}-V_j) + c3 (V_j-V_{j-1}) + c4 V_j,
-//     S_j = (V_{j+1}-V_j) - (V_j-V_{j-1}),
+// ever carries the small increment d, and over X = V - p, p the payoff:
+//     B d = dt A X + q,   X' = max(X + d, 0),   q = dt A p.
+// X is a float-float pair (hi + lo, ~48 significant bits).  The residual dt A X is formed from
+// differences of the pairs, which are exact in FP32, with the operator written as
+//     dt A X_j = c1 S_j + c2 (X_{j+1}-X_j) + c3 (X_j-X_{j-1}) + c4 X_j,
+//     S_j = (X_{j+1}-X_j) - (X_j-X_{j-1}),
 // c1 = dt axx l2, c2 = dt (axx (u2-l2) + ax im), c3 = dt ax im, c4 = dt a0 (the
 // reference's inverse spacings, src/Math/kwFd1d.cpp:87-92), so rounding the
 // coefficients to FP32 perturbs the PDE's coefficients by ~1e-7 relatively instead
-// of breaking the cancellation of the second difference.  The grid, c1..c4, the factors and
+// of breaking the cancellation of the second difference.  q uses the same rounded
+// coefficients (fd1d_onchip.cuh).  The grid, c1..c4, the factors and
 // the payoff are computed in FP64 (src/Pricer/kwFd1d.cpp:110-139); the final
-// interpolation reads V = hi + lo in FP64.
+// interpolation reads V = p + hi + lo in FP64.
+//
+// Over V itself a step compares with the payoff: three more packed operations per two nodes
+// (23 against 20) and 16 bytes of tables per slot instead of the 8 of q.  Per 8192 PDEs: 1024
+// nodes (1024 steps) 9.63 -> 8.59 ms, density 0.25 (512 steps) 6.90 -> 6.08; 4096 of 2048 (512 steps)
+// 5.26 -> 4.36; and 7.60, 5.96, 4.36 with the registers that it freed (budget()).
 #include "fd1d_onchip.cuh"
 
 namespace kwg {
@@ -68,9 +75,8 @@ namespace {
 // 1024-node grids with tables per node and on 2048-node uniform ones, four on 2048-node grids
 // with tables per node; twice as many while every warp still has a scheduler to itself (the
 // rule of fd1d_pair64.cu).  Measured, ms with 1/2/4 warps (512 steps): 128 PDEs of 512 nodes
-// 0.40/0.32/0.26; 8192 PDEs of 1024 nodes, density 0.25, 9.15/7.38/8.46, uniform (1024 steps)
-// 9.63/10.36/13.6; 4096 PDEs of 2048 nodes (1024 steps) -/21.6/18.0, uniform (512 steps)
-// -/5.33/5.87.
+// 0.32/0.27/0.24; 8192 PDEs of 1024 nodes, density 0.25, 6.86/5.96/6.56, uniform
+// 3.95/4.52/5.83; 4096 PDEs of 2048 nodes -/8.95/7.49, uniform -/4.36/4.75.
 int fp32_warps(int m1, bool uni, int m, int sms)
 {
     int w = m1 == 64 ? (uni ? 2 : 4) : m1 == 32 && !uni ? 2 : 1;

@@ -1,7 +1,7 @@
 // fd1d_onchip.cuh -- the on-chip theta-scheme kernel: one, two or four warps per PDE, the
 // whole PDE in registers and shared memory, stepping in FP32.  Two modes:
-//   kPair = false (fd1d_fp32.cu): one FP32 solve per step for the increment, V as an
-//     unevaluated pair of floats;
+//   kPair = false (fd1d_fp32.cu): one FP32 solve per step for the increment, V less the payoff
+//     as an unevaluated pair of floats;
 //   kPair = true (fd1d_pair64.cu): two solves per step and a residual in pair arithmetic --
 //     FP64 accuracy, theta = 1/2.
 //
@@ -114,7 +114,7 @@ __device__ __forceinline__ float2 pair_residual(float2 ah, float2 al, const PP2&
 
 // (h, l) += d for FP32 stepping: h takes the rounded sum and l collects its rounding error by
 // Fast2Sum (exact when |h| >= |d| or h == 0 -- the increment of a step is small next to the
-// value it updates; where it is not, V is near 0 and the loss is an ulp of that tiny sum).
+// value it updates; where it is not, X is near 0 and the loss is an ulp of that tiny sum).
 // The pair is not renormalised: each step adds at most half an ulp of h to l, so over a
 // few thousand steps |l| stays within ~2^11 ulp(h), far below h, and the differences of
 // neighbouring h that the residual takes stay exact.
@@ -153,17 +153,16 @@ __device__ __forceinline__ Split split(double v)
 // FP32 stepping, where it was the busiest unit, 71 %).  Best of 1 to 5 settings each, ms before
 // the tables moved -> now (8192 PDEs of 512 and 1024 nodes, 16384 of 256 and 128, 4096 of 2048;
 // 512 steps, FP32 at 2048 nodes 1024):
-//                          FP32 stepping             pair arithmetic
-//   M = 32 uniform         9.63 (1024 steps)         12.44
-//   M = 16 uniform, W = 1  2.41 -> 2.28              5.84 -> 5.66
-//   M = 16, W = 1          2.94 -> 2.75              6.57 -> 6.41
-//   M = 16, W = 2          7.33 -> 6.90              7.60 -> 7.53 (255 steps)
-//   M = 16, W = 4          18.3 -> 15.5              8.74 -> 7.85 (255 steps)
-//   M = 8 uniform          2.43 -> 2.22              6.16 -> 5.97
-//   M = 8                  2.89 -> 2.52              6.49 -> 6.12
-//   M = 4 uniform          1.54 -> 1.30              3.55 -> 3.55
-// Fewer registers or more warps spill or starve: FP32 M = 32 9.77 at 12 warps, pair M = 16 W = 2
-// 9.58 with all tables, 8.25 at 8 warps.
+//                          FP32 stepping       pair arithmetic (255 steps at 1024 and 2048 nodes)
+//   M = 32 uniform         4.57 -> 3.95        6.79           (FP32: 12 warps at 168 registers, 8 at 236)
+//   M = 16 uniform, W = 1  2.41 -> 2.03        5.84 -> 5.66
+//   M = 16 uniform, W = 2                      6.65
+//   M = 16, W = 1          2.94 -> 2.51        6.57 -> 6.41
+//   M = 16, W = 2          7.33 -> 5.95        7.60 -> 7.57
+//   M = 16, W = 4          18.3 -> 13.4        8.74 -> 7.99
+//   M = 8 uniform          2.43 -> 2.07        6.16 -> 5.97
+//   M = 8                  2.89 -> 2.26        6.49 -> 6.12
+//   M = 4 uniform          1.54 -> 1.31        3.60
 struct Budget {
     int warps, tables;
     bool edges;
@@ -171,10 +170,12 @@ struct Budget {
 __host__ __device__ constexpr Budget budget(int M, int W, bool uni, bool pair)
 {
     if (!pair) {
-        if (M == 32) return {W == 1 ? 8 : 12, 0, false};
-        if (M == 16 && uni) return W == 1 ? Budget{12, 3, false} : Budget{16, 0, false};
-        if (M == 16) return W == 1 ? Budget{12, 1, false} : W == 2 ? Budget{12, 2, false} : Budget{10, 3, false};
-        return W > 1 ? Budget{16, 3, false} : Budget{M == 8 ? 16 : 20, 2, false};  // few PDEs: 128 of 512 nodes 0.25, 0.27 at 20
+        if (M == 32) return uni ? Budget{12, 0, W == 1} : Budget{8, 1, W == 2};
+        if (M == 16 && uni) return W == 1 ? Budget{12, 2, true} : Budget{20, 0, W == 2};
+        if (M == 16) return W == 1 ? Budget{10, 2, true} : W == 2 ? Budget{12, 2, true} : Budget{10, 3, false};
+        if (W > 1) return M == 8 ? (W == 2 ? Budget{10, 3, true} : Budget{16, 3, false}) : Budget{12, 3, false};
+        if (M == 2) return uni ? Budget{16, 1, false} : Budget{20, 2, false};
+        return {M == 8 && !uni ? 16 : 20, 3, false};
     }
     if (M == 32) return {8, 0, true};
     if (M == 16 && uni) return W == 1 ? Budget{10, 2, true} : Budget{12, 0, true};
@@ -183,7 +184,8 @@ __host__ __device__ constexpr Budget budget(int M, int W, bool uni, bool pair)
 }
 
 // Shared-memory layout of one PDE group (floats).  P = M / 2 slots, NL = 32 W lanes.
-//   PPt  [P][NL] float4   payoff (hi_a, hi_b, lo_a, lo_b); hi -inf where no floor applies
+//   PPt  [P][NL] float4   payoff (hi_a, hi_b, lo_a, lo_b), hi -inf where no floor applies; in
+//                         FP32 stepping q [P][NL] float2 in its place
 //   Cht  [S][NL] float4   (A_a, A_b, B_a, B_b) high parts, Clt low parts: the multipliers
 //                         of a slot's two differences (below); S = P, or on uniform grids
 //                         of full lanes the two slots that can hold a boundary node
@@ -259,7 +261,6 @@ __global__ void __launch_bounds__(32 * W, budget(M, W, kUni, kPair).warps / W)
     // row of slot kk in the coefficient tables (uniform grids of full lanes keep slots 0, P-1)
     auto crow = [](int kk) { return kUni ? (kk == 0 ? 0 : Y::S - 1) : kk; };
 
-    const int j0 = K * M;
     for (;;) {
         int pde = 0;
         if constexpr (W == 1) {
@@ -273,6 +274,10 @@ __global__ void __launch_bounds__(32 * W, budget(M, W, kUni, kPair).warps / W)
         }
         if (pde >= b.m) break;
         const int N = shape_x(sh, pde), TL = shape_t(sh, pde);
+        // The lane's first node.  A grid that does not fill the lanes is padded in front (negative
+        // nodes, rows of the identity), so that the last node, which has no floor, is always the last
+        // lane's last.
+        const int j0 = kUni ? K * M : K * M - (NL * M - N);
 
         // ------------------------------------------------------------ setup (FP64)
         // Bound by the FP64 unit and, for few PDEs, by its latency: reciprocals by one cubic
@@ -337,10 +342,10 @@ __global__ void __launch_bounds__(32 * W, budget(M, W, kUni, kPair).warps / W)
         };
         auto x_of = [&](const Walk& v) { return uniform ? v.s : mul(sh.density, v.s); };
         auto alpha_of = [&](int j, double iu, double im) {
-            return j == 0 ? mul(ax_t, iu) : j >= N - 1 ? 0. : mul(im, fma(axx_t, iu, ax_t));
+            return j == 0 ? mul(ax_t, iu) : (j < 0 || j >= N - 1) ? 0. : mul(im, fma(axx_t, iu, ax_t));
         };
         auto beta_of = [&](int j, double im, double id) {
-            return j == N - 1 ? -mul(ax_t, id) : (j == 0 || j >= N) ? 0. : mul(im, fma(axx_t, id, -ax_t));
+            return j == N - 1 ? -mul(ax_t, id) : j <= 0 ? 0. : mul(im, fma(axx_t, id, -ax_t));
         };
         // Payoff and coefficients of node i go to the tables.  The slot's differences are D_s
         // (towards the pivot) and D_(s+1) (away from it): node a = P-k takes alpha D_s - beta
@@ -351,7 +356,7 @@ __global__ void __launch_bounds__(32 * W, budget(M, W, kUni, kPair).warps / W)
         };
         auto increments = [&](int j, double iu, double im, double id) -> Inc {
             const double ax_d = mul(dt, a.ax), axx_d = mul(mul(2., dt), a.axx);
-            if (j >= N) return {0.f, 0.f, 0.f};
+            if (j < 0) return {0.f, 0.f, 0.f};
             if (j == 0) return {0.f, (float)mul(ax_d, iu), 0.f};
             if (j == N - 1) return {0.f, 0.f, (float)mul(ax_d, id)};
             const double drift = mul(ax_d, im), lower = mul(mul(axx_d, id), im);
@@ -360,7 +365,7 @@ __global__ void __launch_bounds__(32 * W, budget(M, W, kUni, kPair).warps / W)
         auto store = [&](int i, double x, double ex, double al, double be, double iu, double im, double id) {
             const int j = j0 + i, s = slot_of(i), c = comp_of(i);
             double p = 0.;
-            if (j < N && ((w < 0) ? (x < 0.) : (x > 0.))) {
+            if (j >= 0 && ((w < 0) ? (x < 0.) : (x > 0.))) {
                 if (!uniform) ex = exp(x);
                 p = fmax(0., (w < 0) ? sub(1., ex) : sub(ex, 1.));
             }
@@ -412,7 +417,7 @@ __global__ void __launch_bounds__(32 * W, budget(M, W, kUni, kPair).warps / W)
                         im = rcp(add(wn.dx, da));
                     }
                     double al = 0., be = 0., bb = 1.;
-                    if (j < N) {
+                    if (j >= 0) {
                         al = alpha_of(j, iu, im);
                         be = beta_of(j, im, ida);
                         bb = sub(add(1., add(al, be)), gamma);
@@ -457,7 +462,7 @@ __global__ void __launch_bounds__(32 * W, budget(M, W, kUni, kPair).warps / W)
                         im = rcp(add(wn.dx, dd));
                     }
                     double al = 0., be = 0., bb = 1.;
-                    if (j < N) {
+                    if (j >= 0) {
                         al = alpha_of(j, iud, im);
                         be = beta_of(j, im, idn);
                         bb = sub(add(1., add(al, be)), gamma);
@@ -652,24 +657,24 @@ __global__ void __launch_bounds__(32 * W, budget(M, W, kUni, kPair).warps / W)
             H[kk] = f2(p.x, p.y);
             L[kk] = f2(p.z, p.w);
         }
-        // no floor on the last node and on the padding
-#pragma unroll
-        for (int kk = 0; kk < P; ++kk) {
-            const int na = j0 + (kk == 0 ? 0 : P - kk), nb = j0 + P + kk;
-            if (na >= N - 1) PPt[kk * NL].x = -INFINITY;
-            if (nb >= N - 1) PPt[kk * NL].y = -INFINITY;
-        }
-        // V = max(V, p) on slot kk
+        if constexpr (kPair)
+            if (K == NL - 1) PPt[(P - 1) * NL].y = -INFINITY;  // the last node has no floor
+        // V = max(V, p) on slot kk; in FP32 stepping X = max(X, 0)
         auto floor_at = [&](int kk, float2& h, float2& l) {
-            const float4 p = PPt[kk * NL];
-            const float2 d = add2(sub2(h, f2(p.x, p.y)), sub2(l, f2(p.z, p.w)));
-            if (d.x < 0.f) {
-                h.x = p.x;
-                l.x = p.z;
-            }
-            if (d.y < 0.f) {
-                h.y = p.y;
-                l.y = p.w;
+            if constexpr (kPair) {
+                const float4 p = PPt[kk * NL];
+                const float2 d = add2(sub2(h, f2(p.x, p.y)), sub2(l, f2(p.z, p.w)));
+                if (d.x < 0.f) {
+                    h.x = p.x;
+                    l.x = p.z;
+                }
+                if (d.y < 0.f) {
+                    h.y = p.y;
+                    l.y = p.w;
+                }
+            } else {
+                if (h.x < 0.f) h.x = l.x = 0.f;
+                if (h.y < 0.f && (kk < P - 1 || K < NL - 1)) h.y = l.y = 0.f;  // not on the last node
             }
         };
         // the multiplier of V itself; uniform grids of full lanes: the interior multipliers
@@ -710,6 +715,120 @@ __global__ void __launch_bounds__(32 * W, budget(M, W, kUni, kPair).warps / W)
             }
         };
         auto coef_s = [&](int kk) { return kUni && kk > 0 && kk < P - 1 ? cAl : C1t[crow(kk) * NL]; };
+        // state of the nodes beside the lane's: node -1 and node M
+        float Hm, Lm, Hp, Lp;
+        auto neighbours = [&]() {
+            const float2 last = P > 1 ? f2(H[P - 1].y, L[P - 1].y) : f2(H[0].y, L[0].y);
+            Hm = __shfl_up_sync(kAll, last.x, 1);
+            Lm = __shfl_up_sync(kAll, last.y, 1);
+            Hp = __shfl_down_sync(kAll, H[0].x, 1);
+            Lp = __shfl_down_sync(kAll, L[0].x, 1);
+            if constexpr (W > 1) {
+                if (k == 0) {
+                    xe[4 * warp] = H[0].x;
+                    xe[4 * warp + 1] = L[0].x;
+                }
+                if (k == 31) {
+                    xe[4 * warp + 2] = last.x;
+                    xe[4 * warp + 3] = last.y;
+                }
+                __syncthreads();
+                if (k == 0 && warp > 0) {
+                    Hm = xe[4 * warp - 2];
+                    Lm = xe[4 * warp - 1];
+                }
+                if (k == 31 && warp < W - 1) {
+                    Hp = xe[4 * warp + 4];
+                    Lp = xe[4 * warp + 5];
+                }
+            }
+            if (K == 0) Hm = Lm = 0.f;
+            if (K == NL - 1) Hp = Lp = 0.f;
+        };
+
+        // FP32 stepping carries X = V - p (fd1d_fp32.cu).  X starts at zero; the payoff waits in
+        // the result row, and its tables give way to the constant part q = dt A p of the
+        // residual, from pair arithmetic with the steps' own rounded coefficients.  FP32 cannot
+        // hold q at the payoff's kink, and the same rounding every step would triple the
+        // error (grid of 2048 nodes, density 0.25: 1.1e-9 to 6e-9); passed on to the next node, where q is
+        // small, it moves by a node instead (1.0e-9).
+        float2* const qt = reinterpret_cast<float2*>(tab + Y::oPP) + K;
+        float2 q_low{};
+        double* const V = vout + shape_row(sh, pde);
+        if (!kPair && run) {
+            neighbours();
+            auto payoff = [&](int kk) {
+                const float4 p = PPt[kk * NL];
+                return PP2{f2(p.x, p.y), f2(p.z, p.w)};
+            };
+            // q of slot kk over its payoffs; V = p
+            auto source = [&](int kk, const PP2& p, const PP2& X, const PP2& Z, const PP2& S) {
+                float2 A, B, low = f2(0.f, 0.f), s1, s2, s, e;
+                coef_h(kk, A, B);
+                auto product = [&](float2 a, const PP2& v) {
+                    const float2 t = mul2(a, v.h);
+                    low = add2(low, fma2(a, v.l, fma2(a, v.h, neg(t))));
+                    return t;
+                };
+                const float2 tS = product(coef_s(kk), S), tX = product(A, X), tZ = product(B, Z), tV = product(gh, p);
+                two_sum(tS, tX, s1, e);
+                low = add2(low, e);
+                two_sum(tZ, tV, s2, e);
+                low = add2(low, e);
+                two_sum(s1, s2, s, e);
+                low = add2(low, e);
+                const float2 h = add2(s, low), l = sub2(low, sub2(h, s));
+                PPt[kk * NL] = make_float4(h.x, h.y, l.x, l.y);
+                const int na = j0 + (kk == 0 ? 0 : P - kk), nb = j0 + P + kk;
+                if (na >= 0) V[na] = (double)p.h.x + (double)p.l.x;
+                if (nb >= 0) V[nb] = (double)p.h.y + (double)p.l.y;
+            };
+            const PP2 p0 = payoff(0);
+            PP2 c = {f2(p0.h.y, p0.h.y), f2(p0.l.y, p0.l.y)}, Dc{}, D1{};
+#pragma unroll 1
+            for (int kk = 1; kk <= P; ++kk) {
+                const PP2 next = kk < P ? payoff(kk) : PP2{f2(p0.h.x, Hp), f2(p0.l.x, Lp)};
+                const PP2 Dn = pair_diff(c, next);
+                if (kk == 1) D1 = Dn;
+                else source(kk - 1, c, Dc, Dn, pair_diff(Dc, Dn));
+                Dc = Dn;
+                c = next;
+            }
+            const PP2 E = pair_diff(p0, {f2(Hm, 0.f), f2(Lm, 0.f)});
+            const PP2 X = {f2(Dc.h.x, D1.h.y), f2(Dc.l.x, D1.l.y)}, Z = {f2(E.h.x, D1.h.x), f2(E.l.x, D1.l.x)};
+            source(0, p0, X, Z, pair_diff({f2(X.h.x, -X.h.y), f2(X.l.x, -X.l.y)}, Z));
+            // lo to the next node, from both ends of the lane to the pivot
+#pragma unroll
+            for (int kk = 0; kk < P; ++kk) {
+                const PP2 v = payoff(kk);
+                H[kk] = v.h;
+                L[kk] = v.l;
+            }
+            if constexpr (P > 1) {
+                float2 rest = f2(L[0].x, 0.f);
+#pragma unroll
+                for (int kk = P - 1; kk >= 1; --kk) {
+                    const float2 l = add2(rest, L[kk]), h = add2(H[kk], l);
+                    rest = sub2(l, sub2(h, H[kk]));
+                    H[kk] = h;
+                }
+                const float lP = (rest.x + rest.y) + L[0].y, hP = H[0].y + lP;
+                const float last = lP - (hP - H[0].y);
+                H[0].y = hP;
+                if (fabsf(H[1].x) < fabsf(H[1].y)) H[1].x += last;
+                else H[1].y += last;
+            } else {
+                q_low = L[0];  // two nodes a lane: both may lie at the kink
+            }
+            if constexpr (W == 1) __syncwarp();
+            else __syncthreads();
+#pragma unroll
+            for (int kk = 0; kk < P; ++kk) {
+                qt[kk * NL] = H[kk];
+                H[kk] = L[kk] = f2(0.f, 0.f);
+            }
+        }
+
         // factors held in registers for the whole PDE (kReg)
         constexpr int P1 = kReg >= 3 ? P : 1, P2 = kReg >= 2 ? P : 1, P3 = kReg >= 1 ? P : 1;
         float2 r1[P1];
@@ -805,31 +924,7 @@ __global__ void __launch_bounds__(32 * W, budget(M, W, kUni, kPair).warps / W)
 
         if (run) {
             for (int step = 1; step < TL; ++step) {
-                // V of the neighbours: node -1 and node M
-                const float2 last = P > 1 ? f2(H[P - 1].y, L[P - 1].y) : f2(H[0].y, L[0].y);
-                float Hm = __shfl_up_sync(kAll, last.x, 1), Lm = __shfl_up_sync(kAll, last.y, 1);
-                float Hp = __shfl_down_sync(kAll, H[0].x, 1), Lp = __shfl_down_sync(kAll, L[0].x, 1);
-                if constexpr (W > 1) {
-                    if (k == 0) {
-                        xe[4 * warp] = H[0].x;
-                        xe[4 * warp + 1] = L[0].x;
-                    }
-                    if (k == 31) {
-                        xe[4 * warp + 2] = last.x;
-                        xe[4 * warp + 3] = last.y;
-                    }
-                    __syncthreads();
-                    if (k == 0 && warp > 0) {
-                        Hm = xe[4 * warp - 2];
-                        Lm = xe[4 * warp - 1];
-                    }
-                    if (k == 31 && warp < W - 1) {
-                        Hp = xe[4 * warp + 4];
-                        Lp = xe[4 * warp + 5];
-                    }
-                }
-                if (K == 0) Hm = Lm = 0.f;
-                if (K == NL - 1) Hp = Lp = 0.f;
+                neighbours();
                 phase_edge<kEdge>();
 
                 // D_k = V of slot k-1 minus V of slot k (the pivot in both components before slot
@@ -841,7 +936,7 @@ __global__ void __launch_bounds__(32 * W, budget(M, W, kUni, kPair).warps / W)
                 float2 y[P];
                 float s1, um;
                 if constexpr (!kPair) {
-                    // the residual dt A V, then V += B^-1 of it
+                    // the residual dt A X + q, then X += B^-1 of it
                     float2 h1, l1;
                     diff(1, h1, l1);
                     float2 hc = h1, lc = l1, dc = add2(h1, l1);
@@ -851,7 +946,7 @@ __global__ void __launch_bounds__(32 * W, budget(M, W, kUni, kPair).warps / W)
                         diff(kk + 1, hn, ln);
                         coef_h(kk, A, B);
                         const float2 dn = add2(hn, ln), S = add2(sub2(hc, hn), sub2(lc, ln));
-                        const float2 r = fma2(coef_s(kk), S, mul2(gh, add2(H[kk], L[kk])));
+                        const float2 r = fma2(coef_s(kk), S, fma2(gh, add2(H[kk], L[kk]), qt[kk * NL]));
                         y[kk] = fma2(B, dn, fma2(A, dc, r));
                         hc = hn;
                         lc = ln;
@@ -861,7 +956,8 @@ __global__ void __launch_bounds__(32 * W, budget(M, W, kUni, kPair).warps / W)
                     coef_h(0, A, B);
                     const float eh = H[0].x - Hm, el = L[0].x - Lm;
                     const float2 S = f2((hc.x - eh) + (lc.x - el), -(h1.y + h1.x) - (l1.y + l1.x));
-                    const float2 r = fma2(coef_s(0), S, mul2(gh, add2(H[0], L[0])));
+                    float2 r = fma2(coef_s(0), S, fma2(gh, add2(H[0], L[0]), qt[0]));
+                    if constexpr (P == 1) r = add2(r, q_low);
                     y[0] = fma2(B, f2(eh + el, h1.x + l1.x), fma2(A, f2(dc.x, h1.y + l1.y), r));
                     solve(y, 0, s1, um);
                     phase_edge<kEdge>();
@@ -960,12 +1056,12 @@ __global__ void __launch_bounds__(32 * W, budget(M, W, kUni, kPair).warps / W)
             if constexpr (W > 1) fin = __syncthreads_and(fin) != 0;
         }
         if (fin) {
-            double* V = vout + shape_row(sh, pde);
 #pragma unroll
             for (int kk = 0; kk < P; ++kk) {
                 const int na = j0 + (kk == 0 ? 0 : P - kk), nb = j0 + P + kk;
-                if (na < N) V[na] = (double)H[kk].x + (double)L[kk].x;
-                if (nb < N) V[nb] = (double)H[kk].y + (double)L[kk].y;
+                const double va = (double)H[kk].x + (double)L[kk].x, vb = (double)H[kk].y + (double)L[kk].y;
+                if (na >= 0) V[na] = kPair ? va : V[na] + va;
+                if (nb >= 0) V[nb] = kPair ? vb : V[nb] + vb;
             }
         }
         if (K == 0) {
@@ -973,7 +1069,9 @@ __global__ void __launch_bounds__(32 * W, budget(M, W, kUni, kPair).warps / W)
             if constexpr (kPair)
                 if (!fin && !bad) rescue[atomicAdd(&counters[2], 1)] = pde;
         }
-        if constexpr (!kPair && W > 1) __syncthreads();  // the tables are rewritten for the next PDE
+        // the tables are rewritten for the next PDE
+        if constexpr (!kPair && W > 1) __syncthreads();
+        else __syncwarp();
     }
 }
 
