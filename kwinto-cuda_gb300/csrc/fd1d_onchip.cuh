@@ -154,15 +154,15 @@ __device__ __forceinline__ Split split(double v)
 // the tables moved -> now (8192 PDEs of 512 and 1024 nodes, 16384 of 256 and 128, 4096 of 2048;
 // 512 steps, FP32 at 2048 nodes 1024):
 //                          FP32 stepping       pair arithmetic (255 steps at 1024 and 2048 nodes)
-//   M = 32 uniform         4.57 -> 3.95        6.79           (FP32: 12 warps at 168 registers, 8 at 236)
+//   M = 32 uniform         4.57 -> 3.95        6.79 -> 5.76   (12 warps at 168 registers, 8 at 236)
 //   M = 16 uniform, W = 1  2.41 -> 2.03        5.84 -> 5.66
-//   M = 16 uniform, W = 2                      6.65
+//   M = 16 uniform, W = 2                      6.65 -> 6.21
 //   M = 16, W = 1          2.94 -> 2.51        6.57 -> 6.41
-//   M = 16, W = 2          7.33 -> 5.95        7.60 -> 7.57
+//   M = 16, W = 2          7.33 -> 5.95        7.60 -> 7.43
 //   M = 16, W = 4          18.3 -> 13.4        8.74 -> 7.99
 //   M = 8 uniform          2.43 -> 2.07        6.16 -> 5.97
 //   M = 8                  2.89 -> 2.26        6.49 -> 6.12
-//   M = 4 uniform          1.54 -> 1.31        3.60
+//   M = 4 uniform          1.54 -> 1.31        3.60 -> 3.55
 struct Budget {
     int warps, tables;
     bool edges;
@@ -177,9 +177,10 @@ __host__ __device__ constexpr Budget budget(int M, int W, bool uni, bool pair)
         if (M == 2) return uni ? Budget{16, 1, false} : Budget{20, 2, false};
         return {M == 8 && !uni ? 16 : 20, 3, false};
     }
-    if (M == 32) return {8, 0, true};
-    if (M == 16 && uni) return W == 1 ? Budget{10, 2, true} : Budget{12, 0, true};
-    if (M == 16) return W == 1 ? Budget{8, 3, false} : W == 2 ? Budget{12, 1, true} : Budget{10, 2, true};
+    if (M == 32) return {12, 0, true};
+    if (M == 16 && uni) return W == 1 ? Budget{10, 2, true} : Budget{16, 0, false};
+    if (M == 16) return W == 1 ? Budget{8, 3, false} : W == 2 ? Budget{10, 1, false} : Budget{10, 2, true};
+    if (M == 4 && (uni || W == 4)) return {16, W == 4 ? 2 : 1, false};
     return {16, 3, M == 8};
 }
 
