@@ -75,8 +75,8 @@ namespace {
 // 1024-node grids with tables per node and on 2048-node uniform ones, four on 2048-node grids
 // with tables per node; twice as many while every warp still has a scheduler to itself (the
 // rule of fd1d_pair64.cu).  Measured, ms with 1/2/4 warps (512 steps): 128 PDEs of 512 nodes
-// 0.32/0.27/0.24; 8192 PDEs of 1024 nodes, density 0.25, 6.86/5.96/6.56, uniform
-// 3.95/4.52/5.83; 4096 PDEs of 2048 nodes -/8.95/7.49, uniform -/4.36/4.75.
+// 0.32/0.24/0.20; 8192 PDEs of 1024 nodes, density 0.25, 6.86/5.77/6.14, uniform
+// 3.95/4.6/5.8; 4096 PDEs of 2048 nodes -/8.55/7.09, uniform -/4.27/4.73.
 int fp32_warps(int m1, bool uni, int m, int sms)
 {
     int w = m1 == 64 ? (uni ? 2 : 4) : m1 == 32 && !uni ? 2 : 1;

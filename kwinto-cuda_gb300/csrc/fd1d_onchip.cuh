@@ -125,6 +125,30 @@ __device__ __forceinline__ void ff_acc2(float2& h, float2& l, float2 d)
     h = s;
 }
 
+// (h, l) += 2 u + 2 e for pairs, renormalised.
+__device__ __forceinline__ void pair_acc2(float2& h, float2& l, float2 u, float2 e)
+{
+    float2 s, r;
+    two_sum(h, add2(u, u), s, r);
+    const float2 t = fma2(f2(2.f, 2.f), e, add2(l, r));
+    h = add2(s, t);
+    l = sub2(t, sub2(h, s));
+}
+
+// (h, l) = max((h, l), (ph, pl))
+__device__ __forceinline__ void floor_to(float2 ph, float2 pl, float2& h, float2& l)
+{
+    const float2 d = add2(sub2(h, ph), sub2(l, pl));
+    if (d.x < 0.f) {
+        h.x = ph.x;
+        l.x = pl.x;
+    }
+    if (d.y < 0.f) {
+        h.y = ph.y;
+        l.y = pl.y;
+    }
+}
+
 // 1 / d by Newton's method in its cubic form, r (1 + e + e^2) with e = 1 - d r, from the
 // hardware's 20-bit estimate: the error left is e^3 ~ 2^-60, then rounding.  Zero and
 // non-finite d give a non-finite result.
@@ -158,11 +182,12 @@ __device__ __forceinline__ Split split(double v)
 //   M = 16 uniform, W = 1  2.41 -> 2.03        5.84 -> 5.66
 //   M = 16 uniform, W = 2                      6.65 -> 6.21
 //   M = 16, W = 1          2.94 -> 2.51        6.57 -> 6.41
-//   M = 16, W = 2          7.33 -> 5.95        7.60 -> 7.43
-//   M = 16, W = 4          18.3 -> 13.4        8.74 -> 7.99
+//   M = 16, W = 2          7.33 -> 5.77        7.60 -> 7.43
+//   M = 16, W = 4          18.3 -> 12.7        8.74 -> 7.96
 //   M = 8 uniform          2.43 -> 2.07        6.16 -> 5.97
 //   M = 8                  2.89 -> 2.26        6.49 -> 6.12
 //   M = 4 uniform          1.54 -> 1.31        3.60 -> 3.55
+//   M = 4                  1.33 -> 1.32        3.66 -> 3.51
 struct Budget {
     int warps, tables;
     bool edges;
@@ -171,17 +196,18 @@ __host__ __device__ constexpr Budget budget(int M, int W, bool uni, bool pair)
 {
     if (!pair) {
         if (M == 32) return uni ? Budget{12, 0, W == 1} : Budget{8, 1, W == 2};
-        if (M == 16 && uni) return W == 1 ? Budget{12, 2, true} : Budget{20, 0, W == 2};
-        if (M == 16) return W == 1 ? Budget{10, 2, true} : W == 2 ? Budget{12, 2, true} : Budget{10, 3, false};
-        if (W > 1) return M == 8 ? (W == 2 ? Budget{10, 3, true} : Budget{16, 3, false}) : Budget{12, 3, false};
+        if (M == 16 && uni) return W == 1 ? Budget{12, 2, true} : Budget{16, 0, true};
+        if (M == 16) return W == 1 ? Budget{10, 2, true} : W == 2 ? Budget{10, 1, false} : Budget{10, 3, false};
+        if (W > 1) return M == 8 ? (W == 2 ? Budget{12, 3, true} : Budget{16, 3, false}) : Budget{12, 3, false};
         if (M == 2) return uni ? Budget{16, 1, false} : Budget{20, 2, false};
         return {M == 8 && !uni ? 16 : 20, 3, false};
     }
     if (M == 32) return {12, 0, true};
     if (M == 16 && uni) return W == 1 ? Budget{10, 2, true} : Budget{16, 0, false};
-    if (M == 16) return W == 1 ? Budget{8, 3, false} : W == 2 ? Budget{10, 1, false} : Budget{10, 2, true};
-    if (M == 4 && (uni || W == 4)) return {16, W == 4 ? 2 : 1, false};
-    return {16, 3, M == 8};
+    if (M == 16) return W == 1 ? Budget{8, 3, false} : W == 2 ? Budget{10, 1, false} : Budget{10, 2, false};
+    if (M == 8) return {W == 2 ? 12 : 16, 3, true};
+    if (M == 4) return W > 1 || uni ? Budget{16, 1, false} : Budget{20, 3, true};
+    return {16, 3, false};
 }
 
 // Shared-memory layout of one PDE group (floats).  P = M / 2 slots, NL = 32 W lanes.
@@ -228,6 +254,7 @@ __global__ void __launch_bounds__(32 * W, budget(M, W, kUni, kPair).warps / W)
     using Y = Lay<M, kUni, W, kPair>;
     constexpr bool kEdge = budget(M, W, kUni, kPair).edges;
     constexpr int kReg = budget(M, W, kUni, kPair).tables;
+    constexpr bool kOwn = W > 1 && (!kPair || M <= 8);  // every lane steps its two neighbour nodes itself
     constexpr int P = Y::P, NL = Y::NL, kStride = Y::kStride;
     static_assert(M >= 2 && M % 2 == 0, "as many rows above the pivot as below");
     extern __shared__ __align__(16) float tab[];
@@ -664,15 +691,7 @@ __global__ void __launch_bounds__(32 * W, budget(M, W, kUni, kPair).warps / W)
         auto floor_at = [&](int kk, float2& h, float2& l) {
             if constexpr (kPair) {
                 const float4 p = PPt[kk * NL];
-                const float2 d = add2(sub2(h, f2(p.x, p.y)), sub2(l, f2(p.z, p.w)));
-                if (d.x < 0.f) {
-                    h.x = p.x;
-                    l.x = p.z;
-                }
-                if (d.y < 0.f) {
-                    h.y = p.y;
-                    l.y = p.w;
-                }
+                floor_to(f2(p.x, p.y), f2(p.z, p.w), h, l);
             } else {
                 if (h.x < 0.f) h.x = l.x = 0.f;
                 if (h.y < 0.f && (kk < P - 1 || K < NL - 1)) h.y = l.y = 0.f;  // not on the last node
@@ -716,14 +735,17 @@ __global__ void __launch_bounds__(32 * W, budget(M, W, kUni, kPair).warps / W)
             }
         };
         auto coef_s = [&](int kk) { return kUni && kk > 0 && kk < P - 1 ? cAl : C1t[crow(kk) * NL]; };
-        // state of the nodes beside the lane's: node -1 and node M
-        float Hm, Lm, Hp, Lp;
+        // State of the nodes beside the lane's, -1 and M.  With one warp per PDE it comes from
+        // the neighbours at the start of a step; with more, that would be one more barrier per step, so
+        // every lane steps these two nodes as well, by the operations of their owners.  FP32
+        // stepping: 128 PDEs of 512 nodes 0.240 -> 0.204 ms, 4096 of 2048 7.49 -> 7.09; pair arithmetic: 12
+        // PDEs of 512 nodes 0.452 -> 0.430, but 4096 of 2048 uniform nodes 6.21 -> 6.46, where the two
+        // nodes cost more than the barrier (kOwn).
+        float2 Hn, Ln;
         auto neighbours = [&]() {
             const float2 last = P > 1 ? f2(H[P - 1].y, L[P - 1].y) : f2(H[0].y, L[0].y);
-            Hm = __shfl_up_sync(kAll, last.x, 1);
-            Lm = __shfl_up_sync(kAll, last.y, 1);
-            Hp = __shfl_down_sync(kAll, H[0].x, 1);
-            Lp = __shfl_down_sync(kAll, L[0].x, 1);
+            Hn = f2(__shfl_up_sync(kAll, last.x, 1), __shfl_down_sync(kAll, H[0].x, 1));
+            Ln = f2(__shfl_up_sync(kAll, last.y, 1), __shfl_down_sync(kAll, L[0].x, 1));
             if constexpr (W > 1) {
                 if (k == 0) {
                     xe[4 * warp] = H[0].x;
@@ -735,16 +757,16 @@ __global__ void __launch_bounds__(32 * W, budget(M, W, kUni, kPair).warps / W)
                 }
                 __syncthreads();
                 if (k == 0 && warp > 0) {
-                    Hm = xe[4 * warp - 2];
-                    Lm = xe[4 * warp - 1];
+                    Hn.x = xe[4 * warp - 2];
+                    Ln.x = xe[4 * warp - 1];
                 }
                 if (k == 31 && warp < W - 1) {
-                    Hp = xe[4 * warp + 4];
-                    Lp = xe[4 * warp + 5];
+                    Hn.y = xe[4 * warp + 4];
+                    Ln.y = xe[4 * warp + 5];
                 }
             }
-            if (K == 0) Hm = Lm = 0.f;
-            if (K == NL - 1) Hp = Lp = 0.f;
+            if (K == 0) Hn.x = Ln.x = 0.f;
+            if (K == NL - 1) Hn.y = Ln.y = 0.f;
         };
 
         // FP32 stepping carries X = V - p (fd1d_fp32.cu).  X starts at zero; the payoff waits in
@@ -788,14 +810,14 @@ __global__ void __launch_bounds__(32 * W, budget(M, W, kUni, kPair).warps / W)
             PP2 c = {f2(p0.h.y, p0.h.y), f2(p0.l.y, p0.l.y)}, Dc{}, D1{};
 #pragma unroll 1
             for (int kk = 1; kk <= P; ++kk) {
-                const PP2 next = kk < P ? payoff(kk) : PP2{f2(p0.h.x, Hp), f2(p0.l.x, Lp)};
+                const PP2 next = kk < P ? payoff(kk) : PP2{f2(p0.h.x, Hn.y), f2(p0.l.x, Ln.y)};
                 const PP2 Dn = pair_diff(c, next);
                 if (kk == 1) D1 = Dn;
                 else source(kk - 1, c, Dc, Dn, pair_diff(Dc, Dn));
                 Dc = Dn;
                 c = next;
             }
-            const PP2 E = pair_diff(p0, {f2(Hm, 0.f), f2(Lm, 0.f)});
+            const PP2 E = pair_diff(p0, {f2(Hn.x, 0.f), f2(Ln.x, 0.f)});
             const PP2 X = {f2(Dc.h.x, D1.h.y), f2(Dc.l.x, D1.l.y)}, Z = {f2(E.h.x, D1.h.x), f2(E.l.x, D1.l.x)};
             source(0, p0, X, Z, pair_diff({f2(X.h.x, -X.h.y), f2(X.l.x, -X.l.y)}, Z));
             // lo to the next node, from both ends of the lane to the pivot
@@ -828,7 +850,10 @@ __global__ void __launch_bounds__(32 * W, budget(M, W, kUni, kPair).warps / W)
                 qt[kk * NL] = H[kk];
                 H[kk] = L[kk] = f2(0.f, 0.f);
             }
+            Hn = Ln = f2(0.f, 0.f);
         }
+        if (kPair && kOwn && run) neighbours();
+        const float2 pHn = Hn, pLn = Ln;  // pairs: the payoffs at the two nodes
 
         // factors held in registers for the whole PDE (kReg)
         constexpr int P1 = kReg >= 3 ? P : 1, P2 = kReg >= 2 ? P : 1, P3 = kReg >= 1 ? P : 1;
@@ -907,7 +932,7 @@ __global__ void __launch_bounds__(32 * W, budget(M, W, kUni, kPair).warps / W)
                 s1 = __shfl_down_sync(kAll, s, 1);
                 if (k == 31) s1 = Sr;
                 // the previous warp's last node, by the operations its owner uses below
-                if constexpr (kPair) um = fmaf(-a_, sr_m, fmaf(-bl_, sl_m, yl));
+                if constexpr (kPair || kOwn) um = fmaf(-a_, sr_m, fmaf(-bl_, sl_m, yl));
             }
             const float2 ms = f2(-s, -s), ms1 = f2(-s1, -s1);
 #pragma unroll
@@ -916,7 +941,7 @@ __global__ void __launch_bounds__(32 * W, budget(M, W, kUni, kPair).warps / W)
                 y[kk] = fma2(ms1, f2(q.z, q.w), fma2(ms, f2(q.x, q.y), y[kk]));
             }
             y[0] = f2(s, fmaf(-s1, p3.w, fmaf(-s, p3.y, yP)));
-            if constexpr (kPair) {
+            if constexpr (kPair || kOwn) {
                 const float last = __shfl_up_sync(kAll, P > 1 ? y[P - 1].y : y[0].y, 1);
                 if (k > 0) um = last;
                 if (K == 0) um = 0.f;
@@ -925,14 +950,14 @@ __global__ void __launch_bounds__(32 * W, budget(M, W, kUni, kPair).warps / W)
 
         if (run) {
             for (int step = 1; step < TL; ++step) {
-                neighbours();
+                if constexpr (!kOwn) neighbours();
                 phase_edge<kEdge>();
 
                 // D_k = V of slot k-1 minus V of slot k (the pivot in both components before slot
                 // 1, nodes 0 and M after slot P-1), high and low parts each exact
                 auto diff = [&](int kk, float2& dh, float2& dl) {
-                    dh = sub2(kk == 1 ? f2(H[0].y, H[0].y) : H[kk - 1], kk == P ? f2(H[0].x, Hp) : H[kk]);
-                    dl = sub2(kk == 1 ? f2(L[0].y, L[0].y) : L[kk - 1], kk == P ? f2(L[0].x, Lp) : L[kk]);
+                    dh = sub2(kk == 1 ? f2(H[0].y, H[0].y) : H[kk - 1], kk == P ? f2(H[0].x, Hn.y) : H[kk]);
+                    dl = sub2(kk == 1 ? f2(L[0].y, L[0].y) : L[kk - 1], kk == P ? f2(L[0].x, Ln.y) : L[kk]);
                 };
                 float2 y[P];
                 float s1, um;
@@ -955,17 +980,24 @@ __global__ void __launch_bounds__(32 * W, budget(M, W, kUni, kPair).warps / W)
                     }
                     float2 A, B;
                     coef_h(0, A, B);
-                    const float eh = H[0].x - Hm, el = L[0].x - Lm;
+                    const float eh = H[0].x - Hn.x, el = L[0].x - Ln.x;
                     const float2 S = f2((hc.x - eh) + (lc.x - el), -(h1.y + h1.x) - (l1.y + l1.x));
                     float2 r = fma2(coef_s(0), S, fma2(gh, add2(H[0], L[0]), qt[0]));
                     if constexpr (P == 1) r = add2(r, q_low);
                     y[0] = fma2(B, f2(eh + el, h1.x + l1.x), fma2(A, f2(dc.x, h1.y + l1.y), r));
-                    solve(y, 0, s1, um);
+                    solve(y, kOwn ? step & 1 : 0, s1, um);
                     phase_edge<kEdge>();
 #pragma unroll
                     for (int kk = 0; kk < P; ++kk) {
                         ff_acc2(H[kk], L[kk], y[kk]);
                         if (amer) floor_at(kk, H[kk], L[kk]);
+                    }
+                    if constexpr (kOwn) {
+                        ff_acc2(Hn, Ln, f2(um, s1));
+                        if (amer) {
+                            if (Hn.x < 0.f) Hn.x = Ln.x = 0.f;
+                            if (Hn.y < 0.f) Hn.y = Ln.y = 0.f;
+                        }
                     }
                 } else {
                     // 1. u0 = B^-1 A' V in FP32.  D_k = V of slot k-1 minus V of slot k (the pivot
@@ -977,8 +1009,8 @@ __global__ void __launch_bounds__(32 * W, budget(M, W, kUni, kPair).warps / W)
                         for (int kk = 1; kk <= P; ++kk) {
                             const float2 hu = kk == 1 ? f2(H[0].y, H[0].y) : H[kk - 1];
                             const float2 lu = kk == 1 ? f2(L[0].y, L[0].y) : L[kk - 1];
-                            const float2 hd = kk == P ? f2(H[0].x, Hp) : H[kk];
-                            const float2 ld = kk == P ? f2(L[0].x, Lp) : L[kk];
+                            const float2 hd = kk == P ? f2(H[0].x, Hn.y) : H[kk];
+                            const float2 ld = kk == P ? f2(L[0].x, Ln.y) : L[kk];
                             const float2 Dn = add2(sub2(hu, hd), sub2(lu, ld));
                             if (kk == 1) {
                                 D1 = Dn;
@@ -991,17 +1023,19 @@ __global__ void __launch_bounds__(32 * W, budget(M, W, kUni, kPair).warps / W)
                         }
                         float2 A, B;
                         coef_h(0, A, B);
-                        const float E = (H[0].x - Hm) + (L[0].x - Lm);
+                        const float E = (H[0].x - Hn.x) + (L[0].x - Ln.x);
                         y[0] = fma2(A, f2(Dc.x, D1.y), fma2(neg(B), f2(E, D1.x), mul2(gh, H[0])));
                     }
                     solve(y, 0, s1, um);
+
+                    const float2 un = f2(um, s1);
 
                     // 2., 3. W = V + u0 and r = A' W - u0
                     float2 u0[P];
                     phase_edge<kEdge>();
                     {
                         const PP2 w0 = shifted(H[0], L[0], y[0]);
-                        const PP2 wn = shifted(f2(Hm, Hp), f2(Lm, Lp), f2(um, s1));  // nodes -1 and M
+                        const PP2 wn = shifted(Hn, Ln, un);  // nodes -1 and M
                         PP2 wc = {f2(w0.h.y, w0.h.y), f2(w0.l.y, w0.l.y)};           // slot k-1
                         u0[0] = y[0];
                         PP2 Dc{}, D1{};
@@ -1038,12 +1072,12 @@ __global__ void __launch_bounds__(32 * W, budget(M, W, kUni, kPair).warps / W)
                     phase_edge<kEdge>();
 #pragma unroll
                     for (int kk = 0; kk < P; ++kk) {
-                        float2 s, e;
-                        two_sum(H[kk], add2(u0[kk], u0[kk]), s, e);
-                        const float2 l = fma2(f2(2.f, 2.f), y[kk], add2(L[kk], e));
-                        H[kk] = add2(s, l);
-                        L[kk] = sub2(l, sub2(H[kk], s));
+                        pair_acc2(H[kk], L[kk], u0[kk], y[kk]);
                         if (amer) floor_at(kk, H[kk], L[kk]);
+                    }
+                    if constexpr (kOwn) {
+                        pair_acc2(Hn, Ln, un, f2(um, s1));
+                        if (amer) floor_to(pHn, pLn, Hn, Ln);
                     }
                 }
             }
