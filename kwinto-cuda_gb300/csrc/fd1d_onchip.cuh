@@ -178,15 +178,15 @@ __device__ __forceinline__ Split split(double v)
 // the tables moved -> now (8192 PDEs of 512 and 1024 nodes, 16384 of 256 and 128, 4096 of 2048;
 // 512 steps, FP32 at 2048 nodes 1024):
 //                          FP32 stepping       pair arithmetic (255 steps at 1024 and 2048 nodes)
-//   M = 32 uniform         4.57 -> 3.95        6.79 -> 5.76   (12 warps at 168 registers, 8 at 236)
-//   M = 16 uniform, W = 1  2.41 -> 2.03        5.84 -> 5.66
-//   M = 16 uniform, W = 2                      6.65 -> 6.21
+//   M = 32 uniform         4.57 -> 3.86        6.79 -> 5.61   (12 warps at 168 registers, 8 at 236)
+//   M = 16 uniform, W = 1  2.41 -> 1.96        5.84 -> 5.56
+//   M = 16 uniform, W = 2                      6.65 -> 6.15
 //   M = 16, W = 1          2.94 -> 2.51        6.57 -> 6.41
 //   M = 16, W = 2          7.33 -> 5.77        7.60 -> 7.43
 //   M = 16, W = 4          18.3 -> 12.7        8.74 -> 7.96
-//   M = 8 uniform          2.43 -> 2.07        6.16 -> 5.97
+//   M = 8 uniform          2.43 -> 2.01        6.16 -> 5.85
 //   M = 8                  2.89 -> 2.26        6.49 -> 6.12
-//   M = 4 uniform          1.54 -> 1.31        3.60 -> 3.55
+//   M = 4 uniform          1.54 -> 1.27        3.60 -> 3.52
 //   M = 4                  1.33 -> 1.32        3.66 -> 3.51
 struct Budget {
     int warps, tables;
@@ -206,8 +206,8 @@ __host__ __device__ constexpr Budget budget(int M, int W, bool uni, bool pair)
     if (M == 16 && uni) return W == 1 ? Budget{10, 2, true} : Budget{16, 0, false};
     if (M == 16) return W == 1 ? Budget{8, 3, false} : W == 2 ? Budget{10, 1, false} : Budget{10, 2, false};
     if (M == 8) return {W == 2 ? 12 : 16, 3, true};
-    if (M == 4) return W > 1 || uni ? Budget{16, 1, false} : Budget{20, 3, true};
-    return {16, 3, false};
+    if (M == 4) return W > 1 ? Budget{10, 3, false} : uni ? Budget{16, 3, false} : Budget{20, 3, true};
+    return {16, 3, true};
 }
 
 // Shared-memory layout of one PDE group (floats).  P = M / 2 slots, NL = 32 W lanes.
@@ -329,7 +329,7 @@ __global__ void __launch_bounds__(32 * W, budget(M, W, kUni, kPair).warps / W)
         // A walk over consecutive nodes.  Sinh grids: sinh and cosh of y_j by the addition
         // formula, with the spacing d (sinh y_(j+1) - sinh y_j) free of cancellation; where
         // the step is coarse a walk would carry the rounding of large values to the middle of
-        // the grid, and every node is evaluated.  Uniform grids: s = y_j, c = e^(y_j).
+        // the grid, and every node is evaluated.  Uniform grids: s = y_j.
         struct Walk {
             double s, c, dx;  // dx: the spacing just crossed
         };
@@ -345,13 +345,13 @@ __global__ void __launch_bounds__(32 * W, budget(M, W, kUni, kPair).warps / W)
         auto y_at = [&](int j) { return fma((double)j, step, -yend); };
         auto walk_at = [&](int j) -> Walk {
             const double y = y_at(j);
-            if (uniform) return {y, exp(y), step};
+            if (uniform) return {y, 0., step};
             const double sy = sinh(y);
             return {sy, sqrt(fma(sy, sy, 1.)), 0.};
         };
         const bool coarse = step > 0.125;
         auto up = [&](const Walk& v, int j) -> Walk {  // to node j from j - 1
-            if (uniform) return {y_at(j), mul(v.c, s1_), step};
+            if (uniform) return {y_at(j), 0., step};
             if (coarse) {
                 const double sy = sinh(y_at(j));
                 return {sy, 0., mul(sh.density, sub(sy, v.s))};
@@ -360,7 +360,7 @@ __global__ void __launch_bounds__(32 * W, budget(M, W, kUni, kPair).warps / W)
             return {add(v.s, ds), add(v.c, fma(v.c, c1_, mul(v.s, s1_))), mul(sh.density, ds)};
         };
         auto down = [&](const Walk& v, int j) -> Walk {  // to node j from j + 1
-            if (uniform) return {y_at(j), mul(v.c, c1_), step};
+            if (uniform) return {y_at(j), 0., step};
             if (coarse) {
                 const double sy = sinh(y_at(j));
                 return {sy, 0., mul(sh.density, sub(v.s, sy))};
@@ -390,36 +390,51 @@ __global__ void __launch_bounds__(32 * W, budget(M, W, kUni, kPair).warps / W)
             const double drift = mul(ax_d, im), lower = mul(mul(axx_d, id), im);
             return {(float)lower, (float)add(fma(mul(axx_d, iu), im, -lower), drift), (float)drift};
         };
-        auto store = [&](int i, double x, double ex, double al, double be, double iu, double im, double id) {
-            const int j = j0 + i, s = slot_of(i), c = comp_of(i);
-            double p = 0.;
-            if (j >= 0 && ((w < 0) ? (x < 0.) : (x > 0.))) {
-                if (!uniform) ex = exp(x);
-                p = fmax(0., (w < 0) ? sub(1., ex) : sub(ex, 1.));
-            }
-            const Split ph = split(p);
-            part(PPt[s * NL], c) = ph.h;
-            part(PPt[s * NL], 2 + c) = ph.l;
-            if (!kUni || i == 0 || i == P || i == 1 || i == M - 1) {
-                const int r = crow(s);
-                if constexpr (kPair) {
-                    const Split sa = split(al), sb = split(be);
-                    const bool swap = c == 1 && i != P;
-                    const float sg = i == P ? -1.f : 1.f;
-                    part(Cht[r * NL], c) = swap ? sb.h : sg * sa.h;
-                    part(Cht[r * NL], 2 + c) = swap ? sa.h : sb.h;
-                    part(Clt[r * NL], c) = swap ? sb.l : sg * sa.l;
-                    part(Clt[r * NL], 2 + c) = swap ? sa.l : sb.l;
-                } else {
-                    // the increments' right-hand side c1 S + c2 D+ + c3 D- + c4 V (S = D+ - D-)
-                    const Inc q = increments(j, iu, im, id);
-                    const bool swap = c == 1 && i != P;
-                    part(Cht[r * NL], c) = i == P ? -q.c2 : swap ? -q.c3 : q.c2;
-                    part(Cht[r * NL], 2 + c) = i == P ? q.c3 : swap ? -q.c2 : q.c3;
-                    reinterpret_cast<float*>(&C1t[r * NL])[c] = q.c1;
-                }
+        auto store_coef = [&](int i, double al, double be, double iu, double im, double id) {
+            const int j = j0 + i, s = slot_of(i), c = comp_of(i), r = crow(s);
+            if constexpr (kPair) {
+                const Split sa = split(al), sb = split(be);
+                const bool swap = c == 1 && i != P;
+                const float sg = i == P ? -1.f : 1.f;
+                part(Cht[r * NL], c) = swap ? sb.h : sg * sa.h;
+                part(Cht[r * NL], 2 + c) = swap ? sa.h : sb.h;
+                part(Clt[r * NL], c) = swap ? sb.l : sg * sa.l;
+                part(Clt[r * NL], 2 + c) = swap ? sa.l : sb.l;
+            } else {
+                // the increments' right-hand side c1 S + c2 D+ + c3 D- + c4 V (S = D+ - D-)
+                const Inc q = increments(j, iu, im, id);
+                const bool swap = c == 1 && i != P;
+                part(Cht[r * NL], c) = i == P ? -q.c2 : swap ? -q.c3 : q.c2;
+                part(Cht[r * NL], 2 + c) = i == P ? q.c3 : swap ? -q.c2 : q.c3;
+                reinterpret_cast<float*>(&C1t[r * NL])[c] = q.c1;
             }
             if (kPair) fit = fit && fabs(al) < kMaxValue && fabs(be) < kMaxValue;
+        };
+        const double sw = w < 0 ? -1. : 1.;
+        auto payoff = [&](double ex) { return split(fmax(0., fma(sw, ex, -sw))); };
+        if (uniform) {
+            // from the pivot outwards, e^x carried from node to node
+            auto real = [&](int i, const Split& p) { return kUni || j0 + i >= 0 ? p : Split{0.f, 0.f}; };
+            const double eP = exp(y_at(j0 + P));
+            double ea = eP, eb = eP;
+#pragma unroll 1
+            for (int kk = 1; kk < P; ++kk) {
+                ea = mul(ea, c1_);
+                eb = mul(eb, s1_);
+                const Split pa = real(P - kk, payoff(ea)), pb = real(P + kk, payoff(eb));
+                PPt[kk * NL] = make_float4(pa.h, pb.h, pa.l, pb.l);
+            }
+            const Split p0 = real(0, payoff(mul(ea, c1_))), pP = real(P, payoff(eP));
+            PPt[0] = make_float4(p0.h, pP.h, p0.l, pP.l);
+        }
+        auto store = [&](int i, double x, double al, double be, double iu, double im, double id) {
+            const int j = j0 + i, s = slot_of(i), c = comp_of(i);
+            if (!uniform) {
+                const Split p = j >= 0 && ((w < 0) ? (x < 0.) : (x > 0.)) ? payoff(exp(x)) : Split{0.f, 0.f};
+                part(PPt[s * NL], c) = p.h;
+                part(PPt[s * NL], 2 + c) = p.l;
+            }
+            if (!kUni || i == 0 || i == P || i == 1 || i == M - 1) store_coef(i, al, be, iu, im, id);
         };
         // Rows of B: bl = -beta, b = 1 + alpha + beta - gamma, bu = -alpha.  The interior block
         // is eliminated from both ends: l, 1/d, u = bu/d above the pivot, m, 1/e, bl/e below.
@@ -427,12 +442,89 @@ __global__ void __launch_bounds__(32 * W, budget(M, W, kUni, kPair).warps / W)
         // R = B_I^-1 (bu_(M-1) e_(M-1)) in FP64 (it nearly cancels on fine grids).
         double b_sep = 1., bl_sep = 0., bu_sep = 0., bl_first = 0., bu_last = 0.;
         double L1 = 0., Llast = 0., R1 = 0., Rlast = 0.;
-        {
+        if constexpr (kUni && P > 1) {
+            // Constant rows: the chains from both ends of a lane are the same, 1/d_k with
+            // d_(k+1) = b - a c / d_k (a = bl, c = bu), and so are the spikes' sums up to
+            // factors; only the last lane's descending chain differs, by its first row.  That lane
+            // runs its own chain and takes the ascending one's results from lane 0.  17 FP64
+            // operations per node instead of 42: 8192 PDEs of 1024 nodes set up in 0.44 ms instead of
+            // 0.78 (pair arithmetic; 0.50 instead of 0.79 in FP32 stepping, 22 and 84 steps' worth).
+            const bool first = K == 0, end = K == NL - 1;
+            const double al = alpha_of(1, iu_u, im_u), be = beta_of(1, im_u, iu_u), edge = mul(ax_t, iu_u);
+            const double ca = -be, cc = -al, cb = sub(add(1., add(al, be)), gamma);
+            const double al0 = first ? edge : al, be0 = first ? 0. : be;
+            bl_sep = -be0;
+            bu_sep = -al0;
+            b_sep = sub(add(1., add(al0, be0)), gamma);
+            bl_first = ca;
+            bu_last = end ? 0. : cc;
+            store_coef(0, al0, be0, iu_u, im_u, iu_u);
+            store_coef(P, al, be, iu_u, im_u, iu_u);
+            store_coef(1, al, be, iu_u, im_u, iu_u);
+            store_coef(M - 1, end ? 0. : al, end ? -edge : be, iu_u, im_u, iu_u);
+            // the chain
+            double r = 0., ar = 0., cr = 0., A = 1., C = 1., sig = 0.;
+            double d = end ? sub(add(1., -edge), gamma) : cb, link = end ? edge : ca;
+#pragma unroll 1
+            for (int kk = P - 1; kk >= 1; --kk) {
+                const float l = (float)ar, m = (float)cr;
+                r = rcp(d);
+                fit = fit && isfinite(r);
+                ar = mul(link, r);
+                cr = mul(cc, r);
+                d = fma(-mul(cc, link), r, cb);
+                sig = fma(mul(A, C), r, sig);
+                A = mul(A, ar);
+                C = mul(C, cr);
+                const float rf = (float)r, af = (float)ar, cf = (float)cr;
+                if (first) {
+                    T1[kk * kStride] = f2(l, m);
+                    T2[kk * kStride] = make_float4(rf, rf, cf, af);
+                    T1[kk * kStride + 1].x = l;
+                    T2[kk * kStride + 1].x = rf;
+                    T2[kk * kStride + 1].z = cf;
+                } else if (end) {
+                    T1[kk * kStride].y = m;
+                    T2[kk * kStride].y = rf;
+                    T2[kk * kStride].w = af;
+                }
+                if (kk > 1) link = ca;
+            }
+            const double mP = cr;  // bu / d of the descending chain
+            {
+                const double A_ = __shfl_sync(kAll, A, 0), C_ = __shfl_sync(kAll, C, 0), s_ = __shfl_sync(kAll, sig, 0),
+                             l_ = __shfl_sync(kAll, ar, 0), d_ = __shfl_sync(kAll, d, 0);
+                if (end) {
+                    A = A_;
+                    C = C_;
+                    sig = s_;
+                    ar = l_;
+                    d = d_;
+                }
+            }
+            const double ig = rcp(fma(-mP, link, d));
+            fit = fit && isfinite(ig);
+            if (writer) {
+                tL(P) = (float)ar;
+                set_iu(P, ig, mP);
+            }
+            const double xl = -mul(mul(ca, A), ig), xr = end ? 0. : -mul(mul(cc, C), ig);
+            L1 = fma(-C, xl, mul(ca, sig));
+            R1 = -mul(C, xr);
+            Llast = -mul(A, xl);
+            Rlast = end ? 0. : fma(-A, xr, mul(cc, sig));
+            if constexpr (W == 1) __syncwarp();
+            else __syncthreads();
+        } else {
             Walk wa = up(walk_at(j0 - 1), j0), wd = down(walk_at(j0 + M), j0 + M - 1);
             // the spacings behind each walk and their reciprocals
             double da = wa.dx, dd = wd.dx, ida = uniform ? iu_u : rcp(da), iud = uniform ? iu_u : rcp(dd);
-            double idp = 1., bup = 0., fa = 0., pua = 1., suma = 0.;  // ascending: 1/d, bu, f, prod(-u), sum
-            double iep = 1., blp = 0., fd = 0., pud = 1., sumd = 0.;  // descending
+            // ascending: 1/d, bu, products of the l and of the u, sum; descending likewise.  A row takes
+            // bl bu / d of the row before it, the same product in either direction, and the first
+            // row's coupling comes in at the end, so that constant rows give what the chain
+            // above does, bit for bit.
+            double idp = 1., bup = 0., fa = 1., pua = 1., suma = 0.;
+            double iep = 1., blp = 0., fd = 1., pud = 1., sumd = 0.;
             double bP = 1., buP = 0., lP = 0.;
 #pragma unroll 1
             for (int i = 0; i <= P; ++i) {
@@ -450,7 +542,7 @@ __global__ void __launch_bounds__(32 * W, budget(M, W, kUni, kPair).warps / W)
                         be = beta_of(j, im, ida);
                         bb = sub(add(1., add(al, be)), gamma);
                     }
-                    store(i, x_of(wa), wa.c, al, be, iu, im, ida);
+                    store(i, x_of(wa), al, be, iu, im, ida);
                     if (i == 0) {
                         bl_sep = -be;
                         b_sep = bb;
@@ -458,8 +550,8 @@ __global__ void __launch_bounds__(32 * W, budget(M, W, kUni, kPair).warps / W)
                     } else {
                         if (i == 1) bl_first = -be;
                         const double l = i == 1 ? 0. : -mul(be, idp);
-                        const double d = fma(-l, bup, bb);
-                        fa = i == 1 ? -be : -mul(l, fa);
+                        const double d = fma(mul(be, bup), idp, bb);
+                        if (i > 1) fa = mul(l, fa);
                         if (i < P) {
                             const double r = rcp(d), u = -mul(al, r);
                             fit = fit && isfinite(r);
@@ -468,7 +560,7 @@ __global__ void __launch_bounds__(32 * W, budget(M, W, kUni, kPair).warps / W)
                                 set_iu(i, r, u);
                             }
                             suma = fma(mul(pua, fa), r, suma);
-                            pua = -mul(pua, u);
+                            pua = mul(pua, u);
                             idp = r;
                             bup = -al;
                         } else {
@@ -495,18 +587,18 @@ __global__ void __launch_bounds__(32 * W, budget(M, W, kUni, kPair).warps / W)
                         be = beta_of(j, im, idn);
                         bb = sub(add(1., add(al, be)), gamma);
                     }
-                    store(id_, x_of(wd), wd.c, al, be, iud, im, idn);
+                    store(id_, x_of(wd), al, be, iud, im, idn);
                     if (i == 1) bu_last = -al;
                     const double m = i == 1 ? 0. : -mul(al, iep);
-                    const double r = rcp(fma(-m, blp, bb)), u = -mul(be, r);
+                    const double r = rcp(fma(mul(al, blp), iep, bb)), u = -mul(be, r);
                     fit = fit && isfinite(r);
-                    fd = i == 1 ? -al : -mul(m, fd);
+                    if (i > 1) fd = mul(m, fd);
                     if (writer) {
                         tL(id_) = (float)m;
                         set_iu(id_, r, u);
                     }
                     sumd = fma(mul(pud, fd), r, sumd);
-                    pud = -mul(pud, u);
+                    pud = mul(pud, u);
                     iep = r;
                     blp = -be;
                     dd = wn.dx;
@@ -519,16 +611,18 @@ __global__ void __launch_bounds__(32 * W, budget(M, W, kUni, kPair).warps / W)
             const double ig = rcp(fma(-mP, blp, bP));
             fit = fit && isfinite(ig);
             if (P == 1) bu_last = buP;
-            fd = P > 1 ? -mul(mP, fd) : buP;
+            if (P > 1) fd = mul(mP, fd);
             if (writer) {
                 tL(P) = (float)lP;
                 set_iu(P, ig, mP);
             }
-            const double xl = mul(fa, ig), xr = mul(fd, ig);  // the spikes at the pivot
-            L1 = fma(pua, xl, suma);
-            Llast = mul(pud, xl);
-            R1 = mul(pua, xr);
-            Rlast = fma(pud, xr, sumd);
+            // the spikes at the pivot; P - 1 sign changes, P even or 1
+            const double sg = P > 1 ? -1. : 1.;
+            const double xl = sg * mul(mul(bl_first, fa), ig), xr = sg * mul(mul(bu_last, fd), ig);
+            L1 = fma(sg * pua, xl, mul(bl_first, suma));
+            Llast = mul(sg * pud, xl);
+            R1 = mul(sg * pua, xr);
+            Rlast = fma(sg * pud, xr, mul(bu_last, sumd));
         }
         if (writer) {
             // spikes L = B_I^-1 (bl_1 e_1), R = B_I^-1 (bu_(M-1) e_(M-1)) by the steps' own solve
