@@ -43,9 +43,11 @@ inline uint64_t host_key_hash(const kwg_option& o, int32_t x_dim, int32_t t_dim)
 
 // Fills asset2pde (n entries) and pde2asset (the first option of each distinct key)
 // and returns the number of PDEs.  x_dims, t_dims: per-option grid shape of an
-// uneven batch, or nullptr.
+// uneven batch, or nullptr.  idx: the n options are opts[idx[0]], opts[idx[1]], ... (and
+// pde2asset holds such numbers), or nullptr for all of them in order.
 inline size_t dedup_host(const kwg_option* opts, size_t n, const int32_t* x_dims, const int32_t* t_dims,
-                         std::vector<int32_t>& asset2pde, std::vector<uint32_t>& pde2asset)
+                         std::vector<int32_t>& asset2pde, std::vector<uint32_t>& pde2asset,
+                         const uint32_t* idx = nullptr)
 {
     size_t cap = 16;
     while (cap < 2 * n) cap <<= 1;
@@ -55,15 +57,16 @@ inline size_t dedup_host(const kwg_option* opts, size_t n, const int32_t* x_dims
     pde2asset.clear();
     pde2asset.reserve(n);
     for (size_t i = 0; i < n; ++i) {
-        const kwg_option& o = opts[i];
-        const int32_t xi = x_dims ? x_dims[i] : 0, ti = t_dims ? t_dims[i] : 0;
+        const size_t at = idx ? idx[i] : i;
+        const kwg_option& o = opts[at];
+        const int32_t xi = x_dims ? x_dims[at] : 0, ti = t_dims ? t_dims[at] : 0;
         size_t h = host_key_hash(o, xi, ti) & mask;
         for (;;) {
             const int32_t p = table[h];
             if (p < 0) {
                 table[h] = (int32_t)pde2asset.size();
                 asset2pde[i] = table[h];
-                pde2asset.push_back((uint32_t)i);
+                pde2asset.push_back((uint32_t)at);
                 break;
             }
             const uint32_t a = pde2asset[p];
@@ -86,7 +89,10 @@ inline size_t dedup_host(const kwg_option* opts, size_t n, const int32_t* x_dims
 inline void radix_sort_pairs(std::vector<std::pair<uint64_t, uint32_t>>& kv)
 {
     const size_t m = kv.size();
-    if (m < 2) return;
+    if (m < 2048) {  // clearing the counters would cost more
+        std::sort(kv.begin(), kv.end());
+        return;
+    }
     uint64_t all_or = 0, all_and = ~0ull;
     for (const auto& e : kv) {
         all_or |= e.first;

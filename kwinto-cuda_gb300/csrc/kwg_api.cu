@@ -586,6 +586,12 @@ void kwg_destroy(kwg_ctx* ctx)
     if (ctx->d_counter) cudaFree(ctx->d_counter);
     if (ctx->h_io) cudaFreeHost(ctx->h_io);
     if (ctx->graph_exec) cudaGraphExecDestroy(ctx->graph_exec);
+    for (auto& b : ctx->buckets) {
+        if (b.stream) cudaStreamDestroy(b.stream);
+        if (b.d_work) cudaFree(b.d_work);
+        if (b.d_io) cudaFree(b.d_io);
+        if (b.h_io) cudaFreeHost(b.h_io);
+    }
     for (auto& e : ctx->events) {
         cudaEventDestroy(e.start);
         cudaEventDestroy(e.stop);

@@ -29,8 +29,16 @@ struct kwg_ctx {
     // pinned host staging
     void* h_io = nullptr;
     size_t h_io_bytes = 0;
-    // solve-kernel timing (kwg_set_profiling)
-    // uneven batches: the captured device sequence and the layout it was built for
+    // uneven batches, warp-per-PDE solvers: stream and grow-only buffers of each nodes-per-lane
+    // bucket (2 to 64), which prepare, solve and copy independently
+    struct Bucket {
+        cudaStream_t stream = nullptr;
+        void *d_io = nullptr, *d_work = nullptr, *h_io = nullptr;
+        size_t io_bytes = 0, work_bytes = 0, h_io_bytes = 0;
+    };
+    Bucket buckets[6];
+    // uneven batches, thread per option: the captured device sequence and the layout it was
+    // built for
     cudaGraphExec_t graph_exec = nullptr;
     uint64_t graph_sig = 0;
     int graph_launches = 0;
@@ -44,6 +52,7 @@ struct kwg_ctx {
         int sm_blocks = 0;
     };
     std::map<uint64_t, Tuned> tuned;
+    // solve-kernel timing (kwg_set_profiling)
     bool profiling = false;
     std::vector<kwg::SolveEvents> events;  // pool, reused across reads
     size_t events_used = 0;

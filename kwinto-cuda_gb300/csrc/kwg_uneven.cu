@@ -9,17 +9,17 @@
 //   * FP64 (thread per option): PDEs of equal x_dim are packed 32 to a tile, sorted
 //     by t_dim so that the lanes of a tile finish together, and all tiles run in ONE
 //     persistent launch whose queue hands out the longest tiles first; each lane
-//     steps its own t_dim - 1 times;
-//   * warp-per-option solvers (FP32, or FP64 with KWG_SOLVER_PCR): one launch per
-//     nodes-per-lane bucket, each PDE with its own x_dim and t_dim;
-//   * the device sequence (H2D copy, kernels, D2H copy) is captured once into a CUDA
-//     graph and replayed while the batch layout stays the same.
+//     steps its own t_dim - 1 times.  The device sequence (H2D copy, kernels, D2H copy) is
+//     captured once into a CUDA graph and replayed while the batch layout stays the same;
+//   * warp-per-PDE solvers (FP32, FP64 in pair arithmetic, or KWG_SOLVER_PCR): the options
+//     are split into one bucket per nodes-per-lane count, and every bucket is prepared, solved and
+//     copied on a stream of its own, the heaviest first (price_buckets).
 #include <algorithm>
 #include <cstdint>
 #include <cstdio>
 #include <cstring>
+#include <new>
 #include <numeric>
-#include <tuple>
 #include <vector>
 
 #include <cuda_runtime.h>
@@ -69,6 +69,184 @@ UnevenLayout uneven_layout(size_t m, size_t n, size_t ntiles)
     return L;
 }
 
+// Warp-per-PDE solvers.  Preparing a batch (dedup, sort by work, packing) takes the host ~85 ns per
+// option: 11 of the 52 ms of 131072 options in FP32 when the whole batch was prepared before
+// the first kernel, and the solves of the buckets waited for one another's last PDEs.  By buckets, all but the
+// first one's preparation hides behind the device, and a bucket's tail behind the
+// next one's start: 42.8 ms (FP64: 143.9 -> 129.9).  With profiling on all run on the context's stream, one after
+// the other.
+int price_buckets(kwg_ctx* ctx, const kwg_option* opts, const int32_t* x_dims, const int32_t* t_dims, size_t n,
+                  const kwg_fd1d_params& q, const kwg_ctx::Tuned& tn, bool pair, double* prices, int32_t* status)
+{
+    constexpr int kBuckets = sizeof(ctx->buckets) / sizeof(ctx->buckets[0]);
+    auto mlane = [&](int x) {
+        return q.precision == KWG_FP32 || pair ? kwg::fd1d_fp32_nodes_per_lane(x) : kwg::fd1d_pcr64_nodes_per_lane(x);
+    };
+    // options by bucket, in the caller's order within one
+    struct Part {
+        size_t begin = 0, end = 0, at = 0;
+        uint64_t work = 0;
+        UnevenLayout L;
+    } part[kBuckets];
+    std::vector<uint8_t> id(n);
+    for (size_t i = 0; i < n; ++i) {
+        const int M = mlane(x_dims[i]);
+        int b = 0;
+        while (b < kBuckets - 1 && (2 << b) < M) ++b;
+        if (M < 0) return set_err(ctx, KWG_ERR_INVALID, "kwg: grid too large for the chosen solver");
+        id[i] = (uint8_t)b;
+        ++part[b].end;
+        part[b].work += (uint64_t)x_dims[i] * (uint64_t)(t_dims[i] - 1);
+    }
+    size_t off = 0;
+    for (Part& p : part) {
+        p.begin = p.at = off;
+        off = p.end += off;
+    }
+    std::vector<uint32_t> order(n);
+    for (size_t i = 0; i < n; ++i) order[part[id[i]].at++] = (uint32_t)i;
+    int by_work[kBuckets];
+    std::iota(by_work, by_work + kBuckets, 0);
+    std::stable_sort(by_work, by_work + kBuckets, [&](int a, int b) { return part[a].work > part[b].work; });
+
+    std::vector<int32_t> asset2pde, pde_slot;
+    std::vector<uint32_t> pde2asset;
+    std::vector<std::pair<uint64_t, uint32_t>> kv;
+    auto prepare = [&](int bi) -> int {
+        const Part& p = part[bi];
+        kwg_ctx::Bucket& bk = ctx->buckets[bi];
+        const uint32_t* const idx = order.data() + p.begin;
+        const size_t nb = p.end - p.begin;
+        const size_t m = kwg::dedup_host(opts, nb, x_dims, t_dims, asset2pde, pde2asset, idx);
+        // node-steps descending (x_dim <= 2048 here, so node-steps < 2^43), ties by PDE number
+        kv.resize(m);
+        int x_max = 0, x_min = INT32_MAX;
+        long long nodes = 0;
+        for (size_t i = 0; i < m; ++i) {
+            const int x = x_dims[pde2asset[i]];
+            kv[i] = {((1ull << 50) - 1) - (uint64_t)x * (uint64_t)(t_dims[pde2asset[i]] - 1), (uint32_t)i};
+            x_max = std::max(x_max, x);
+            x_min = std::min(x_min, x);
+            nodes += x;
+        }
+        kwg::radix_sort_pairs(kv);
+        UnevenLayout& L = part[bi].L;
+        L = uneven_layout(m, nb, 0);
+        const size_t counters = align_up(L.total, 256), wbytes = pair ? kwg::fd1d_pair64_work_bytes((int)m, nodes)
+                                                                      : (size_t)nodes * sizeof(double);
+        if (int rc = ensure_host(ctx, &bk.h_io, &bk.h_io_bytes, L.total)) return rc;
+        if (int rc = ensure_device(ctx, &bk.d_io, &bk.io_bytes, counters + 4 * sizeof(int))) return rc;
+        if (int rc = ensure_device(ctx, &bk.d_work, &bk.work_bytes, wbytes)) return rc;
+        if (!bk.stream) KWG_CUDA(ctx, cudaStreamCreateWithFlags(&bk.stream, cudaStreamNonBlocking));
+        char *h = (char*)bk.h_io, *io = (char*)bk.d_io;
+        pde_slot.resize(m);
+        long long row = 0;
+        for (size_t sl = 0; sl < m; ++sl) {
+            const uint32_t at = pde2asset[kv[sl].second];
+            const kwg_option& o = opts[at];
+            pde_slot[kv[sl].second] = (int32_t)sl;
+            ((double*)(h + L.t))[sl] = o.t;
+            ((double*)(h + L.z))[sl] = o.z;
+            ((double*)(h + L.r))[sl] = o.r;
+            ((double*)(h + L.q))[sl] = o.q;
+            ((int32_t*)(h + L.px))[sl] = x_dims[at];
+            ((int32_t*)(h + L.pt))[sl] = t_dims[at];
+            ((int8_t*)(h + L.w))[sl] = o.w;
+            ((uint8_t*)(h + L.e))[sl] = o.e;
+            ((long long*)(h + L.rows))[sl] = row;
+            row += x_dims[at];
+        }
+        for (size_t i = 0; i < nb; ++i) {
+            ((double*)(h + L.s))[i] = opts[idx[i]].s;
+            ((double*)(h + L.k))[i] = opts[idx[i]].k;
+            ((int32_t*)(h + L.pde))[i] = pde_slot[asset2pde[i]];
+        }
+        kwg::PdeBatch b;
+        b.t = (const double*)(io + L.t);
+        b.z = (const double*)(io + L.z);
+        b.r = (const double*)(io + L.r);
+        b.q = (const double*)(io + L.q);
+        b.w = (const int8_t*)(io + L.w);
+        b.e = (const uint8_t*)(io + L.e);
+        b.m = b.m_pad = (int)m;
+        kwg::AssetBatch a;
+        a.s = (const double*)(io + L.s);
+        a.k = (const double*)(io + L.k);
+        a.pde = (const int32_t*)(io + L.pde);
+        a.n = (int)nb;
+        kwg::Fd1dShape sh = make_shape(&q);
+        sh.x_dim = x_max;
+        sh.block_warps = tn.block_warps;
+        sh.option_warps = tn.option_warps;
+        sh.sm_blocks = tn.sm_blocks;
+        sh.pde_x = (const int32_t*)(io + L.px);
+        sh.pde_t = (const int32_t*)(io + L.pt);
+        sh.row_off = (const long long*)(io + L.rows);
+        sh.full_lanes = x_min == kwg::kTile * mlane(x_max);  // all fill the lanes
+        double *v = (double*)bk.d_work, *d_prices = (double*)(io + L.prices);
+        int32_t *d_status = (int32_t*)(io + L.status), *d_pde_status = (int32_t*)(io + L.pde_status);
+        int* const d_counters = (int*)(io + counters);
+        const cudaStream_t st = ctx->profiling ? ctx->stream : bk.stream;
+        KWG_CUDA(ctx, cudaMemcpyAsync(io, h, L.in_bytes, cudaMemcpyHostToDevice, st));
+        const kwg::SolveEvents* ev = ctx->next_events();
+        const int r =
+            pair ? kwg::fd1d_pair64_launch(b, a, sh, v, (int32_t*)(v + nodes), d_pde_status, d_counters, d_prices,
+                                           d_status, ctx->device, st, ev)
+            : q.precision == KWG_FP32 ? kwg::fd1d_fp32_launch(b, a, sh, v, d_pde_status, d_counters, d_prices,
+                                                              d_status, ctx->device, st, ev)
+                                      : kwg::fd1d_pcr64_launch(b, a, sh, v, d_pde_status, d_counters, d_prices,
+                                                               d_status, ctx->device, st, ev);
+        if (r < 0) return set_err(ctx, KWG_ERR_INVALID, "kwg: grid too large for the chosen solver");
+        ctx->launches += r;
+        KWG_CUDA(ctx, cudaGetLastError());
+        KWG_CUDA(ctx, cudaMemcpyAsync(h + L.prices, io + L.prices, L.out_bytes, cudaMemcpyDeviceToHost, st));
+        return KWG_OK;
+    };
+
+    int rc = KWG_OK;
+    for (int bi : by_work) {
+        if (rc == KWG_OK && part[bi].end > part[bi].begin) {
+            try {
+                rc = prepare(bi);
+            } catch (const std::bad_alloc&) {  // buckets in flight are drained below
+                rc = set_err(ctx, KWG_ERR_INVALID, "kwg: out of host memory");
+            }
+        }
+    }
+    // results, bucket by bucket while later ones run; after an error the streams are drained
+    for (int bi : by_work) {
+        const Part& p = part[bi];
+        kwg_ctx::Bucket& bk = ctx->buckets[bi];
+        if (p.end == p.begin || !bk.stream) continue;
+        const cudaError_t e = cudaStreamSynchronize(ctx->profiling ? ctx->stream : bk.stream);
+        if (rc != KWG_OK) continue;
+        if (e != cudaSuccess) {
+            rc = cuda_err(ctx, e, "kwg: uneven batch");
+            continue;
+        }
+        const double* hp = (const double*)((char*)bk.h_io + p.L.prices);
+        const int32_t* hs = (const int32_t*)((char*)bk.h_io + p.L.status);
+        for (size_t i = p.begin; i < p.end; ++i) {
+            prices[order[i]] = hp[i - p.begin];
+            status[order[i]] = hs[i - p.begin];
+        }
+    }
+    return rc;
+}
+
+// Strict mode: the first asset without a price is an error.
+int check_strict(kwg_ctx* ctx, const int32_t* status, size_t n)
+{
+    for (size_t i = 0; i < n; ++i) {
+        if (status[i] == KWG_STATUS_OK) continue;
+        char msg[256];
+        std::snprintf(msg, sizeof msg, "Fd1dGpu_Pricer::price: asset %zu: %s", i,
+                      status[i] == KWG_STATUS_OUT_OF_GRID ? "not in grid range" : "failed");
+        return set_err(ctx, status[i] == KWG_STATUS_OUT_OF_GRID ? KWG_ERR_OUT_OF_GRID : KWG_ERR_SOLVER, msg);
+    }
+    return KWG_OK;
+}
+
 uint64_t mix(uint64_t h, uint64_t v)
 {
     h ^= v + 0x9e3779b97f4a7c15ull + (h << 6) + (h >> 2);
@@ -105,8 +283,8 @@ extern "C" int kwg_fd1d_price_uneven(kwg_ctx* ctx, const kwg_option* opts, const
     q.t_dim = t_max;
     if (int rc = check_params(ctx, &q)) return rc;
     // launch choices: the explicit ones, else what kwg_autotune_uneven recorded for
-    // uneven batches of this precision and size, else Thomas with one warp per block
-    // (FP64) and one warp per option (FP32)
+    // uneven batches of this precision and size, else the on-chip solvers with warps by the
+    // bucket's size, or (theta != 1/2, more than 2048 nodes) Thomas with one warp per block
     kwg_ctx::Tuned tn;
     if (q.precision == KWG_FP64 && q.solver == KWG_SOLVER_AUTO && pair64_ok(&q)) tn.solver = KWG_SOLVER_PCR;
     {
@@ -126,6 +304,15 @@ extern "C" int kwg_fd1d_price_uneven(kwg_ctx* ctx, const kwg_option* opts, const
     const bool pcr = q.precision == KWG_FP32 || q.solver == KWG_SOLVER_PCR;
     const bool pair = q.solver == KWG_SOLVER_PCR && pair64_ok(&q);
     KWG_CUDA(ctx, cudaSetDevice(ctx->device));
+    if (pcr) {
+        std::vector<int32_t> own;
+        if (!status) {
+            own.resize(n);
+            status = own.data();
+        }
+        const int rc = price_buckets(ctx, opts, x_dims, t_dims, n, q, tn, pair, prices, status);
+        return rc == KWG_OK && p->strict ? check_strict(ctx, status, n) : rc;
+    }
 
     // 1. dedup by (t, r, q, z, e, w, x_dim, t_dim)
     std::vector<int32_t> asset2pde;
@@ -134,14 +321,10 @@ extern "C" int kwg_fd1d_price_uneven(kwg_ctx* ctx, const kwg_option* opts, const
     auto xd = [&](size_t pde) { return x_dims[pde2asset[pde]]; };
     auto td = [&](size_t pde) { return t_dims[pde2asset[pde]]; };
 
-    // 2. layout: slot order and (Thomas) tiles or (PCR) nodes-per-lane buckets
-    std::vector<uint32_t> slot_pde;          // slot -> PDE (replicas pad Thomas tiles)
+    // 2. layout: slot order and tiles
+    std::vector<uint32_t> slot_pde;          // slot -> PDE (replicas pad tiles)
     std::vector<int32_t> pde_slot(m, -1);    // PDE -> its first slot
     std::vector<kwg::TileDesc> tiles;
-    std::vector<long long> rows;
-    std::vector<std::pair<int, int>> buckets;  // PCR: [begin, end) slot ranges per bucket
-    std::vector<int> bucket_x;
-    std::vector<bool> bucket_full;
     long long node_lanes = 0;
     // PDEs in layout order: sorted on one packed integer key per PDE (ties by PDE
     // number, so the layout is deterministic)
@@ -152,74 +335,40 @@ extern "C" int kwg_fd1d_price_uneven(kwg_ctx* ctx, const kwg_option* opts, const
         kwg::radix_sort_pairs(kv);
         for (size_t i = 0; i < m; ++i) by[i] = kv[i].second;
     };
-    if (!pcr) {
-        // x_dim ascending, t_dim descending
-        sort_by([&](uint32_t p) { return (uint64_t)(uint32_t)xd(p) << 32 | (uint32_t)(INT32_MAX - td(p)); });
-        struct Chunk {
-            size_t begin, count;
-            int x, tmax;
-        };
-        std::vector<Chunk> chunks;
-        for (size_t i = 0; i < m;) {
-            size_t j = i;
-            while (j < m && xd(by[j]) == xd(by[i])) ++j;
-            for (size_t c = i; c < j; c += kwg::kTile) {
-                const size_t cnt = std::min((size_t)kwg::kTile, j - c);
-                chunks.push_back({c, cnt, xd(by[c]), td(by[c])});  // sorted: first has the largest t_dim
-            }
-            i = j;
+    // x_dim ascending, t_dim descending
+    sort_by([&](uint32_t p) { return (uint64_t)(uint32_t)xd(p) << 32 | (uint32_t)(INT32_MAX - td(p)); });
+    struct Chunk {
+        size_t begin, count;
+        int x, tmax;
+    };
+    std::vector<Chunk> chunks;
+    for (size_t i = 0; i < m;) {
+        size_t j = i;
+        while (j < m && xd(by[j]) == xd(by[i])) ++j;
+        for (size_t c = i; c < j; c += kwg::kTile) {
+            const size_t cnt = std::min((size_t)kwg::kTile, j - c);
+            chunks.push_back({c, cnt, xd(by[c]), td(by[c])});  // sorted: first has the largest t_dim
         }
-        std::stable_sort(chunks.begin(), chunks.end(), [](const Chunk& a, const Chunk& b) {
-            return (long long)a.x * (a.tmax - 1) > (long long)b.x * (b.tmax - 1);
-        });
-        for (const Chunk& c : chunks) {
-            tiles.push_back(kwg::TileDesc{c.x, c.tmax, node_lanes});
-            node_lanes += (long long)kwg::kTile * c.x;
-            for (int l = 0; l < kwg::kTile; ++l) {
-                const uint32_t pde = by[c.begin + std::min((size_t)l, c.count - 1)];
-                if (pde_slot[pde] < 0) pde_slot[pde] = (int32_t)slot_pde.size();
-                slot_pde.push_back(pde);
-            }
-        }
-    } else {
-        auto mlane = [&](uint32_t pde) {
-            return q.precision == KWG_FP32 || pair ? kwg::fd1d_fp32_nodes_per_lane(xd(pde))
-                                           : kwg::fd1d_pcr64_nodes_per_lane(xd(pde));
-        };
-        // nodes per lane ascending, node-steps descending (x_dim <= 2048 here, so
-        // node-steps < 2^43)
-        sort_by([&](uint32_t p) {
-            const uint64_t work = (uint64_t)xd(p) * (uint64_t)(td(p) > 1 ? td(p) - 1 : 0);
-            return (uint64_t)(mlane(p) + 1) << 50 | (((1ull << 50) - 1) - work);
-        });
-        long long off = 0;
-        for (size_t i = 0; i < m; ++i) {
-            const uint32_t pde = by[i];
-            pde_slot[pde] = (int32_t)i;
+        i = j;
+    }
+    std::stable_sort(chunks.begin(), chunks.end(), [](const Chunk& a, const Chunk& b) {
+        return (long long)a.x * (a.tmax - 1) > (long long)b.x * (b.tmax - 1);
+    });
+    for (const Chunk& c : chunks) {
+        tiles.push_back(kwg::TileDesc{c.x, c.tmax, node_lanes});
+        node_lanes += (long long)kwg::kTile * c.x;
+        for (int l = 0; l < kwg::kTile; ++l) {
+            const uint32_t pde = by[c.begin + std::min((size_t)l, c.count - 1)];
+            if (pde_slot[pde] < 0) pde_slot[pde] = (int32_t)slot_pde.size();
             slot_pde.push_back(pde);
-            rows.push_back(off);
-            off += xd(pde);
-            const bool full = (int)xd(pde) == kwg::kTile * mlane(pde);
-            if (i == 0 || mlane(pde) != mlane(by[i - 1])) {
-                buckets.push_back({(int)i, (int)i + 1});
-                bucket_x.push_back(xd(pde));
-                bucket_full.push_back(full);
-            } else {
-                buckets.back().second = (int)i + 1;
-                bucket_x.back() = std::max(bucket_x.back(), (int)xd(pde));
-                bucket_full.back() = bucket_full.back() && full;
-            }
         }
-        node_lanes = off;  // rows of final values, in doubles
     }
     const size_t ms = slot_pde.size();
 
     // 3. pack inputs into pinned memory
     const UnevenLayout L = uneven_layout(ms, n, tiles.size());
     if (int rc = ensure_host(ctx, &ctx->h_io, &ctx->h_io_bytes, L.total)) return rc;
-    const size_t wbytes = pair  ? kwg::fd1d_pair64_work_bytes((int)ms, node_lanes)
-                          : pcr ? (size_t)node_lanes * sizeof(double)
-                                : kwg::fd1d_fp64_work_bytes_nl((int)ms, node_lanes);
+    const size_t wbytes = kwg::fd1d_fp64_work_bytes_nl((int)ms, node_lanes);
     // the graph bakes in device addresses: grow buffers before deciding on replay
     if (int rc = ensure_device(ctx, &ctx->d_io, &ctx->io_bytes, L.total)) return rc;
     if (int rc = ensure_device(ctx, &ctx->d_work, &ctx->work_bytes, wbytes)) return rc;
@@ -241,7 +390,6 @@ extern "C" int kwg_fd1d_price_uneven(kwg_ctx* ctx, const kwg_option* opts, const
         ((int32_t*)(h + L.pde))[i] = pde_slot[asset2pde[i]];
     }
     if (!tiles.empty()) std::memcpy(h + L.tiles, tiles.data(), tiles.size() * sizeof(kwg::TileDesc));
-    if (!rows.empty()) std::memcpy(h + L.rows, rows.data(), rows.size() * sizeof(long long));
 
     // 4. the device sequence, as a CUDA graph when not profiling
     char* io = (char*)ctx->d_io;
@@ -261,85 +409,35 @@ extern "C" int kwg_fd1d_price_uneven(kwg_ctx* ctx, const kwg_option* opts, const
     a.n = (int)n;
     kwg::Fd1dShape sh = make_shape(&q);
     sh.block_warps = tn.block_warps;
-    sh.option_warps = tn.option_warps;
     sh.sm_blocks = tn.sm_blocks;
     sh.pde_x = (const int32_t*)(io + L.px);
     sh.pde_t = (const int32_t*)(io + L.pt);
-    if (!pcr) {
-        sh.tiles = (const kwg::TileDesc*)(io + L.tiles);
-        sh.node_lanes = node_lanes;
-    } else {
-        sh.row_off = (const long long*)(io + L.rows);
-    }
+    sh.tiles = (const kwg::TileDesc*)(io + L.tiles);
+    sh.node_lanes = node_lanes;
     double* d_prices = (double*)(io + L.prices);
     int32_t* d_status = (int32_t*)(io + L.status);
     int32_t* d_pde_status = (int32_t*)(io + L.pde_status);
 
     auto enqueue = [&](cudaStream_t st) -> int {
-        int launches = 0;
         cudaMemcpyAsync(ctx->d_io, ctx->h_io, L.in_bytes, cudaMemcpyHostToDevice, st);
-        if (!pcr) {
-            const int blocks = kwg::fd1d_fp64_solve_blocks((int)tiles.size(), ctx->device, sh.block_warps,
-                                                         sh.sm_blocks);
-            launches += kwg::fd1d_fp64_launch(b, a, sh, (double*)ctx->d_work, d_pde_status, ctx->d_counter, d_prices,
-                                              d_status, blocks, st, ctx->next_events());
-        } else {
-            for (size_t bi = 0; bi < buckets.size(); ++bi) {
-                const int beg = buckets[bi].first, end = buckets[bi].second;
-                kwg::PdeBatch sb = b;
-                sb.t += beg;
-                sb.z += beg;
-                sb.r += beg;
-                sb.q += beg;
-                sb.w += beg;
-                sb.e += beg;
-                sb.m = sb.m_pad = end - beg;
-                kwg::Fd1dShape ss = sh;
-                ss.x_dim = bucket_x[bi];
-                ss.full_lanes = bucket_full[bi];
-                ss.pde_x += beg;
-                ss.pde_t += beg;
-                ss.row_off += beg;
-                kwg::AssetBatch none = a;
-                none.n = 0;
-                double* v = (double*)ctx->d_work;
-                const int r = pair ? kwg::fd1d_pair64_launch(sb, none, ss, v, (int32_t*)(v + node_lanes) + beg,
-                                                             d_pde_status + beg, ctx->d_counter, d_prices, d_status,
-                                                             ctx->device, st, ctx->next_events())
-                              : q.precision == KWG_FP32
-                                  ? kwg::fd1d_fp32_launch(sb, none, ss, (double*)ctx->d_work, d_pde_status + beg,
-                                                          ctx->d_counter, d_prices, d_status, ctx->device, st,
-                                                          ctx->next_events())
-                                  : kwg::fd1d_pcr64_launch(sb, none, ss, (double*)ctx->d_work, d_pde_status + beg,
-                                                           ctx->d_counter, d_prices, d_status, ctx->device, st,
-                                                           ctx->next_events());
-                if (r < 0) return -1;
-                launches += r;
-            }
-            kwg::fd1d_interp_rows<<<(unsigned)((n + 127) / 128), 128, 0, st>>>(b, a, sh, (double*)ctx->d_work,
-                                                                               d_pde_status, d_prices, d_status);
-            ++launches;
-        }
+        const int blocks =
+            kwg::fd1d_fp64_solve_blocks((int)tiles.size(), ctx->device, sh.block_warps, sh.sm_blocks);
+        const int launches = kwg::fd1d_fp64_launch(b, a, sh, (double*)ctx->d_work, d_pde_status, ctx->d_counter, d_prices,
+                                                   d_status, blocks, st, ctx->next_events());
         cudaMemcpyAsync(h + L.prices, io + L.prices, L.out_bytes, cudaMemcpyDeviceToHost, st);
         return launches;
     };
 
     uint64_t sig = 0x5eed;
-    for (uint64_t v : {(uint64_t)q.precision, (uint64_t)pcr, (uint64_t)pair, (uint64_t)sh.block_warps, (uint64_t)sh.option_warps,
-                       (uint64_t)sh.sm_blocks,
-                       (uint64_t)n, (uint64_t)ms, (uint64_t)tiles.size(),
-                       (uint64_t)node_lanes, (uint64_t)(uintptr_t)ctx->d_io, (uint64_t)(uintptr_t)ctx->d_work,
-                       (uint64_t)(uintptr_t)ctx->h_io})
+    for (uint64_t v : {(uint64_t)q.precision, (uint64_t)sh.block_warps, (uint64_t)sh.sm_blocks, (uint64_t)n, (uint64_t)ms,
+                       (uint64_t)tiles.size(), (uint64_t)node_lanes, (uint64_t)(uintptr_t)ctx->d_io,
+                       (uint64_t)(uintptr_t)ctx->d_work, (uint64_t)(uintptr_t)ctx->h_io})
         sig = mix(sig, v);
     for (double v : {q.theta, q.scale, q.density}) {
         uint64_t u;
         std::memcpy(&u, &v, 8);
         sig = mix(sig, u);
     }
-    for (size_t bi = 0; bi < buckets.size(); ++bi)
-        sig = mix(mix(mix(mix(sig, (uint64_t)buckets[bi].first), (uint64_t)buckets[bi].second), (uint64_t)bucket_x[bi]),
-                  (uint64_t)bucket_full[bi]);
-
     if (ctx->profiling) {
         const int r = enqueue(ctx->stream);
         if (r < 0) return set_err(ctx, KWG_ERR_INVALID, "kwg: grid too large for the chosen solver");
@@ -376,16 +474,7 @@ extern "C" int kwg_fd1d_price_uneven(kwg_ctx* ctx, const kwg_option* opts, const
     const int32_t* hs = (const int32_t*)(h + L.status);
     std::memcpy(prices, hp, n * sizeof(double));
     if (status) std::memcpy(status, hs, n * sizeof(int32_t));
-    if (p->strict) {
-        for (size_t i = 0; i < n; ++i) {
-            if (hs[i] == KWG_STATUS_OK) continue;
-            char msg[256];
-            std::snprintf(msg, sizeof msg, "Fd1dGpu_Pricer::price: asset %zu: %s", i,
-                          hs[i] == KWG_STATUS_OUT_OF_GRID ? "not in grid range" : "failed");
-            return set_err(ctx, hs[i] == KWG_STATUS_OUT_OF_GRID ? KWG_ERR_OUT_OF_GRID : KWG_ERR_SOLVER, msg);
-        }
-    }
-    return KWG_OK;
+    return p->strict ? check_strict(ctx, hs, n) : KWG_OK;
 }
 
 extern "C" int kwg_autotune_uneven(kwg_ctx* ctx, const kwg_option* opts, const int32_t* x_dims,
