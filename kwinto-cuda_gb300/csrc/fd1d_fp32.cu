@@ -73,14 +73,20 @@ namespace {
 
 // Warps per PDE by the batch size: one up to 512 nodes and on 1024-node uniform grids, two on
 // 1024-node grids with tables per node and on 2048-node uniform ones, four on 2048-node grids
-// with tables per node; twice as many while every warp still has a scheduler to itself (the
-// rule of fd1d_pair64.cu).  Measured, ms with 1/2/4 warps (512 steps): 128 PDEs of 512 nodes
-// 0.32/0.24/0.20; 8192 PDEs of 1024 nodes, density 0.25, 6.86/5.77/6.14, uniform
-// 3.95/4.6/5.8; 4096 PDEs of 2048 nodes -/8.55/7.09, uniform -/4.27/4.73.
+// with tables per node; twice as many while every warp still has a scheduler to itself, and
+// from 1024 nodes (512 with tables per node) while they fit 12 to an SM.  Measured, ms with
+// 1/2/4 warps: 256 steps, uniform grids of 512 nodes, 150 PDEs 0.141/0.115/0.104, 300 of them
+// 0.141/0.115/0.130, 600 of them 0.145/0.149/0.196; of 1024 nodes, 300 of them 0.242/0.186/0.166, 600 of
+// them 0.258/0.245/0.270, 900 of them 0.344/0.331/0.393, 1200 of them 0.370/0.422/0.487; 512 nodes at
+// density 0.25, 600 of them 0.206/0.190/0.299; 512 steps, 8192 PDEs of 1024 nodes, density 0.25,
+// 6.86/5.77/6.14, uniform 3.86/4.4/5.8; 4096 PDEs of 2048 nodes -/8.55/6.89, uniform -/4.12/4.72.
 int fp32_warps(int m1, bool uni, int m, int sms)
 {
     int w = m1 == 64 ? (uni ? 2 : 4) : m1 == 32 && !uni ? 2 : 1;
-    while (m1 >= 8 && w < 4 && (long long)m * 2 * w <= 4ll * sms) w *= 2;
+    for (; m1 >= 8 && w < 4; w *= 2) {
+        const bool shared = m1 >= 32 || (m1 == 16 && !uni && w == 1);
+        if ((long long)m * 2 * w > (shared ? 12ll : 4ll) * sms) break;
+    }
     return w;
 }
 

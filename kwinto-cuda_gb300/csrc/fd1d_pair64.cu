@@ -7,11 +7,11 @@
 // (fd1d_fp64.cu) therefore cost 6 scheduler cycles per node; the ~76 FP32 operations here
 // cost 2.4, and their latency is 4 cycles instead of 64.
 //
-// Bound by the FP32 pipe (two thirds busy at 1024 uniform nodes) and, for few PDEs, by the
+// Bound by the FP32 pipe (75 % busy at 1024 uniform nodes) and, for few PDEs, by the
 // latency of the two separator solves per step.  Measured against the FP64 solvers that took
-// these shapes before (whole calls): 32768 PDEs, 1024 x 1024 uniform, 192 -> 93 ms; 8192 PDEs,
+// these shapes before (whole calls): 32768 PDEs, 1024 x 1024 uniform, 192 -> 84 ms; 8192 PDEs,
 // 1024 x 1024, density 0.25, 186 -> 28 ms; 777 PDEs, 1000 x 731, 12.4 -> 2.8 ms; 600 PDEs,
-// 512 x 512, 2.50 -> 0.87 ms; 12 PDEs 2.35 -> 0.52 ms; 131072 uneven PDEs 339 -> 155 ms.
+// 512 x 512, 2.50 -> 0.77 ms; 12 PDEs 2.35 -> 0.46 ms; 131072 uneven PDEs 340 -> 130 ms.
 //
 // Numerics.  The reference step B V' = E V (src/Math/kwFd1d.cpp:61-132) is taken in
 // increments.  With A' = theta dt A and u = theta (V' - V) it reads
@@ -46,15 +46,16 @@ namespace {
 // (more warps repeat the separator solve) -- one up to 1024 nodes, two on 1024-node grids
 // whose tables are per node (45 KB per PDE: five PDEs per SM, so ten warps instead of five),
 // four beyond.  Fewer PDEs: twice the warps while every warp still has a scheduler to
-// itself, up to four (at eight, or below two nodes per lane, the exchange costs more than
-// the shorter chains save).  Measured, ms (512 steps, density 0.25): 12 PDEs of 512 nodes with
-// 1/2/4/8 warps 0.76/0.59/0.50/0.61, 300 of them 0.76/0.62/0.63/0.93, 600 of them
-// 0.82/0.88/1.01; 8192 PDEs of 1024 nodes 18.4/15.0/17.1/28.2, on the uniform grid (1024
-// steps) 24.2/25.1/29.4/51.0.
+// itself, from 1024 nodes while they fit 12 to an SM, up to four (at eight, or below two nodes
+// per lane, the exchange costs more than the shorter chains save).  Measured, ms with 1/2/4
+// warps (256 steps): density 0.25, 150 PDEs of 512 nodes 0.355/0.271/0.228, 300 of them
+// 0.356/0.278/0.293, 450 of them 0.359/0.383/0.377; uniform, 300 of 1024 nodes 0.623/0.424/0.409, 450 of
+// them 0.629/0.568/0.533, 600 of them 0.648/0.582/0.672, 900 of them 0.936/0.793/0.958, 1200 of them
+// 0.963/1.015/1.287; 8192 of 1024 nodes, density 0.25 (512 steps) -/15.0/17.1.
 int pair64_warps(int m1, bool uni, int m, int sms)
 {
     int w = m1 == 64 ? 4 : m1 == 32 && !uni ? 2 : 1;
-    while (m1 >= 8 && w < 4 && (long long)m * 2 * w <= 4ll * sms) w *= 2;
+    while (m1 >= 8 && w < 4 && (long long)m * 2 * w <= (m1 >= 32 ? 12ll : 4ll) * sms) w *= 2;
     return w;
 }
 
