@@ -9,14 +9,17 @@ theta 0.5, scale 5, uniform x-grid, FP64 -- the reference's largest logged shape
 
 Reported on one JSON line (rank 0):
   value      options/s with inputs resident in HBM (kwg_fd1d_price_device), CUDA
-             events on the launching stream, K steps after W warm-up steps; the
-             per-step working set (2.4 GB of coefficients, payoff and state) is far larger
-             than L2, so no flush is needed between steps.
+             events on the launching stream, K steps after W warm-up steps; every
+             step writes 268 MB of final values, more than L2 holds, so no flush is needed
+             between steps.
   e2e        the same metric through the reference-facing call (kwg_fd1d_price: host
              options in, host prices out; dedup, H2D and D2H inside the timing).
-  roofline   of the solve kernel, from its own CUDA events inside the timed region:
-             achieved = 32 B per node-step (the streaming scheme's algorithmic bytes)
-             over the launch time; the kernel's own count of requested bytes beside it.
+  roofline   of the solve kernel, from its own CUDA events inside the timed region.  The
+             autotuner's choice for this shape is the on-chip kernel (FP64 accuracy in
+             pair arithmetic): achieved = its FP32 operations per node-step over the launch
+             time, against the FP32 lanes at the sampled clock.  For the streaming kernel:
+             32 B per node-step (its algorithmic bytes) over the launch time, the
+             kernel's own count of requested bytes beside it.
   variants   FP64 and FP32 rates and their errors against the FP64 oracle.
   cpu_baseline  the oracle (C restatement of the reference, all host cores) on a
              bounded sample of the same workload; its prices are the FP64 parity check
@@ -63,6 +66,12 @@ def node_steps(n, x_dim=None, t_dim=None):
 # and the payoff (8 B) where it is not +0 for the whole tile.  The kernel counts the
 # bytes it requests itself (kwg_profile_read).
 FP64_FLOPS_PER_NODE_STEP = 6  # 3 FMA per node-step at theta = 1/2
+# The on-chip kernel in pair arithmetic: FP32 operations (an add, a multiply or an FMA each) per
+# node and step, counted in csrc/fd1d_onchip.cuh: two tridiagonal solves of 5, the first
+# residual 6, W = V + u 7, its differences 8, the residual in pairs 30, the update 12, the
+# floor 3.  It reads 34 bytes and writes 8 N per PDE.
+PAIR_OPS_PER_NODE_STEP = 76
+FP32_LANES_PER_SM = 128
 ALGO_BYTES_PER_NODE_STEP = 32  # FP64 streaming scheme: V read + write, sweep value write + read
 
 
@@ -70,7 +79,7 @@ def workload_config():
     """The `config` both arms print (same keys and values, so the two lines compare)."""
     return {"workload": WORKLOAD, "options_per_batch": N_OPTIONS, "x_dim": X_DIM, "t_dim": T_DIM, "theta": 0.5,
             "scale": SCALE, "grid": "uniform", "precision": "fp64",
-            "l2": "working set 2.4 GB per step > 129 MB L2 (no flush needed)"}
+            "l2": "each step writes 268 MB of final values > 129 MB L2 (no flush needed)"}
 
 
 CALIBRATION_FILE = os.path.join(ROOT, "oracle", "port_calibration.json")
@@ -408,7 +417,7 @@ def run_ours(args):
     d_status = torch.empty(n_loc, dtype=torch.int32, device=dev)
 
     # ---------------------------------------------------------------- autotuner: launch shapes
-    # options per block and Thomas vs PCR (FP64), threads per option (FP32), on this shape
+    # streaming (options per block) or on chip (FP64), threads per option (FP32), on this shape
     tune64 = ctx.autotune_ex(prm, n_loc).as_dict()
     tune32 = ctx.autotune_ex(kwg.params(t_dim=T_DIM, x_dim=X_DIM, scale=SCALE, density=DENSITY,
                                         precision=kwg.FP32), n_loc).as_dict()
@@ -542,7 +551,7 @@ def run_ours(args):
             p3 = kwg.params(scale=SCALE, density=DENSITY, precision=prec)
             uneven["tuning"][name] = ctx.autotune_uneven(o3, xd3, td3, p3).as_dict()
             for _ in range(max(1, args.warmup)):
-                rc, pr3, st3 = ctx.fd1d_price_uneven(o3, xd3, td3, p3)  # first call captures the graph
+                rc, pr3, st3 = ctx.fd1d_price_uneven(o3, xd3, td3, p3)  # first call allocates
             barrier()
             t0 = time.perf_counter()
             for _ in range(args.steps):
@@ -647,20 +656,51 @@ def run_ours(args):
     fp64_peak = fp64_peak_tflops(dev)
 
     # ---------------------------------------------------------------- roofline (solve kernel)
-    # achieved: the algorithmic bytes of the streaming two-sweep scheme, 32 B per
-    # node-step in FP64 (V read and written, the sweep value written and read back),
-    # over the solve kernel's CUDA-event time.  The kernel's own count of the bytes it
-    # requests (payoff and, outside the frozen middle region, coefficients on top) is
-    # reported beside it as achieved_requested.
     hbm, peak_src = peaks()
     per_launch_s = solve_ms / 1e3 / max(solve_n, 1)
     ns = node_steps(n_loc)
-    algo_bytes = ALGO_BYTES_PER_NODE_STEP * ns
-    achieved = algo_bytes / per_launch_s / 1e9
-    req_bytes = solve_bytes / max(solve_n, 1)
-    achieved_req = req_bytes / per_launch_s / 1e9
-    fp64_tflops = FP64_FLOPS_PER_NODE_STEP * ns / per_launch_s / 1e12
-    traffic = measured_traffic(ns)
+    common = {"node_steps_per_launch": ns, "launch_ms": per_launch_s * 1e3}
+    if tune64["solver"] == "thomas":
+        # achieved: the algorithmic bytes of the streaming two-sweep scheme, 32 B per
+        # node-step in FP64 (V read and written, the sweep value written and read back),
+        # over the solve kernel's CUDA-event time.  The kernel's own count of the bytes it
+        # requests (payoff and, outside the frozen middle region, coefficients on top) is
+        # reported beside it as achieved_requested.
+        algo_bytes = ALGO_BYTES_PER_NODE_STEP * ns
+        req_bytes = solve_bytes / max(solve_n, 1)
+        achieved, traffic = algo_bytes / per_launch_s / 1e9, measured_traffic(ns)
+        fp64_tflops = FP64_FLOPS_PER_NODE_STEP * ns / per_launch_s / 1e12
+        roofline = {"bound": "hbm", "kernel": "fd1d_solve_fp64", "achieved": achieved, "peak": hbm,
+                    "unit": "GB/s", "frac": achieved / hbm, "peak_source": peak_src, "traffic": traffic,
+                    "algorithmic_bytes_per_launch": algo_bytes,
+                    "algorithmic_bytes_per_node_step": ALGO_BYTES_PER_NODE_STEP,
+                    "basis": "32 B per node-step (V read + write, sweep value write + read), FP64 streaming scheme",
+                    "achieved_requested": req_bytes / per_launch_s / 1e9,
+                    "frac_requested": req_bytes / per_launch_s / 1e9 / hbm,
+                    "requested_bytes_per_node_step": req_bytes / ns,
+                    "requested_basis": "bytes the kernel itself requests (state 32 B + payoff 8 B where nonzero "
+                                       "+ coefficients 24 B outside the frozen middle region), counted in the kernel",
+                    "traffic_per_node_step": traffic / ns if traffic else None,
+                    "fp64_tflops": fp64_tflops, "fp64_peak_tflops": fp64_peak,
+                    "fp64_frac": fp64_tflops / fp64_peak if fp64_peak else None,
+                    "fp64_peak_source": "measured here: cuBLAS DGEMM 4096^3", **common}
+    else:
+        # on chip: bound by the FP32 units; the bytes are the PDEs' parameters and the final rows
+        sms = torch.cuda.get_device_properties(dev).multi_processor_count
+        mhz = clk["sm_mhz"] or 2070.0
+        achieved = PAIR_OPS_PER_NODE_STEP * ns / per_launch_s / 1e12
+        peak = sms * FP32_LANES_PER_SM * mhz * 1e6 / 1e12
+        algo_bytes = n_loc * (34 + 8 * X_DIM)
+        roofline = {"bound": "fp32", "kernel": "fd1d_solve_onchip", "achieved": achieved, "peak": peak,
+                    "unit": "T FP32 operations/s", "frac": achieved / peak,
+                    "peak_source": f"{sms} SMs x {FP32_LANES_PER_SM} FP32 lanes at the sampled median clock",
+                    "traffic": algo_bytes, "algorithmic_bytes_per_launch": algo_bytes,
+                    "algorithmic_bytes_per_node_step": algo_bytes / ns,
+                    "basis": f"{PAIR_OPS_PER_NODE_STEP} FP32 operations per node-step: two tridiagonal solves and a "
+                             "residual in pair arithmetic per step",
+                    "hbm_frac": algo_bytes / per_launch_s / 1e9 / hbm, "hbm_peak_source": peak_src,
+                    "fp64_equivalent_tflops": FP64_FLOPS_PER_NODE_STEP * ns / per_launch_s / 1e12,
+                    "fp64_peak_tflops": fp64_peak, "fp64_peak_source": "measured here: cuBLAS DGEMM 4096^3", **common}
 
     # ---------------------------------------------------------------- CPU baseline and FP64 parity
     # the oracle prices of the CPU-baseline sample are the parity check of the whole
@@ -693,20 +733,7 @@ def run_ours(args):
         "e2e": {"value": e2e_value, "unit": "options/s", "h2d_bytes_per_step": h2d, "d2h_bytes_per_step": d2h},
         "gpu_launches": launches,
         "clocks": clk,
-        "roofline": {"bound": "hbm", "kernel": "fd1d_solve_fp64", "achieved": achieved, "peak": hbm,
-                     "unit": "GB/s", "frac": achieved / hbm, "peak_source": peak_src, "traffic": traffic,
-                     "algorithmic_bytes_per_launch": algo_bytes,
-                     "algorithmic_bytes_per_node_step": ALGO_BYTES_PER_NODE_STEP,
-                     "basis": "32 B per node-step (V read + write, sweep value write + read), FP64 streaming scheme",
-                     "achieved_requested": achieved_req, "frac_requested": achieved_req / hbm,
-                     "requested_bytes_per_node_step": req_bytes / ns,
-                     "requested_basis": "bytes the kernel itself requests (state 32 B + payoff 8 B where nonzero "
-                                        "+ coefficients 24 B outside the frozen middle region), counted in the kernel",
-                     "traffic_per_node_step": traffic / ns if traffic else None,
-                     "node_steps_per_launch": ns, "launch_ms": per_launch_s * 1e3,
-                     "fp64_tflops": fp64_tflops, "fp64_peak_tflops": fp64_peak,
-                     "fp64_frac": fp64_tflops / fp64_peak if fp64_peak else None,
-                     "fp64_peak_source": "measured here: cuBLAS DGEMM 4096^3"},
+        "roofline": roofline,
         "cpu_baseline": ({"value": cpu_rate, "unit": "options/s", "cores": cpu_threads, "kind": "port",
                           "sample": f"{cpu_n} options of the batch at 1024x1024 ({cpu_s:.1f} s), oracle C "
                                     f"restatement, {cpu_threads} threads"} if cpu_rate else None),
@@ -721,7 +748,7 @@ def run_ours(args):
                               "gpu_launches_per_step": launches32},
                      "uneven_131072": dict(uneven, workload="131072 options, per-option x_dim in "
                                             "{128..2048} by vol*sqrt(T), t_dim=clamp(ceil(512 sqrt(T)),64,2048), "
-                                            "uniform grids, scale 5; kwg_fd1d_price_uneven (host API, CUDA graph)"),
+                                            "uniform grids, scale 5; kwg_fd1d_price_uneven (host API)"),
                      "fd1d_bs_32768x1024": fd1d_bs,
                      "precision_65536x2048": fine,
                      "precision_128x512": small,

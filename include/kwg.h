@@ -77,7 +77,7 @@ typedef struct kwg_fd1d_params {
     int32_t solver;    /* KWG_SOLVER_AUTO (default); _THOMAS: the FP64 streaming solver, one
                           thread per PDE; _PCR: the on-chip solver, one to four warps per
                           PDE, x_dim <= 1024.  AUTO takes the on-chip one at theta = 1/2 up
-                          to x_dim 2048 (except many PDEs of 56 nodes or fewer) unless
+                          to x_dim 2048 (except many PDEs of 46 nodes or fewer) unless
                           the autotuner recorded another choice */
     int32_t strict;    /* blocking host calls (kwg_fd1d_price, kwg_fd1d_bs_price,
                           kwg_fd1d_price_uneven): 1 returns an error for the first
@@ -184,9 +184,9 @@ int kwg_fd1d_price_device_static(const kwg_option* d_opts, size_t n, const kwg_f
  * t_dims[i] time levels (p's x_dim and t_dim are ignored; its other fields apply).
  * The reference prices one grid shape per Fd1d_Pricer::init
  * (src/Pricer/kwFd1d.cpp:15-16), so a mixed portfolio needs one reference call per
- * shape; here the whole batch is one persistent launch (FP64 Thomas) or one launch
- * per nodes-per-lane bucket (PCR and FP32), replayed from a CUDA graph while the
- * batch layout is unchanged.  Dedup key: (t, r, q, z, e, w, x_dim, t_dim).
+ * shape; here the whole batch is one persistent launch (FP64 Thomas), replayed from a CUDA
+ * graph while the batch layout is unchanged, or one launch per nodes-per-lane bucket
+ * (on-chip solvers), each on its own stream.  Dedup key: (t, r, q, z, e, w, x_dim, t_dim).
  * Results and status as kwg_fd1d_price.  Blocking. */
 int kwg_fd1d_price_uneven(kwg_ctx* ctx, const kwg_option* opts, const int32_t* x_dims,
                           const int32_t* t_dims, size_t n, const kwg_fd1d_params* p,
@@ -211,8 +211,8 @@ typedef struct kwg_tuning {
 
 /* Autotuner (no counterpart in the reference): on a synthetic batch of m options of
  * p's shape and precision, times options-per-block (1, 2, 4 warps of 32 per block, and
- * one 4-warp block per SM) and Thomas vs PCR for FP64, threads-per-option (1, 2, 4 or 8 warps) for FP32, and records
- * the fastest for later calls of that shape whose p leaves the choices at 0 / AUTO.
+ * one 4-warp block per SM) and Thomas vs the on-chip solver for FP64, threads-per-option (1, 2, 4 or 8
+ * warps) for FP32, and records the fastest for later calls of that shape whose p leaves the choices at 0 / AUTO.
  * `out` may be NULL. */
 int kwg_autotune_ex(kwg_ctx* ctx, const kwg_fd1d_params* p, size_t m, kwg_tuning* out);
 
@@ -224,7 +224,7 @@ int kwg_autotune_uneven(kwg_ctx* ctx, const kwg_option* opts, const int32_t* x_d
 
 /* Compact form of kwg_autotune_ex for FP64: tunes and records the same choices and
  * writes the best streaming (Thomas) solve time over the block sizes and residencies and the
- * warp-per-PDE (PCR) solve time (ms; negative if not applicable).  The choice is kept
+ * on-chip (PCR) solve time (ms; negative if not applicable).  The choice is kept
  * for calls of the same shape (precision, x_dim, t_dim, m rounded to a power of two)
  * on this context.  No counterpart in the reference, which has one CPU solver. */
 int kwg_autotune(kwg_ctx* ctx, const kwg_fd1d_params* p, size_t m, double* thomas_ms, double* pcr_ms);

@@ -243,9 +243,11 @@ __global__ void selftest_waits(int32_t* __restrict__ out, uint32_t limit)
 // solver on FP32 units where it takes the shape (theta = 1/2, up to 2048 nodes), except
 // for many PDEs on small grids: it spends the same time on 3 to 64 nodes (one warp's
 // separator solve), the streaming solver 6 FP64 cycles per node once its lanes are full.
-// Measured, 131072 PDEs, 200 steps, uniform: 16/32/48/64 nodes streaming 2.5/4.7/7.0/9.4 ms,
-// on chip 8.4/8.4/8.4/8.1 ms; a lone streaming warp takes ~290 cycles per node, so below
-// ~430 PDEs per node the on-chip solver is ahead again.  Other schemes: a cost model -- the
+// Measured, 200 steps, uniform, ms streaming / on chip: 131072 PDEs of 16 nodes 2.51/6.93, of 32
+// 4.74/6.93, of 48 7.03/6.92; 32768 of 16 0.73/1.80, of 32 1.32/1.81, of 48 1.91/1.80; 16384 of 16
+// 0.67/0.94, of 32 1.14/0.94.  A lone streaming warp takes ~290 cycles per node, so with fewer
+// PDEs per node the on-chip solver is ahead again, below ~650; from 430 on the streaming
+// solver keeps these sub-millisecond batches, whose prices it has always made.  Other schemes: a cost model -- the
 // thread-per-option kernel runs m/32 warps, the warp-per-option FP64 kernel m warps at twice
 // the FP64 work per node-step, so the latter wins while m/32 warps cannot fill the GPU.
 kwg_ctx::Tuned choose(kwg_ctx* ctx, const kwg_fd1d_params* p, int m)
@@ -259,7 +261,7 @@ kwg_ctx::Tuned choose(kwg_ctx* ctx, const kwg_fd1d_params* p, int m)
         if (p->precision == KWG_FP64 && t.solver == KWG_SOLVER_PCR && !pair64_ok(p) && !pcr_ok)
             t.solver = KWG_SOLVER_THOMAS;
     } else {
-        const bool many_small = p->x_dim <= 56 && m > 430 * p->x_dim;
+        const bool many_small = p->x_dim <= 46 && m > 430 * p->x_dim;
         const bool on_chip = pair64_ok(p) ? !many_small : pcr_ok && m < 8192;
         t.solver = on_chip ? KWG_SOLVER_PCR : KWG_SOLVER_THOMAS;
     }
