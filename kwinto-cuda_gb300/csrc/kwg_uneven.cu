@@ -73,7 +73,7 @@ UnevenLayout uneven_layout(size_t m, size_t n, size_t ntiles)
 // option: 11 of the 52 ms of 131072 options in FP32 when the whole batch was prepared before
 // the first kernel, and the solves of the buckets waited for one another's last PDEs.  By buckets, all but the
 // first one's preparation hides behind the device, and a bucket's tail behind the
-// next one's start: 42.8 ms (FP64: 143.9 -> 129.9).  With profiling on all run on the context's stream, one after
+// next one's start: 42.8 ms (FP64: 143.9 -> 128.8).  With profiling on all run on the context's stream, one after
 // the other.
 int price_buckets(kwg_ctx* ctx, const kwg_option* opts, const int32_t* x_dims, const int32_t* t_dims, size_t n,
                   const kwg_fd1d_params& q, const kwg_ctx::Tuned& tn, bool pair, double* prices, int32_t* status)
@@ -105,9 +105,13 @@ int price_buckets(kwg_ctx* ctx, const kwg_option* opts, const int32_t* x_dims, c
     }
     std::vector<uint32_t> order(n);
     for (size_t i = 0; i < n; ++i) order[part[id[i]].at++] = (uint32_t)i;
+    // The heaviest bucket first.  The others by work as well, but in pair arithmetic upwards: a
+    // bucket's rescue launch (fd1d_pair64.cu), one PDE's FP64 latency however short its list, then runs
+    // beside the next bucket (4000 options 6.8 -> 5.4 ms; in FP32, which has none, 1.86 -> 1.97).
     int by_work[kBuckets];
     std::iota(by_work, by_work + kBuckets, 0);
     std::stable_sort(by_work, by_work + kBuckets, [&](int a, int b) { return part[a].work > part[b].work; });
+    if (pair) std::reverse(by_work + 1, by_work + kBuckets);
 
     std::vector<int32_t> asset2pde, pde_slot;
     std::vector<uint32_t> pde2asset;
