@@ -79,7 +79,7 @@ namespace {
 // 0.141/0.115/0.130, 600 of them 0.145/0.149/0.196; of 1024 nodes, 300 of them 0.242/0.186/0.166, 600 of
 // them 0.258/0.245/0.270, 900 of them 0.344/0.331/0.393, 1200 of them 0.370/0.422/0.487; 512 nodes at
 // density 0.25, 600 of them 0.206/0.190/0.299; 512 steps, 8192 PDEs of 1024 nodes, density 0.25,
-// 6.86/5.77/6.14, uniform 3.86/4.4/5.8; 4096 PDEs of 2048 nodes -/8.55/6.89, uniform -/4.12/4.72.
+// 6.81/5.71/6.77, uniform 3.86/4.42/5.8; 4096 PDEs of 2048 nodes -/8.48/6.58, uniform -/4.17/5.48.
 int fp32_warps(int m1, bool uni, int m, int sms)
 {
     int w = m1 == 64 ? (uni ? 2 : 4) : m1 == 32 && !uni ? 2 : 1;

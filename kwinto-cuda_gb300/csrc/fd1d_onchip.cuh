@@ -180,14 +180,18 @@ __device__ __forceinline__ Split split(double v)
 //                          FP32 stepping       pair arithmetic (255 steps at 1024 and 2048 nodes)
 //   M = 32 uniform         4.57 -> 3.86        6.79 -> 5.61   (12 warps at 168 registers, 8 at 236)
 //   M = 16 uniform, W = 1  2.41 -> 1.96        5.84 -> 5.56
-//   M = 16 uniform, W = 2                      6.65 -> 6.15
+//   M = 16 uniform, W = 4                      6.65 -> 6.15
 //   M = 16, W = 1          2.94 -> 2.51        6.57 -> 6.41
-//   M = 16, W = 2          7.33 -> 5.77        7.60 -> 7.43
-//   M = 16, W = 4          18.3 -> 12.7        8.74 -> 7.96
-//   M = 8 uniform          2.43 -> 2.01        6.16 -> 5.85
+//   M = 16, W = 2          7.33 -> 5.71        7.60 -> 7.47
+//   M = 16, W = 4          18.3 -> 12.5        8.74 -> 7.96
+//   M = 8 uniform          2.43 -> 2.00        6.16 -> 5.85
 //   M = 8                  2.89 -> 2.26        6.49 -> 6.12
-//   M = 4 uniform          1.54 -> 1.27        3.60 -> 3.52
+//   M = 4 uniform          1.54 -> 1.24        3.60 -> 3.52
 //   M = 4                  1.33 -> 1.32        3.66 -> 3.51
+// Variants that only small batches take (more warps per PDE than a large batch would) need
+// registers, not resident warps: 26 PDEs of 567 nodes (500 steps) 0.652 -> 0.520 pair, 0.267 -> 0.256
+// FP32; 150 of 1024 uniform nodes (256 steps) 0.318 -> 0.267 pair; 300 of 2048 uniform nodes 0.267 -> 0.239
+// FP32.
 struct Budget {
     int warps, tables;
     bool edges;
@@ -196,16 +200,16 @@ __host__ __device__ constexpr Budget budget(int M, int W, bool uni, bool pair)
 {
     if (!pair) {
         if (M == 32) return uni ? Budget{12, 0, W == 1} : Budget{8, 1, W == 2};
-        if (M == 16 && uni) return W == 1 ? Budget{12, 2, true} : Budget{16, 0, true};
-        if (M == 16) return W == 1 ? Budget{10, 2, true} : W == 2 ? Budget{10, 1, false} : Budget{10, 3, false};
-        if (W > 1) return M == 8 ? (W == 2 ? Budget{12, 3, true} : Budget{16, 3, false}) : Budget{12, 3, false};
-        if (M == 2) return uni ? Budget{16, 1, false} : Budget{20, 2, false};
-        return {M == 8 && !uni ? 16 : 20, 3, false};
+        if (M == 16 && uni) return W == 1 ? Budget{12, 2, true} : W == 2 ? Budget{12, 1, false} : Budget{10, 3, false};
+        if (M == 16) return W == 1 ? Budget{10, 2, true} : W == 2 ? Budget{8, 3, true} : Budget{10, 3, false};
+        if (W > 1) return M == 8 && uni && W == 4 ? Budget{10, 3, false} : Budget{12, 3, M == 8};
+        if (M == 2) return {20, 0, false};
+        return {M == 8 && !uni ? 16 : 20, uni ? 2 : 3, false};
     }
     if (M == 32) return {12, 0, true};
-    if (M == 16 && uni) return W == 1 ? Budget{10, 2, true} : Budget{16, 0, false};
+    if (M == 16 && uni) return W == 1 ? Budget{10, 2, true} : W == 2 ? Budget{10, 1, false} : Budget{16, 0, false};
     if (M == 16) return W == 1 ? Budget{8, 3, false} : W == 2 ? Budget{10, 1, false} : Budget{10, 2, false};
-    if (M == 8) return {W == 2 ? 12 : 16, 3, true};
+    if (M == 8) return {W > 1 ? 12 : 16, 3, true};
     if (M == 4) return W > 1 ? Budget{10, 3, false} : uni ? Budget{16, 3, false} : Budget{20, 3, true};
     return {16, 3, true};
 }
@@ -657,7 +661,7 @@ __global__ void __launch_bounds__(32 * W, budget(M, W, kUni, kPair).warps / W)
         // separator system: warp-local cyclic reduction (multipliers in FP32), and for W > 1
         // the responses to the neighbours' values and the inverse of the boundary system
         float ka[5], kc[5], ib, rq = 0.f, rs = 0.f;
-        float sl_m = 0.f, sr_m = 0.f;  // spikes of the previous lane's last node (warp boundaries)
+        float sl_m = 0.f, sr_m = 0.f;  // W > 1: spikes of the previous lane's last node, as its owner uses them
         {
             double Lprev = __shfl_up_sync(kAll, Llast, 1), Rprev = __shfl_up_sync(kAll, Rlast, 1);
             if constexpr (W > 1) {
@@ -713,13 +717,10 @@ __global__ void __launch_bounds__(32 * W, budget(M, W, kUni, kPair).warps / W)
                     e[5 * warp] = vq;
                     e[5 * warp + 1] = vs;
                     e[5 * warp + 4] = Lprev;
-                    sl_m = (float)Lprev;
-                    sr_m = (float)Rprev;
                 }
                 if (k == 31) {
                     e[5 * warp + 2] = vq;
                     e[5 * warp + 3] = vs;
-                    // the spikes as this lane's steps use them (the next warp repeats its update)
                     const float4 q = T3[(P - 1) * kStride];  // node M-1 (the pivot when P = 1)
                     xs[2 * warp] = q.y;
                     xs[2 * warp + 1] = q.w;
@@ -770,6 +771,15 @@ __global__ void __launch_bounds__(32 * W, budget(M, W, kUni, kPair).warps / W)
         bool run = __all_sync(kAll, fit) && !bad;
         if constexpr (W > 1) run = __syncthreads_and(run) != 0;
         else __syncwarp();
+        if constexpr (W > 1) {
+            const float4 q = T3[(P - 1) * kStride];  // node M-1 (the pivot when P = 1)
+            const float l = __shfl_up_sync(kAll, q.y, 1), r = __shfl_up_sync(kAll, q.w, 1);
+            if (k > 0) {
+                sl_m = l;
+                sr_m = r;
+            }
+        }
+        const float sl0 = W > 1 ? __shfl_sync(kAll, sl_m, 0) : 0.f;
 
         // ------------------------------------------------------------ time steps
         float2 H[P], L[P];
@@ -833,7 +843,8 @@ __global__ void __launch_bounds__(32 * W, budget(M, W, kUni, kPair).warps / W)
         // the neighbours at the start of a step; with more, that would be one more barrier per step, so
         // every lane steps these two nodes as well, by the operations of their owners.  FP32
         // stepping: 128 PDEs of 512 nodes 0.240 -> 0.204 ms, 4096 of 2048 7.49 -> 7.09; pair arithmetic: 12
-        // PDEs of 512 nodes 0.452 -> 0.430, but 4096 of 2048 uniform nodes 6.21 -> 6.46, where the two
+        // PDEs of 512 nodes 0.452 -> 0.430 (0.404 since solve() gives the neighbour's value without
+        // waiting for its owner), but 4096 of 2048 uniform nodes 6.21 -> 6.46, where the two
         // nodes cost more than the barrier (kOwn).
         float2 Hn, Ln;
         auto neighbours = [&]() {
@@ -1018,15 +1029,21 @@ __global__ void __launch_bounds__(32 * W, budget(M, W, kUni, kPair).warps / W)
                 const float b_ = __shfl_sync(kAll, x, warp < W - 1 ? 2 * warp : 0);        // own last
                 const float ar = __shfl_sync(kAll, x, warp < W - 1 ? 2 * warp + 1 : 0);    // right warp's first
                 const float yl = warp > 0 ? v[Y::n + warp - 1] : 0.f;
-                const float sl0 = __shfl_sync(kAll, sl_m, 0);
                 const float Q = warp > 0 ? fmaf(-sl0, bl_, yl) : 0.f, Sr = warp < W - 1 ? ar : 0.f;
                 s = fmaf(-rs, Sr, fmaf(rq, Q, s));
                 if (k == 0 && warp > 0) s = a_;
                 if (k == 31 && warp < W - 1) s = b_;
                 s1 = __shfl_down_sync(kAll, s, 1);
                 if (k == 31) s1 = Sr;
-                // the previous warp's last node, by the operations its owner uses below
-                if constexpr (kPair || kOwn) um = fmaf(-a_, sr_m, fmaf(-bl_, sl_m, yl));
+                if constexpr (kPair || kOwn) {
+                    // by the operations its owner uses below, without waiting for them
+                    float s_prev = __shfl_up_sync(kAll, s, 1);
+                    if (k == 0) {
+                        s_prev = bl_;
+                        ylp = yl;
+                    }
+                    um = fmaf(-s, sr_m, fmaf(-s_prev, sl_m, ylp));
+                }
             }
             const float2 ms = f2(-s, -s), ms1 = f2(-s1, -s1);
 #pragma unroll
@@ -1035,9 +1052,8 @@ __global__ void __launch_bounds__(32 * W, budget(M, W, kUni, kPair).warps / W)
                 y[kk] = fma2(ms1, f2(q.z, q.w), fma2(ms, f2(q.x, q.y), y[kk]));
             }
             y[0] = f2(s, fmaf(-s1, p3.w, fmaf(-s, p3.y, yP)));
-            if constexpr (kPair || kOwn) {
-                const float last = __shfl_up_sync(kAll, P > 1 ? y[P - 1].y : y[0].y, 1);
-                if (k > 0) um = last;
+            if constexpr (kPair && W == 1) {
+                um = __shfl_up_sync(kAll, P > 1 ? y[P - 1].y : y[0].y, 1);
                 if (K == 0) um = 0.f;
             }
         };
