@@ -201,17 +201,17 @@ __host__ __device__ constexpr Budget budget(int M, int W, bool uni, bool pair)
     if (!pair) {
         if (M == 32) return uni ? Budget{12, 0, W == 1} : Budget{8, 1, W == 2};
         if (M == 16 && uni) return W == 1 ? Budget{12, 2, true} : W == 2 ? Budget{12, 1, false} : Budget{10, 3, false};
-        if (M == 16) return W == 1 ? Budget{10, 2, true} : W == 2 ? Budget{8, 3, true} : Budget{10, 3, false};
+        if (M == 16) return W == 4 ? Budget{12, 2, false} : Budget{10, 2, true};
         if (W > 1) return M == 8 && uni && W == 4 ? Budget{10, 3, false} : Budget{12, 3, M == 8};
         if (M == 2) return {20, 0, false};
         return {M == 8 && !uni ? 16 : 20, uni ? 2 : 3, false};
     }
     if (M == 32) return {12, 0, true};
     if (M == 16 && uni) return W == 1 ? Budget{10, 2, true} : W == 2 ? Budget{10, 1, false} : Budget{16, 0, false};
-    if (M == 16) return W == 1 ? Budget{8, 3, false} : W == 2 ? Budget{10, 1, false} : Budget{10, 2, false};
+    if (M == 16) return W == 1 ? Budget{8, 3, false} : W == 2 ? Budget{10, 1, false} : Budget{12, 1, false};
     if (M == 8) return {W > 1 ? 12 : 16, 3, true};
     if (M == 4) return W > 1 ? Budget{10, 3, false} : uni ? Budget{16, 3, false} : Budget{20, 3, true};
-    return {16, 3, true};
+    return uni ? Budget{16, 3, true} : Budget{10, 3, false};
 }
 
 // Shared-memory layout of one PDE group (floats).  P = M / 2 slots, NL = 32 W lanes.
@@ -233,7 +233,8 @@ struct Lay {
     static constexpr int oCl = oCh + 4 * S * NL;
     static constexpr int oT2 = oCl + (kPair ? 4 : 2) * S * NL;
     static constexpr int oT3 = oT2 + 4 * P * kStride;
-    static constexpr int oT1 = oT3 + 4 * P * kStride;
+    static constexpr bool kSpikeRegs = !kUni && budget(M, W, kUni, kPair).tables >= 1;  // no T3
+    static constexpr int oT1 = oT3 + (kSpikeRegs ? 0 : 4 * P * kStride);
     static constexpr int oX = oT1 + 2 * P * kStride;
     static constexpr int n = 2 * (W - 1), nv = 3 * (W - 1);  // boundary unknowns and their inputs
     // exchange area: edges [W][4], inputs of the two solves [2][nv], inverse [nv][n],
@@ -628,6 +629,9 @@ __global__ void __launch_bounds__(32 * W, budget(M, W, kUni, kPair).warps / W)
             R1 = mul(sg * pua, xr);
             Rlast = fma(sg * pud, xr, mul(bu_last, sumd));
         }
+        // the spikes, per lane straight into registers where they stay there (kReg)
+        constexpr int P3 = kReg >= 1 ? P : 1;
+        float4 r3[P3] = {};
         if (writer) {
             // spikes L = B_I^-1 (bl_1 e_1), R = B_I^-1 (bu_(M-1) e_(M-1)) by the steps' own solve
             auto spike = [&](float v1, float vn, int f) {
@@ -650,14 +654,27 @@ __global__ void __launch_bounds__(32 * W, budget(M, W, kUni, kPair).warps / W)
                 }
 #pragma unroll
                 for (int kk = 0; kk < P; ++kk) {
-                    float* const q = reinterpret_cast<float*>(&T3[kk * kStride]) + 2 * f;
-                    if (kk > 0) q[0] = v[kk].x;
-                    q[1] = kk > 0 ? v[kk].y : xP;
+                    const float b = kk > 0 ? v[kk].y : xP;
+                    if constexpr (Y::kSpikeRegs) {
+                        float4& q = r3[Y::kSpikeRegs ? kk : 0];
+                        if (f == 0) {
+                            q.x = v[kk].x;
+                            q.y = b;
+                        } else {
+                            q.z = v[kk].x;
+                            q.w = b;
+                        }
+                    } else {
+                        float* const q = reinterpret_cast<float*>(&T3[kk * kStride]) + 2 * f;
+                        if (kk > 0) q[0] = v[kk].x;
+                        q[1] = b;
+                    }
                 }
             };
             spike((float)bl_first, 0.f, 0);
             spike(0.f, (float)bu_last, 1);
         }
+        auto last_spike = [&] { return Y::kSpikeRegs ? r3[P3 - 1] : T3[(P - 1) * kStride]; };  // of node M-1
         // separator system: warp-local cyclic reduction (multipliers in FP32), and for W > 1
         // the responses to the neighbours' values and the inverse of the boundary system
         float ka[5], kc[5], ib, rq = 0.f, rs = 0.f;
@@ -721,7 +738,7 @@ __global__ void __launch_bounds__(32 * W, budget(M, W, kUni, kPair).warps / W)
                 if (k == 31) {
                     e[5 * warp + 2] = vq;
                     e[5 * warp + 3] = vs;
-                    const float4 q = T3[(P - 1) * kStride];  // node M-1 (the pivot when P = 1)
+                    const float4 q = last_spike();
                     xs[2 * warp] = q.y;
                     xs[2 * warp + 1] = q.w;
                 }
@@ -772,7 +789,7 @@ __global__ void __launch_bounds__(32 * W, budget(M, W, kUni, kPair).warps / W)
         if constexpr (W > 1) run = __syncthreads_and(run) != 0;
         else __syncwarp();
         if constexpr (W > 1) {
-            const float4 q = T3[(P - 1) * kStride];  // node M-1 (the pivot when P = 1)
+            const float4 q = last_spike();
             const float l = __shfl_up_sync(kAll, q.y, 1), r = __shfl_up_sync(kAll, q.w, 1);
             if (k > 0) {
                 sl_m = l;
@@ -961,15 +978,17 @@ __global__ void __launch_bounds__(32 * W, budget(M, W, kUni, kPair).warps / W)
         const float2 pHn = Hn, pLn = Ln;  // pairs: the payoffs at the two nodes
 
         // factors held in registers for the whole PDE (kReg)
-        constexpr int P1 = kReg >= 3 ? P : 1, P2 = kReg >= 2 ? P : 1, P3 = kReg >= 1 ? P : 1;
+        constexpr int P1 = kReg >= 3 ? P : 1, P2 = kReg >= 2 ? P : 1;
         float2 r1[P1];
-        float4 r2[P2], r3[P3];
+        float4 r2[P2];
 #pragma unroll
         for (int kk = 0; kk < P1; ++kk) r1[kk] = T1[kk * kStride];
 #pragma unroll
         for (int kk = 0; kk < P2; ++kk) r2[kk] = T2[kk * kStride];
+        if constexpr (!Y::kSpikeRegs) {
 #pragma unroll
-        for (int kk = 0; kk < P3; ++kk) r3[kk] = T3[kk * kStride];
+            for (int kk = 0; kk < P3; ++kk) r3[kk] = T3[kk * kStride];
+        }
         auto fac1 = [&](int kk) -> float2 { return kReg >= 3 ? r1[kReg >= 3 ? kk : 0] : T1[kk * kStride]; };
         auto fac2 = [&](int kk) -> float4 { return kReg >= 2 ? r2[kReg >= 2 ? kk : 0] : T2[kk * kStride]; };
         auto fac3 = [&](int kk) -> float4 { return kReg >= 1 ? r3[kReg >= 1 ? kk : 0] : T3[kk * kStride]; };
