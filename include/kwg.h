@@ -199,7 +199,8 @@ typedef struct kwg_tuning {
                              KWG_SOLVER_AUTO: the on-chip FP64 solver on a grid of 1025 to
                              2048 nodes, which only AUTO selects there */
     int32_t block_warps;  /* warps (32 options each) per block of the streaming FP64 solver */
-    int32_t option_warps; /* warps (32 threads each) per option of the FP32 solver */
+    int32_t option_warps; /* warps (32 threads each) per option of the FP32 solver; 0 (uneven batches):
+                             by each bucket's size */
     int32_t sm_blocks;    /* resident blocks per SM of the streaming FP64 solver (0: as many as fit) */
     double thomas_ms[3];  /* streaming FP64 solver with 1, 2, 4 warps per block */
     double pcr_ms;        /* FP64 on-chip solver (KWG_SOLVER_PCR) */

@@ -15,6 +15,7 @@
 //     are split into one bucket per nodes-per-lane count, and every bucket is prepared, solved and
 //     copied on a stream of its own, the heaviest first (price_buckets).
 #include <algorithm>
+#include <chrono>
 #include <cstdint>
 #include <cstdio>
 #include <cstring>
@@ -496,9 +497,33 @@ extern "C" int kwg_autotune_uneven(kwg_ctx* ctx, const kwg_option* opts, const i
     ctx->tuned.erase(key);
     kwg_fd1d_params widest = *p;
     widest.x_dim = x_max;
-    const kwg_ctx::Tuned best = tune(ctx, p, pcr_ok, pair64_ok(&widest), [&](const kwg_fd1d_params& q) {
+    auto call = [&](const kwg_fd1d_params& q) {
         return kwg_fd1d_price_uneven(ctx, opts, x_dims, t_dims, n, &q, prices.data(), nullptr);
-    }, out);
+    };
+    kwg_ctx::Tuned best = tune(ctx, p, pcr_ok, pair64_ok(&widest), call, out);
+    if (p->precision == KWG_FP32) {
+        // One number of warps for all buckets against each bucket's own by its size.  Whole calls
+        // decide: the candidates' solves were timed one after the other, and buckets that run side
+        // by side want fewer warps (5321 options: 8 warps 3.0 ms a call, by size 2.8).
+        kwg_fd1d_params q = *p;
+        q.strict = 0;
+        auto wall = [&](int warps) {
+            q.option_warps = warps;
+            double ms = -1.;
+            for (int i = 0; i < 4; ++i) {
+                const auto t0 = std::chrono::steady_clock::now();
+                if (call(q) != KWG_OK) return -1.;
+                const double d = std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - t0).count();
+                if (ms < 0. || d < ms) ms = d;
+            }
+            return ms;
+        };
+        const double fixed = wall(best.option_warps), own = wall(0);
+        if (own >= 0. && own <= 1.02 * fixed) {
+            best.option_warps = 0;
+            if (out) out->option_warps = 0;
+        }
+    }
     ctx->tuned[key] = best;
     ctx->err.clear();
     return KWG_OK;
