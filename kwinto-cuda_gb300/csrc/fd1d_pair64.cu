@@ -10,8 +10,8 @@
 // Bound by the FP32 pipe (75 % busy at 1024 uniform nodes) and, for few PDEs, by the
 // latency of the two separator solves per step.  Measured against the FP64 solvers that took
 // these shapes before (whole calls): 32768 PDEs, 1024 x 1024 uniform, 192 -> 84 ms; 8192 PDEs,
-// 1024 x 1024, density 0.25, 186 -> 28 ms; 777 PDEs, 1000 x 731, 12.4 -> 2.8 ms; 600 PDEs,
-// 512 x 512, 2.50 -> 0.77 ms; 12 PDEs 2.35 -> 0.46 ms; 131072 uneven PDEs 340 -> 130 ms.
+// 1024 x 1024, density 0.25, 186 -> 26 ms; 777 PDEs, 1000 x 731, 12.4 -> 2.4 ms; 600 PDEs,
+// 512 x 512, 2.50 -> 0.77 ms; 12 PDEs 2.35 -> 0.44 ms; 131072 uneven PDEs 340 -> 129 ms.
 //
 // Numerics.  The reference step B V' = E V (src/Math/kwFd1d.cpp:61-132) is taken in
 // increments.  With A' = theta dt A and u = theta (V' - V) it reads
@@ -44,7 +44,7 @@ namespace {
 
 // Warps per PDE.  Enough PDEs to give every scheduler a warp: as few as the registers allow
 // (more warps repeat the separator solve) -- one up to 1024 nodes, two on 1024-node grids
-// whose tables are per node (45 KB per PDE: five PDEs per SM, so ten warps instead of five),
+// whose tables are per node (37 KB per PDE: six PDEs per SM, so twelve warps instead of six),
 // four beyond.  Fewer PDEs: twice the warps while every warp still has a scheduler to
 // itself, from 1024 nodes while they fit 12 to an SM, up to four (at eight, or below two nodes
 // per lane, the exchange costs more than the shorter chains save).  Measured, ms with 1/2/4

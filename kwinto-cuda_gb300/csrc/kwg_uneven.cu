@@ -74,7 +74,7 @@ UnevenLayout uneven_layout(size_t m, size_t n, size_t ntiles)
 // option: 11 of the 52 ms of 131072 options in FP32 when the whole batch was prepared before
 // the first kernel, and the solves of the buckets waited for one another's last PDEs.  By buckets, all but the
 // first one's preparation hides behind the device, and a bucket's tail behind the
-// next one's start: 42.8 ms (FP64: 143.9 -> 128.8).  With profiling on all run on the context's stream, one after
+// next one's start: 42.8 ms (FP64: 143.9 -> 129.9).  With profiling on all run on the context's stream, one after
 // the other.
 int price_buckets(kwg_ctx* ctx, const kwg_option* opts, const int32_t* x_dims, const int32_t* t_dims, size_t n,
                   const kwg_fd1d_params& q, const kwg_ctx::Tuned& tn, bool pair, double* prices, int32_t* status)
@@ -86,7 +86,7 @@ int price_buckets(kwg_ctx* ctx, const kwg_option* opts, const int32_t* x_dims, c
     // options by bucket, in the caller's order within one
     struct Part {
         size_t begin = 0, end = 0, at = 0;
-        uint64_t work = 0;
+        uint64_t work = 0, nodes = 0;
         UnevenLayout L;
     } part[kBuckets];
     std::vector<uint8_t> id(n);
@@ -98,6 +98,7 @@ int price_buckets(kwg_ctx* ctx, const kwg_option* opts, const int32_t* x_dims, c
         id[i] = (uint8_t)b;
         ++part[b].end;
         part[b].work += (uint64_t)x_dims[i] * (uint64_t)(t_dims[i] - 1);
+        part[b].nodes += (uint64_t)x_dims[i];
     }
     size_t off = 0;
     for (Part& p : part) {
@@ -108,11 +109,33 @@ int price_buckets(kwg_ctx* ctx, const kwg_option* opts, const int32_t* x_dims, c
     for (size_t i = 0; i < n; ++i) order[part[id[i]].at++] = (uint32_t)i;
     // The heaviest bucket first.  The others by work as well, but in pair arithmetic upwards: a
     // bucket's rescue launch (fd1d_pair64.cu), one PDE's FP64 latency however short its list, then runs
-    // beside the next bucket (4000 options 6.8 -> 5.4 ms; in FP32, which has none, 1.86 -> 1.97).
+    // beside the next bucket (4000 options 6.8 -> 5.4 ms; in FP32, which has none, 1.86 -> 1.97).  In
+    // large batches the heavy buckets' own tails weigh more (131072 options 129.9 -> 132.1).
     int by_work[kBuckets];
     std::iota(by_work, by_work + kBuckets, 0);
     std::stable_sort(by_work, by_work + kBuckets, [&](int a, int b) { return part[a].work > part[b].work; });
-    if (pair) std::reverse(by_work + 1, by_work + kBuckets);
+    if (pair && n < 32768) std::reverse(by_work + 1, by_work + kBuckets);
+
+    // Buffers for all buckets before the first launch, at the size they have without duplicates:
+    // growing one later would wait for the solves in flight.  Batches beyond 2 GB of rows, and what
+    // does not fit, grow bucket by bucket to the size after dedup.
+    uint64_t rows = 0;
+    for (const Part& p : part) rows += p.nodes * sizeof(double);
+    for (int b = 0; b < kBuckets && rows <= 2000000000ull; ++b) {
+        const size_t nb = part[b].end - part[b].begin;
+        kwg_ctx::Bucket& bk = ctx->buckets[b];
+        if (nb == 0) continue;
+        const size_t io = uneven_layout(nb, nb, 0).total,
+                     work = pair ? kwg::fd1d_pair64_work_bytes((int)nb, (long long)part[b].nodes)
+                                 : (size_t)part[b].nodes * sizeof(double);
+        if (ensure_host(ctx, &bk.h_io, &bk.h_io_bytes, io) ||
+            ensure_device(ctx, &bk.d_io, &bk.io_bytes, align_up(io, 256) + 4 * sizeof(int)) ||
+            ensure_device(ctx, &bk.d_work, &bk.work_bytes, work)) {
+            ctx->err.clear();
+            cudaGetLastError();
+            break;
+        }
+    }
 
     std::vector<int32_t> asset2pde, pde_slot;
     std::vector<uint32_t> pde2asset;

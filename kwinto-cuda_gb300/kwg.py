@@ -255,7 +255,7 @@ class Context:
         return a.value, b.value
 
     def autotune_ex(self, params: Fd1dParams, m: int) -> Tuning:
-        """Times options-per-block and Thomas vs PCR (FP64) or threads-per-option (FP32) on
+        """Times options-per-block and streaming vs on chip (FP64) or threads-per-option (FP32) on
         a synthetic batch of m options of params' shape; records and returns the choice."""
         t = Tuning()
         if self._L.kwg_autotune_ex(self.ptr, ctypes.byref(params), m, ctypes.byref(t)):
