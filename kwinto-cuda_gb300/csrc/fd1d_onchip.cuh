@@ -35,6 +35,8 @@ constexpr unsigned kAll = 0xffffffffu;
 // Half-widths that the drift may cross; beyond it the boundary's growth reaches the
 // middle of the grid and FP32's range no longer holds it.
 constexpr double kMaxDrift = 0.3;
+// Separators whose multipliers are below this (2^-45) no longer see each other.
+constexpr float kNoCoupling = 2.8e-14f;
 // Payoffs and coefficients above this leave no room for the pair arithmetic in FP32's range.
 constexpr double kMaxValue = 1e30, kMaxLog = 69.;
 
@@ -178,15 +180,15 @@ __device__ __forceinline__ Split split(double v)
 // the tables moved -> now (8192 PDEs of 512 and 1024 nodes, 16384 of 256 and 128, 4096 of 2048;
 // 512 steps, FP32 at 2048 nodes 1024):
 //                          FP32 stepping       pair arithmetic (255 steps at 1024 and 2048 nodes)
-//   M = 32 uniform         4.57 -> 3.86        6.79 -> 5.61   (12 warps at 168 registers, 8 at 236)
-//   M = 16 uniform, W = 1  2.41 -> 1.96        5.84 -> 5.56
+//   M = 32 uniform         4.57 -> 3.78        6.79 -> 5.61   (12 warps at 168 registers, 8 at 236)
+//   M = 16 uniform, W = 1  2.41 -> 1.95        5.84 -> 5.54
 //   M = 16 uniform, W = 4                      6.65 -> 6.15
 //   M = 16, W = 1          2.94 -> 2.51        6.57 -> 6.41
 //   M = 16, W = 2          7.33 -> 5.71        7.60 -> 7.47
 //   M = 16, W = 4          18.3 -> 12.5        8.74 -> 7.96
-//   M = 8 uniform          2.43 -> 2.00        6.16 -> 5.85
+//   M = 8 uniform          2.43 -> 1.94        6.16 -> 5.78
 //   M = 8                  2.89 -> 2.26        6.49 -> 6.12
-//   M = 4 uniform          1.54 -> 1.24        3.60 -> 3.52
+//   M = 4 uniform          1.54 -> 1.12        3.60 -> 3.46
 //   M = 4                  1.33 -> 1.32        3.66 -> 3.51
 // Variants that only small batches take (more warps per PDE than a large batch would) need
 // registers, not resident warps: 26 PDEs of 567 nodes (500 steps) 0.652 -> 0.520 pair, 0.267 -> 0.256
@@ -259,6 +261,13 @@ __global__ void __launch_bounds__(32 * W, budget(M, W, kUni, kPair).warps / W)
     using Y = Lay<M, kUni, W, kPair>;
     constexpr bool kEdge = budget(M, W, kUni, kPair).edges;
     constexpr int kReg = budget(M, W, kUni, kPair).tables;
+    // Stop the cyclic reduction at the level where the separators no longer see each other: the multipliers
+    // square from level to level, and at 1024 uniform nodes only the first counts.  The branch
+    // splits the solve for the compiler's scheduling, so only where it pays: FP32, 16384 PDEs of 64 uniform
+    // nodes 0.845 -> 0.745 ms, 128 1.24 -> 1.12, 256 2.00 -> 1.94, 8192 of 1024 3.86 -> 3.78; pair, 16384 of 128
+    // 1.83 -> 1.75, 3 of 51 nodes 0.604 -> 0.454.  Not with several warps (128 PDEs of 512 nodes, FP32, 0.200 ->
+    // 0.221) or on most grids with tables per node (16384 of 128, 1.32 -> 1.35).
+    constexpr bool kCut = W == 1 && (kUni ? !kPair || M < 32 : M == 2 || (M == 16 && !kPair));
     constexpr bool kOwn = W > 1 && (!kPair || M <= 8);  // every lane steps its two neighbour nodes itself
     constexpr int P = Y::P, NL = Y::NL, kStride = Y::kStride;
     static_assert(M >= 2 && M % 2 == 0, "as many rows above the pivot as below");
@@ -678,6 +687,7 @@ __global__ void __launch_bounds__(32 * W, budget(M, W, kUni, kPair).warps / W)
         // separator system: warp-local cyclic reduction (multipliers in FP32), and for W > 1
         // the responses to the neighbours' values and the inverse of the boundary system
         float ka[5], kc[5], ib, rq = 0.f, rs = 0.f;
+        int levels = 0;  // of the reduction, as far as a multiplier is above kNoCoupling
         float sl_m = 0.f, sr_m = 0.f;  // W > 1: spikes of the previous lane's last node, as its owner uses them
         {
             double Lprev = __shfl_up_sync(kAll, Llast, 1), Rprev = __shfl_up_sync(kAll, Rlast, 1);
@@ -711,6 +721,7 @@ __global__ void __launch_bounds__(32 * W, budget(M, W, kUni, kPair).warps / W)
                 const double ma = (k - sg < 0) ? 0. : mul(al, rbm), mc = (k + sg > 31) ? 0. : mul(ga, rbp);
                 ka[lv] = (float)ma;
                 kc[lv] = (float)mc;
+                if (kCut && __any_sync(kAll, !(fabsf(ka[lv]) <= kNoCoupling && fabsf(kc[lv]) <= kNoCoupling))) levels = lv + 1;
                 if constexpr (W > 1) {
                     const double qm = __shfl_up_sync(kAll, vq, sg), qp = __shfl_down_sync(kAll, vq, sg);
                     const double sm = __shfl_up_sync(kAll, vs, sg), sp = __shfl_down_sync(kAll, vs, sg);
@@ -1017,6 +1028,7 @@ __global__ void __launch_bounds__(32 * W, budget(M, W, kUni, kPair).warps / W)
             float rho = fmaf(-buf, y_first, fmaf(-blf, ylp, y[0].x));
 #pragma unroll
             for (int lv = 0; lv < 5; ++lv) {
+                if (kCut && lv >= levels) break;
                 const float rm = __shfl_up_sync(kAll, rho, 1 << lv), rp = __shfl_down_sync(kAll, rho, 1 << lv);
                 rho = fmaf(-kc[lv], rp, fmaf(-ka[lv], rm, rho));
             }

@@ -30,3 +30,23 @@ def test_padding_and_kink(ctx, x_dim, warps, density):
     assert rc == kwg.KWG_OK and rc_ref == 0, msg
     assert (st == 0).all() and (st_ref == 0).all()
     assert np.max(np.abs(got - want) / o["k"]) <= TOL
+
+
+@pytest.mark.parametrize("precision,tol", [(0, 1e-11), (1, TOL)])
+@pytest.mark.parametrize("t_dim", [16, 40, 1500])
+@pytest.mark.parametrize("x_dim", [51, 64, 128, 256, 512, 1024])
+def test_reduction_levels(ctx, x_dim, t_dim, precision, tol):
+    """Time steps from coarse to fine: all five levels of the separators' reduction down to one (FP64
+    accuracy: 1e-11 of the strike, a tenth of the parity bar)."""
+    import kwg
+    import kwor
+    import portfolio
+
+    o = portfolio.american_portfolio(8, seed=t_dim)
+    p = kwg.params(t_dim=t_dim, x_dim=x_dim, scale=5.0, density=math.inf, precision=precision,
+                   option_warps=1 if precision else 0)
+    rc, got, st = ctx.fd1d_price(o, p)
+    rc_ref, msg, want, st_ref = kwor.fd1d_price(o, t_dim=t_dim, x_dim=x_dim, scale=5.0, density=math.inf)
+    assert rc == kwg.KWG_OK and rc_ref == 0, msg
+    assert (st == 0).all() and (st_ref == 0).all()
+    assert np.max(np.abs(got - want) / o["k"]) <= tol
