@@ -77,8 +77,9 @@ typedef struct kwg_fd1d_params {
     int32_t solver;    /* KWG_SOLVER_AUTO (default); _THOMAS: the FP64 streaming solver, one
                           thread per PDE; _PCR: the on-chip solver, one to four warps per
                           PDE, x_dim <= 1024.  AUTO takes the on-chip one at theta = 1/2 up
-                          to x_dim 2048 (except many PDEs of 46 nodes or fewer) unless
-                          the autotuner recorded another choice */
+                          to x_dim 2048 (the streaming one where many PDEs of few nodes or
+                          few steps run faster there) unless the autotuner recorded another
+                          choice */
     int32_t strict;    /* blocking host calls (kwg_fd1d_price, kwg_fd1d_bs_price,
                           kwg_fd1d_price_uneven): 1 returns an error for the first
                           bad option, like the reference

@@ -1,0 +1,123 @@
+// fp64_route.h -- which FP64 solver takes a batch at theta = 1/2 on up to 2048 nodes: a cost
+// model of the three, shared by every entry point.
+//   kPair    pair arithmetic on chip; PDEs that it leaves over (fd1d_pair64.cu) go through its setup and
+//            then to the warp-per-PDE FP64 kernel, in a launch of their own;
+//   kOnChip  the warp-per-PDE FP64 kernel for all of them;
+//   kStream  the streaming solver, one thread per PDE.
+// Without PDEs left over pair arithmetic wins wherever the steps count.  Its setup is the dearer one
+// on few nodes and on uniform grids that do not fill the lanes, so few steps of many such PDEs stream,
+// and so do many PDEs of few nodes: one to 64 nodes cost it the same.
+//
+// The terms are fits to measured calls (in ns, 152 SMs), within a fifth of them from 2 to 1000 steps, 8 to
+// 2048 nodes and 60 to 131072 PDEs.  Both sides at the lines, ms streaming / pair: 131072 uniform PDEs of 65 nodes, 2
+// steps 1.51/2.73, 99 steps (32768) 1.68/1.60; 32768 of 513, 2 steps 3.03/3.56, 29 steps 5.52/4.77; 16384 of 16 nodes, 199
+// steps 0.75/0.94, of 32 nodes 1.27/0.89; 131072 of 40, 999 steps 30.7/30.1.
+#pragma once
+
+#include <algorithm>
+
+#include "fd1d_kernels.h"
+
+namespace kwg {
+
+enum class Fp64Route { kPair, kOnChip, kStream };
+
+// A batch by what its cost depends on: PDEs and time steps by padded node count (64, 128, ... 2048).
+struct Fp64Batch {
+    struct Kind {
+        long long n = 0, steps = 0;
+        int longest = 0;
+
+        void add(long long count, int s)
+        {
+            n += count;
+            steps += count * s;
+            longest = std::max(longest, s);
+        }
+    };
+    struct Cost {
+        double sum = 0., longest = 0.;  // throughput, and one PDE's latency
+
+        double ns() const { return std::max(sum, longest); }
+    };
+    static constexpr int kSizes = 6;
+    bool uniform;
+    Kind plain[kSizes], left[kSizes];
+    bool ragged[kSizes] = {};  // a PDE that does not fill the lanes
+    double nodes = 0., node_steps = 0.;
+    long long most_nodes = 0, most_node_steps = 0;
+
+    explicit Fp64Batch(bool uniform_grid) : uniform(uniform_grid) {}
+
+    // `count` PDEs of x nodes (2048 at most) and s steps, `leaves` of them left over by pair arithmetic
+    void add(long long count, int x, int s, long long leaves = 0)
+    {
+        int k = 0;
+        while ((64 << k) < x && k < kSizes - 1) ++k;
+        ragged[k] = ragged[k] || x != 64 << k;
+        if (count > leaves) plain[k].add(count - leaves, s);
+        if (leaves > 0) left[k].add(leaves, s);
+        nodes += (double)count * x;
+        node_steps += (double)count * x * s;
+        most_nodes = std::max(most_nodes, (long long)x);
+        most_node_steps = std::max(most_node_steps, (long long)x * s);
+    }
+
+    bool any_left() const
+    {
+        for (const Kind& l : left)
+            if (l.n > 0) return true;
+        return false;
+    }
+    double setup_ns(int k) const
+    {
+        const double n = 64 << k;
+        return !uniform ? 20. + 0.145 * n : ragged[k] ? 10. + 0.103 * n : 12. + 0.038 * n;
+    }
+    // the warp-per-PDE FP64 kernel
+    static void add_fp64(Cost& c, const Kind& d, int k)
+    {
+        const double n = 64 << k;
+        c.sum += 0.16 * n * (double)d.n + (n > 1024. ? 0.029 * n : 0.5 + 0.0135 * n) * (double)d.steps;
+        c.longest = std::max(c.longest, d.longest * (1200. + 8.8 * n));
+    }
+    double pair_ns() const
+    {
+        Cost c, rest;
+        for (int k = 0; k < kSizes; ++k) {
+            const double n = 64 << k, setup = setup_ns(k) * (double)plain[k].n;
+            c.sum += std::max(setup, 0.5 * setup + std::max(0.23, 0.0028 * n) * (double)plain[k].steps);
+            c.longest = std::max(c.longest, plain[k].longest * (500. + 0.8 * n));
+            rest.sum += setup_ns(k) * (double)left[k].n;
+            add_fp64(rest, left[k], k);
+        }
+        return c.ns() + rest.ns();
+    }
+    double on_chip_ns() const
+    {
+        Cost c;
+        for (int k = 0; k < kSizes; ++k) {
+            add_fp64(c, plain[k], k);
+            add_fp64(c, left[k], k);
+        }
+        return c.ns();
+    }
+    double stream_ns() const
+    {
+        int longest = 0;
+        for (int k = 0; k < kSizes; ++k) longest = std::max({longest, plain[k].longest, left[k].longest});
+        const double x = (double)most_nodes, xs = (double)most_node_steps, s = longest;
+        return std::max(uniform ? 0.175 * nodes + 0.0055 * node_steps : 0.33 * nodes + 0.0078 * node_steps,
+                        uniform ? 4100. * x + 140. * xs + 1100. * s : 7100. * x + 155. * xs + 1250. * s);
+    }
+    // FP64 stepping, whichever of the two
+    Fp64Route fp64() const { return on_chip_ns() <= stream_ns() ? Fp64Route::kOnChip : Fp64Route::kStream; }
+    Fp64Route best() const
+    {
+        const double p = pair_ns();
+        if (any_left() && on_chip_ns() < p && fp64() == Fp64Route::kOnChip) return Fp64Route::kOnChip;
+        return stream_ns() < p ? Fp64Route::kStream : Fp64Route::kPair;
+    }
+};
+
+}  // namespace kwg

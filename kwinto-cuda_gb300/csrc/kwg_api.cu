@@ -22,6 +22,7 @@
 #include <cuda_runtime.h>
 
 #include "fd1d_kernels.h"
+#include "fp64_route.h"
 #include "host_dedup.h"
 #include "kwg.h"
 #include "kwg_ctx.h"
@@ -239,17 +240,10 @@ __global__ void selftest_waits(int32_t* __restrict__ out, uint32_t limit)
 
 
 // Launch choices for a batch of m PDEs: the explicit ones in p, else what the
-// autotuner recorded for the shape, else defaults.  FP64 solver default: the on-chip
-// solver on FP32 units where it takes the shape (theta = 1/2, up to 2048 nodes), except
-// for many PDEs on small grids: it spends the same time on 3 to 64 nodes (one warp's
-// separator solve), the streaming solver 6 FP64 cycles per node once its lanes are full.
-// Measured, 200 steps, uniform, ms streaming / on chip: 131072 PDEs of 16 nodes 2.51/6.93, of 32
-// 4.74/6.93, of 48 7.03/6.92; 32768 of 16 0.73/1.80, of 32 1.32/1.81, of 48 1.91/1.80; 16384 of 16
-// 0.67/0.94, of 32 1.14/0.94.  A lone streaming warp takes ~290 cycles per node, so with fewer
-// PDEs per node the on-chip solver is ahead again, below ~650; from 430 on the streaming
-// solver keeps these sub-millisecond batches, whose prices it has always made.  Other schemes: a cost model -- the
-// thread-per-option kernel runs m/32 warps, the warp-per-option FP64 kernel m warps at twice
-// the FP64 work per node-step, so the latter wins while m/32 warps cannot fill the GPU.
+// autotuner recorded for the shape, else defaults.  FP64 solver default: at theta = 1/2 up to 2048
+// nodes the cost model of fp64_route.h.  Other schemes: the thread-per-option kernel runs m/32 warps, the
+// warp-per-option FP64 kernel m warps at twice the FP64 work per node-step, so the latter wins
+// while m/32 warps cannot fill the GPU.
 kwg_ctx::Tuned choose(kwg_ctx* ctx, const kwg_fd1d_params* p, int m)
 {
     kwg_ctx::Tuned t;
@@ -261,8 +255,12 @@ kwg_ctx::Tuned choose(kwg_ctx* ctx, const kwg_fd1d_params* p, int m)
         if (p->precision == KWG_FP64 && t.solver == KWG_SOLVER_PCR && !pair64_ok(p) && !pcr_ok)
             t.solver = KWG_SOLVER_THOMAS;
     } else {
-        const bool many_small = p->x_dim <= 46 && m > 430 * p->x_dim;
-        const bool on_chip = pair64_ok(p) ? !many_small : pcr_ok && m < 8192;
+        bool on_chip = pcr_ok && m < 8192;
+        if (pair64_ok(p)) {
+            kwg::Fp64Batch b(std::isinf(p->density));
+            b.add(m, p->x_dim, p->t_dim - 1);
+            on_chip = b.best() != kwg::Fp64Route::kStream;
+        }
         t.solver = on_chip ? KWG_SOLVER_PCR : KWG_SOLVER_THOMAS;
     }
     if (p->precision == KWG_FP32) t.solver = KWG_SOLVER_PCR;
@@ -688,7 +686,8 @@ int kwg_autotune_ex(kwg_ctx* ctx, const kwg_fd1d_params* p, size_t m, kwg_tuning
     std::vector<double> prices(m);
     const bool pcr_ok = kwg::fd1d_pcr64_nodes_per_lane(p->x_dim) > 0;
     const uint64_t key = tune_key(p->precision, p->x_dim, p->t_dim, (int)m);
-    ctx->tuned.erase(key);
+    ctx->tuned[key] = kwg_ctx::Tuned();
+    ctx->tuned[key].solver = KWG_SOLVER_PCR;
     const kwg_ctx::Tuned best = tune(ctx, p, pcr_ok, pair64_ok(p), [&](const kwg_fd1d_params& q) {
         return kwg_fd1d_price(ctx, opts.data(), m, &q, prices.data(), nullptr);
     }, out);

@@ -185,7 +185,7 @@ inline double time_solve(kwg_ctx* ctx, F&& call)
 // (when pcr_ok); FP32 -- 1, 2, 4 and 8 warps per option.  auto_on_chip: a call with AUTO and
 // no record takes the on-chip FP64 solver although KWG_SOLVER_PCR is refused (grids of 1025
 // to 2048 nodes); it is then timed through AUTO, and reported as KWG_SOLVER_AUTO.  The
-// caller has dropped the shape's earlier record.
+// caller has set the shape's record to the on-chip solver, so that AUTO takes it.
 template <typename F>
 inline kwg_ctx::Tuned tune(kwg_ctx* ctx, const kwg_fd1d_params* p, bool pcr_ok, bool auto_on_chip, F&& fn,
                            kwg_tuning* out)

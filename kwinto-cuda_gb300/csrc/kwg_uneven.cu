@@ -16,6 +16,7 @@
 //     copied on a stream of its own, the heaviest first (price_buckets).
 #include <algorithm>
 #include <chrono>
+#include <cmath>
 #include <cstdint>
 #include <cstdio>
 #include <cstring>
@@ -26,6 +27,7 @@
 #include <cuda_runtime.h>
 
 #include "fd1d_kernels.h"
+#include "fp64_route.h"
 #include "host_dedup.h"
 #include "kwg.h"
 #include "kwg_ctx.h"
@@ -275,6 +277,14 @@ int check_strict(kwg_ctx* ctx, const int32_t* status, size_t n)
     return KWG_OK;
 }
 
+// The FP64 solver of an uneven batch at theta = 1/2, every option a PDE of its own.
+kwg::Fp64Route uneven_route(const int32_t* x_dims, const int32_t* t_dims, size_t n, const kwg_fd1d_params& q)
+{
+    kwg::Fp64Batch b(std::isinf(q.density));
+    for (size_t i = 0; i < n; ++i) b.add(1, x_dims[i], t_dims[i] - 1);
+    return b.best();
+}
+
 uint64_t mix(uint64_t h, uint64_t v)
 {
     h ^= v + 0x9e3779b97f4a7c15ull + (h << 6) + (h >> 2);
@@ -312,14 +322,15 @@ extern "C" int kwg_fd1d_price_uneven(kwg_ctx* ctx, const kwg_option* opts, const
     if (int rc = check_params(ctx, &q)) return rc;
     // launch choices: the explicit ones, else what kwg_autotune_uneven recorded for
     // uneven batches of this precision and size, else the on-chip solvers with warps by the
-    // bucket's size, or (theta != 1/2, more than 2048 nodes) Thomas with one warp per block
+    // bucket's size, or (theta != 1/2, more than 2048 nodes, and where the cost model of fp64_route.h
+    // says so) Thomas with one warp per block
     kwg_ctx::Tuned tn;
-    if (q.precision == KWG_FP64 && q.solver == KWG_SOLVER_AUTO && pair64_ok(&q)) tn.solver = KWG_SOLVER_PCR;
     {
         const auto it = ctx->tuned.find(tune_key(q.precision, 0, 0, (long long)n));
-        if (it != ctx->tuned.end()) {
+        if (it != ctx->tuned.end())
             tn = it->second;
-        }
+        else if (q.solver == KWG_SOLVER_AUTO && pair64_ok(&q) && uneven_route(x_dims, t_dims, n, q) != kwg::Fp64Route::kStream)
+            tn.solver = KWG_SOLVER_PCR;
         if (q.precision == KWG_FP64 && q.solver == KWG_SOLVER_AUTO &&
             (tn.solver != KWG_SOLVER_PCR || pair64_ok(&q) || kwg::fd1d_pcr64_nodes_per_lane(x_max) > 0))
             q.solver = tn.solver;
@@ -517,7 +528,8 @@ extern "C" int kwg_autotune_uneven(kwg_ctx* ctx, const kwg_option* opts, const i
     std::vector<double> prices(n);
     const bool pcr_ok = kwg::fd1d_pcr64_nodes_per_lane(x_max) > 0;
     const uint64_t key = tune_key(p->precision, 0, 0, (long long)n);
-    ctx->tuned.erase(key);
+    ctx->tuned[key] = kwg_ctx::Tuned();
+    ctx->tuned[key].solver = KWG_SOLVER_PCR;
     kwg_fd1d_params widest = *p;
     widest.x_dim = x_max;
     auto call = [&](const kwg_fd1d_params& q) {
