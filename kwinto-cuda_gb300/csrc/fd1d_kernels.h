@@ -109,6 +109,10 @@ int fd1d_fp32_launch(const PdeBatch& b, const AssetBatch& a, const Fd1dShape& sh
 int fd1d_pcr64_nodes_per_lane(int x_dim);
 int fd1d_pcr64_rescue(const PdeBatch& b, const Fd1dShape& sh, double* vout, const int32_t* list, int32_t* pde_status,
                       int* counters, int sms, cudaStream_t stream);
+// theta = 1/2 for a whole batch (x_dim <= 2048)
+int fd1d_pcr64_half_launch(const PdeBatch& b, const AssetBatch& a, const Fd1dShape& sh, double* vout, int32_t* pde_status,
+                           int* counters, double* prices, int32_t* status, int device, cudaStream_t stream,
+                           const SolveEvents* ev);
 int fd1d_pcr64_launch(const PdeBatch& b, const AssetBatch& a, const Fd1dShape& sh, double* vout, int32_t* pde_status,
                       int* counters, double* prices, int32_t* status, int device, cudaStream_t stream,
                       const SolveEvents* ev);
@@ -117,6 +121,17 @@ int fd1d_pcr64_launch(const PdeBatch& b, const AssetBatch& a, const Fd1dShape& s
 // four warps per PDE.  The work buffer holds the final V of every PDE and the list of the
 // PDEs left to the FP64 kernel (`rescue`, m ints); -1 for shapes it does not take.
 size_t fd1d_pair64_work_bytes(int m, long long nodes);
+// PDEs that it leaves over by their inputs: a drift of more than kMaxDrift half-widths, beyond which the
+// boundary's growth reaches the middle of the grid and FP32's range no longer holds it, and
+// calls on a grid that passes e^kMaxLog.  (Beyond e^700 FP64 has no price either; those, and inputs that are not
+// finite, are not counted.)
+constexpr double kMaxDrift = 0.3, kMaxLog = 69.;
+__host__ __device__ inline bool pair64_leaves(double t, double z, double r, double q, int w, double scale)
+{
+    const double drift = r - q - 0.5 * z * z, half = scale * z;  // half: the half-width over sqrt(t)
+    return drift * drift * t > kMaxDrift * kMaxDrift * half * half ||
+           (w >= 0 && half * half * t >= kMaxLog * kMaxLog && half * half * t < 700. * 700.);
+}
 int fd1d_pair64_launch(const PdeBatch& b, const AssetBatch& a, const Fd1dShape& sh, double* vout, int32_t* rescue,
                        int32_t* pde_status, int* counters, double* prices, int32_t* status, int device,
                        cudaStream_t stream, const SolveEvents* ev);

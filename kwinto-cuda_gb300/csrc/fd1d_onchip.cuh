@@ -32,13 +32,10 @@ namespace kwg {
 namespace {
 
 constexpr unsigned kAll = 0xffffffffu;
-// Half-widths that the drift may cross; beyond it the boundary's growth reaches the
-// middle of the grid and FP32's range no longer holds it.
-constexpr double kMaxDrift = 0.3;
 // Separators whose multipliers are below this (2^-45) no longer see each other.
 constexpr float kNoCoupling = 2.8e-14f;
 // Payoffs and coefficients above this leave no room for the pair arithmetic in FP32's range.
-constexpr double kMaxValue = 1e30, kMaxLog = 69.;
+constexpr double kMaxValue = 1e30;
 
 __device__ __forceinline__ float2 f2(float a, float b) { return make_float2(a, b); }
 __device__ __forceinline__ float2 neg(float2 a) { return make_float2(-a.x, -a.y); }
@@ -346,7 +343,7 @@ __global__ void __launch_bounds__(32 * W, budget(M, W, kUni, kPair).warps / W)
         const double ax_t = mul(tdt, a.ax), axx_t = mul(mul(2., tdt), a.axx);
         const double xend = mul(mul(sh.scale, z), sqrt(t));  // the grid is [-xend, xend]
         const double dy = dvd(2., (double)(N - 1));
-        bool fit = !kPair || (fabs(a.ax) * t <= kMaxDrift * xend && (w < 0 || xend < kMaxLog));
+        bool fit = !kPair || !pair64_leaves(t, z, rr, qq, w, sh.scale);
         // x_j = d sinh(y_j), y_j = yend (j dy - 1), or y_j itself on a uniform grid
         const bool uniform = kUni || sh.uniform;
         const double yend = uniform ? xend : asinh(dvd(xend, sh.density));

@@ -4,7 +4,8 @@
 // V' = max(y - cV, p) on nodes < N-1 (src/Math/kwFd1d.cpp:61-132), but the 32 lanes
 // of a warp share one PDE, so a batch of m options keeps m warps busy instead of
 // m/32.  It serves theta != 1/2 on small batches, where the thread-per-option kernel cannot
-// fill the GPU, and the PDEs that the solver on FP32 units (fd1d_pair64.cu) leaves over.
+// fill the GPU, and at theta = 1/2 the PDEs that the solver on FP32 units (fd1d_pair64.cu) leaves over,
+// or a batch with many of them (fp64_route.h).
 //
 // Solve of T y = V (N_p = 32 M nodes, lane k owns nodes kM .. kM+M-1; the grid is
 // padded to N_p with decoupled identity rows):
@@ -298,7 +299,7 @@ void prepare_pcr64()
 {
     prepare_pcr64_variant<M, false, false>();
     prepare_pcr64_variant<M, false, true>();
-    prepare_pcr64_variant<M, true, false>();  // theta = 1/2: listed PDEs only
+    prepare_pcr64_variant<M, true, false>();  // theta = 1/2
 }
 
 template <int M, bool kShared>
@@ -333,13 +334,27 @@ int launch_pcr64(const PdeBatch& b, const AssetBatch& a, const Fd1dShape& sh, do
     return launch_pcr64_variant<M, false>(b, a, sh, vout, pde_status, counters, prices, status, sms, stream, ev);
 }
 
+// theta = 1/2: the listed PDEs, or all without a list
 template <int M>
-void launch_rescue(const PdeBatch& b, const Fd1dShape& sh, double* vout, const int32_t* list, int32_t* pde_status,
-                   int* counters, int sms, cudaStream_t stream)
+void launch_half(const PdeBatch& b, const Fd1dShape& sh, double* vout, const int32_t* list, int32_t* pde_status,
+                 int* counters, int sms, cudaStream_t stream)
 {
     const int cap = sms * per_sm_pcr64<M, true, false>();
     fd1d_solve_fp64_pcr<M, true, false><<<b.m < cap ? b.m : cap, 32, pcr64_smem<M, false>(), stream>>>(
         b, sh, vout, pde_status, counters, list);
+}
+
+void launch_half(const PdeBatch& b, const Fd1dShape& sh, double* vout, const int32_t* list, int32_t* pde_status,
+                 int* counters, int sms, cudaStream_t stream)
+{
+    switch (fd1d_fp32_nodes_per_lane(sh.x_dim)) {
+    case 2: launch_half<2>(b, sh, vout, list, pde_status, counters, sms, stream); break;
+    case 4: launch_half<4>(b, sh, vout, list, pde_status, counters, sms, stream); break;
+    case 8: launch_half<8>(b, sh, vout, list, pde_status, counters, sms, stream); break;
+    case 16: launch_half<16>(b, sh, vout, list, pde_status, counters, sms, stream); break;
+    case 32: launch_half<32>(b, sh, vout, list, pde_status, counters, sms, stream); break;
+    default: launch_half<64>(b, sh, vout, list, pde_status, counters, sms, stream); break;
+    }
 }
 
 }  // namespace
@@ -361,20 +376,29 @@ int fd1d_pcr64_nodes_per_lane(int x_dim)
     return m <= 32 ? m : -1;
 }
 
-// The PDEs that fd1d_solve_pair64 left on its list (counters[2] of them, queue
+// The PDEs that pair arithmetic (fd1d_pair64.cu) left on its list (counters[2] of them, queue
 // counters[3]); up to 2048 nodes.
 int fd1d_pcr64_rescue(const PdeBatch& b, const Fd1dShape& sh, double* vout, const int32_t* list, int32_t* pde_status,
                       int* counters, int sms, cudaStream_t stream)
 {
-    switch (fd1d_fp32_nodes_per_lane(sh.x_dim)) {
-    case 2: launch_rescue<2>(b, sh, vout, list, pde_status, counters, sms, stream); break;
-    case 4: launch_rescue<4>(b, sh, vout, list, pde_status, counters, sms, stream); break;
-    case 8: launch_rescue<8>(b, sh, vout, list, pde_status, counters, sms, stream); break;
-    case 16: launch_rescue<16>(b, sh, vout, list, pde_status, counters, sms, stream); break;
-    case 32: launch_rescue<32>(b, sh, vout, list, pde_status, counters, sms, stream); break;
-    default: launch_rescue<64>(b, sh, vout, list, pde_status, counters, sms, stream); break;
-    }
+    launch_half(b, sh, vout, list, pde_status, counters, sms, stream);
     return 1;
+}
+
+int fd1d_pcr64_half_launch(const PdeBatch& b, const AssetBatch& a, const Fd1dShape& sh, double* vout, int32_t* pde_status,
+                           int* counters, double* prices, int32_t* status, int device, cudaStream_t stream,
+                           const SolveEvents* ev)
+{
+    int sms = 0;
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
+    if (fd1d_fp32_nodes_per_lane(sh.x_dim) < 0) return -1;
+    cudaMemsetAsync(counters, 0, 4 * sizeof(int), stream);
+    if (ev) cudaEventRecord(ev->start, stream);
+    launch_half(b, sh, vout, nullptr, pde_status, counters, sms, stream);
+    if (ev) cudaEventRecord(ev->stop, stream);
+    if (a.n == 0) return 1;
+    fd1d_interp_rows<<<(a.n + 127) / 128, 128, 0, stream>>>(b, a, sh, vout, pde_status, prices, status);
+    return 2;
 }
 
 int fd1d_pcr64_launch(const PdeBatch& b, const AssetBatch& a, const Fd1dShape& sh, double* vout, int32_t* pde_status,

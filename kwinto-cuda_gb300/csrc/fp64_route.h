@@ -12,6 +12,9 @@
 // 2048 nodes and 60 to 131072 PDEs.  Both sides at the lines, ms streaming / pair: 131072 uniform PDEs of 65 nodes, 2
 // steps 1.51/2.73, 99 steps (32768) 1.68/1.60; 32768 of 513, 2 steps 3.03/3.56, 29 steps 5.52/4.77; 16384 of 16 nodes, 199
 // steps 0.75/0.94, of 32 nodes 1.27/0.89; 131072 of 40, 999 steps 30.7/30.1.
+// PDEs left over (a drift across the grid: vol 2 to 5 %, rates of 6 to 10 %) cost pair arithmetic its setup and the FP64
+// kernel five times a step, or its latency: ms streaming / pair, all PDEs left over, 99 steps: 32768 of 1024 nodes
+// 24.0/50.2, 12000 of them 19.4/18.8; 300 of 512 nodes, 30 of them left over, 255 steps: FP64 on chip 1.19, pair 1.47.
 #pragma once
 
 #include <algorithm>
@@ -44,23 +47,22 @@ struct Fp64Batch {
     bool uniform;
     Kind plain[kSizes], left[kSizes];
     bool ragged[kSizes] = {};  // a PDE that does not fill the lanes
-    double nodes = 0., node_steps = 0.;
-    long long most_nodes = 0, most_node_steps = 0;
+    long long nodes = 0, node_steps = 0, most_nodes = 0, most_node_steps = 0;
 
     explicit Fp64Batch(bool uniform_grid) : uniform(uniform_grid) {}
 
     // `count` PDEs of x nodes (2048 at most) and s steps, `leaves` of them left over by pair arithmetic
     void add(long long count, int x, int s, long long leaves = 0)
     {
-        int k = 0;
-        while ((64 << k) < x && k < kSizes - 1) ++k;
+        const int k = x <= 64 ? 0 : 26 - __builtin_clz((unsigned)x - 1u);
         ragged[k] = ragged[k] || x != 64 << k;
         if (count > leaves) plain[k].add(count - leaves, s);
         if (leaves > 0) left[k].add(leaves, s);
-        nodes += (double)count * x;
-        node_steps += (double)count * x * s;
+        const long long xs = (long long)x * s;
+        nodes += count * x;
+        node_steps += count * xs;
         most_nodes = std::max(most_nodes, (long long)x);
-        most_node_steps = std::max(most_node_steps, (long long)x * s);
+        most_node_steps = std::max(most_node_steps, xs);
     }
 
     bool any_left() const
@@ -75,19 +77,28 @@ struct Fp64Batch {
         return !uniform ? 20. + 0.145 * n : ragged[k] ? 10. + 0.103 * n : 12. + 0.038 * n;
     }
     // the warp-per-PDE FP64 kernel
-    static void add_fp64(Cost& c, const Kind& d, int k)
+    void add_fp64(Cost& c, const Kind& d, int k) const
     {
         const double n = 64 << k;
-        c.sum += 0.16 * n * (double)d.n + (n > 1024. ? 0.029 * n : 0.5 + 0.0135 * n) * (double)d.steps;
-        c.longest = std::max(c.longest, d.longest * (1200. + 8.8 * n));
+        c.sum += 0.16 * n * (double)d.n +
+                 (uniform ? 1. : 1.12) * (n > 1024. ? 0.029 * n : 0.5 + 0.0135 * n) * (double)d.steps;
+        c.longest = std::max(c.longest, d.longest * (1200. + 8.8 * n) * (d.n > 304 ? 1.25 : 1.));
     }
     double pair_ns() const
     {
         Cost c, rest;
+        long long n_plain = 0, n_all = 0;
+        for (int k = 0; k < kSizes; ++k) {
+            n_plain += plain[k].n;
+            n_all += plain[k].n + left[k].n;
+        }
+        const double wave = n_plain < 2500 ? 1.5 : 1.;  // a last wave of warps that is mostly empty
+        const double warps = n_all <= 304 ? 1. : n_all <= 912 ? 1.4 : 2.2;  // fewer warps per PDE: longer chains
         for (int k = 0; k < kSizes; ++k) {
             const double n = 64 << k, setup = setup_ns(k) * (double)plain[k].n;
-            c.sum += std::max(setup, 0.5 * setup + std::max(0.23, 0.0028 * n) * (double)plain[k].steps);
-            c.longest = std::max(c.longest, plain[k].longest * (500. + 0.8 * n));
+            c.sum += wave * std::max(setup, 0.5 * setup + std::max(0.23, 0.0028 * n) * (double)plain[k].steps);
+            c.longest = std::max(c.longest, plain[k].longest * (uniform ? 600. + 0.8 * n : 700. + n) *
+                                                (k >= 2 && k <= 4 ? warps : 1.));
             rest.sum += setup_ns(k) * (double)left[k].n;
             add_fp64(rest, left[k], k);
         }
@@ -102,13 +113,22 @@ struct Fp64Batch {
         }
         return c.ns();
     }
-    double stream_ns() const
+    Cost stream() const
     {
         int longest = 0;
         for (int k = 0; k < kSizes; ++k) longest = std::max({longest, plain[k].longest, left[k].longest});
         const double x = (double)most_nodes, xs = (double)most_node_steps, s = longest;
-        return std::max(uniform ? 0.175 * nodes + 0.0055 * node_steps : 0.33 * nodes + 0.0078 * node_steps,
-                        uniform ? 4100. * x + 140. * xs + 1100. * s : 7100. * x + 155. * xs + 1250. * s);
+        const double all = (double)nodes, all_steps = (double)node_steps;
+        if (uniform) return {0.175 * all + 0.0055 * all_steps, 4100. * x + 140. * xs + 1100. * s};
+        return {0.33 * all + 0.0078 * all_steps, 7100. * x + 155. * xs + 1250. * s};
+    }
+    double stream_ns() const { return stream().ns(); }
+    // The longest tiles of a streaming launch bind it: they want a scheduler to themselves (one 4-warp block per
+    // SM; 131072 PDEs of up to 2048 nodes and 1144 steps, 585 -> 342 ms).
+    bool few_long_chains() const
+    {
+        const Cost c = stream();
+        return c.longest > 0.5 * c.sum;
     }
     // FP64 stepping, whichever of the two
     Fp64Route fp64() const { return on_chip_ns() <= stream_ns() ? Fp64Route::kOnChip : Fp64Route::kStream; }

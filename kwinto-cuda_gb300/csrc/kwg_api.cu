@@ -239,32 +239,35 @@ __global__ void selftest_waits(int32_t* __restrict__ out, uint32_t limit)
 }
 
 
-// Launch choices for a batch of m PDEs: the explicit ones in p, else what the
-// autotuner recorded for the shape, else defaults.  FP64 solver default: at theta = 1/2 up to 2048
-// nodes the cost model of fp64_route.h.  Other schemes: the thread-per-option kernel runs m/32 warps, the
+// Launch choices for a batch of m PDEs, `left` of which pair arithmetic would leave over: the explicit ones
+// in p, else what the autotuner recorded for the shape, else defaults.  FP64 solver default: at theta =
+// 1/2 up to 2048 nodes the cost model of fp64_route.h, which PDEs left over also bring in where the solver is
+// recorded (the tuner's batch has none).  Other schemes: the thread-per-option kernel runs m/32 warps, the
 // warp-per-option FP64 kernel m warps at twice the FP64 work per node-step, so the latter wins
 // while m/32 warps cannot fill the GPU.
-kwg_ctx::Tuned choose(kwg_ctx* ctx, const kwg_fd1d_params* p, int m)
+kwg_ctx::Tuned choose(kwg_ctx* ctx, const kwg_fd1d_params* p, int m, int left)
 {
     kwg_ctx::Tuned t;
     auto it = ctx->tuned.find(tune_key(p->precision, p->x_dim, p->t_dim, m));
     const bool pcr_ok = kwg::fd1d_pcr64_nodes_per_lane(p->x_dim) > 0;
-    if (it != ctx->tuned.end()) {
+    const bool recorded = it != ctx->tuned.end();
+    if (recorded) {
         t = it->second;
         // recorded for theta = 1/2, which the key does not hold
         if (p->precision == KWG_FP64 && t.solver == KWG_SOLVER_PCR && !pair64_ok(p) && !pcr_ok)
             t.solver = KWG_SOLVER_THOMAS;
     } else {
-        bool on_chip = pcr_ok && m < 8192;
-        if (pair64_ok(p)) {
-            kwg::Fp64Batch b(std::isinf(p->density));
-            b.add(m, p->x_dim, p->t_dim - 1);
-            on_chip = b.best() != kwg::Fp64Route::kStream;
-        }
-        t.solver = on_chip ? KWG_SOLVER_PCR : KWG_SOLVER_THOMAS;
+        t.solver = pcr_ok && m < 8192 ? KWG_SOLVER_PCR : KWG_SOLVER_THOMAS;
     }
     if (p->precision == KWG_FP32) t.solver = KWG_SOLVER_PCR;
     else if (p->solver != KWG_SOLVER_AUTO) t.solver = p->solver;
+    if (pair64_ok(p)) {
+        kwg::Fp64Batch b(std::isinf(p->density));
+        b.add(m, p->x_dim, p->t_dim - 1, left);
+        const bool open = p->solver == KWG_SOLVER_AUTO && (!recorded || (left > 0 && t.solver == KWG_SOLVER_PCR));
+        if (open) t.solver = b.best() == kwg::Fp64Route::kStream ? KWG_SOLVER_THOMAS : KWG_SOLVER_PCR;
+        t.fp64_steps = t.solver == KWG_SOLVER_PCR && left > 0 && b.on_chip_ns() < b.pair_ns();
+    }
     // an explicit block size or residency replaces the recorded pair (the tuner timed
     // every block size at full residency)
     if (p->block_warps || p->sm_blocks) {
@@ -276,7 +279,7 @@ kwg_ctx::Tuned choose(kwg_ctx* ctx, const kwg_fd1d_params* p, int m)
 }
 
 int run_batch(kwg_ctx* ctx, char* io, const IoLayout& L, int m, int n, const kwg_fd1d_params* p,
-              double* prices, int32_t* status, cudaStream_t stream, int twin_tiles = 0)
+              double* prices, int32_t* status, cudaStream_t stream, int twin_tiles = 0, int left = 0)
 {
     const int m_pad = (m + kwg::kTile - 1) / kwg::kTile * kwg::kTile;
     kwg::PdeBatch b;
@@ -295,7 +298,7 @@ int run_batch(kwg_ctx* ctx, char* io, const IoLayout& L, int m, int n, const kwg
     a.n = n;
     kwg::Fd1dShape sh = make_shape(p);
     sh.twin_tiles = twin_tiles;
-    const kwg_ctx::Tuned tn = choose(ctx, p, m);
+    const kwg_ctx::Tuned tn = choose(ctx, p, m, left);
     const int solver = tn.solver;
     sh.block_warps = tn.block_warps;
     sh.option_warps = tn.option_warps;
@@ -304,9 +307,12 @@ int run_batch(kwg_ctx* ctx, char* io, const IoLayout& L, int m, int n, const kwg
         const long long nodes = (long long)m * sh.x_dim;
         if (int rc = ensure_device(ctx, &ctx->d_work, &ctx->work_bytes, kwg::fd1d_pair64_work_bytes(m, nodes))) return rc;
         double* v = (double*)ctx->d_work;
-        const int n_launch = kwg::fd1d_pair64_launch(b, a, sh, v, (int32_t*)(v + nodes), (int32_t*)(io + L.pde_status),
-                                                     ctx->d_counter, prices, status, ctx->device, stream,
-                                                     ctx->next_events());
+        int32_t* const pde_status = (int32_t*)(io + L.pde_status);
+        const int n_launch =
+            tn.fp64_steps ? kwg::fd1d_pcr64_half_launch(b, a, sh, v, pde_status, ctx->d_counter, prices, status,
+                                                        ctx->device, stream, ctx->next_events())
+                          : kwg::fd1d_pair64_launch(b, a, sh, v, (int32_t*)(v + nodes), pde_status, ctx->d_counter, prices,
+                                                    status, ctx->device, stream, ctx->next_events());
         if (n_launch < 0) return set_err(ctx, KWG_ERR_INVALID, "kwg: the on-chip FP64 solver supports x_dim <= 2048");
         ctx->launches += n_launch;
     } else if (p->precision == KWG_FP64 && solver == KWG_SOLVER_PCR) {
@@ -422,8 +428,10 @@ int price_host(kwg_ctx* ctx, const kwg_option* user_opts, size_t n_user, const k
     double *t = (double*)(h + L.t), *z = (double*)(h + L.z), *r = (double*)(h + L.r), *q = (double*)(h + L.q);
     int8_t* w = (int8_t*)(h + L.w);
     uint8_t* e = (uint8_t*)(h + L.e);
+    int left = 0;
     for (size_t j = 0; j < m; ++j) {
         const kwg_option& o = opts[pde2asset[j]];
+        left += kwg::pair64_leaves(o.t, o.z, o.r, o.q, o.w, p->scale);
         t[j] = o.t;
         z[j] = o.z;
         r[j] = o.r;
@@ -443,7 +451,7 @@ int price_host(kwg_ctx* ctx, const kwg_option* user_opts, size_t n_user, const k
     // 3. kernels
     char* dio = (char*)ctx->d_io;
     if (int rc = run_batch(ctx, dio, L, (int)m, (int)n, p, (double*)(dio + L.prices), (int32_t*)(dio + L.status),
-                           ctx->stream, twin_tiles))
+                           ctx->stream, twin_tiles, left))
         return rc;
     if (control_variate) {
         bs_control_variate<<<(unsigned)((n_user + 255) / 256), 256, 0, ctx->stream>>>(

@@ -50,6 +50,7 @@ struct kwg_ctx {
         int block_warps = 1;
         int option_warps = 0;  // 0: by the batch size
         int sm_blocks = 0;
+        bool fp64_steps = false;  // on chip at theta = 1/2: FP64 stepping instead of pair arithmetic
     };
     std::map<uint64_t, Tuned> tuned;
     // solve-kernel timing (kwg_set_profiling)

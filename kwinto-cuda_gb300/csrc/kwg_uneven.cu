@@ -72,6 +72,11 @@ UnevenLayout uneven_layout(size_t m, size_t n, size_t ntiles)
     return L;
 }
 
+bool leaves(const kwg_option& o, const kwg_fd1d_params& q)
+{
+    return kwg::pair64_leaves(o.t, o.z, o.r, o.q, o.w, q.scale);
+}
+
 // Warp-per-PDE solvers.  Preparing a batch (dedup, sort by work, packing) takes the host ~85 ns per
 // option: 11 of the 52 ms of 131072 options in FP32 when the whole batch was prepared before
 // the first kernel, and the solves of the buckets waited for one another's last PDEs.  By buckets, all but the
@@ -152,8 +157,10 @@ int price_buckets(kwg_ctx* ctx, const kwg_option* opts, const int32_t* x_dims, c
         kv.resize(m);
         int x_max = 0, x_min = INT32_MAX;
         long long nodes = 0;
+        kwg::Fp64Batch costs(std::isinf(q.density));
         for (size_t i = 0; i < m; ++i) {
             const int x = x_dims[pde2asset[i]];
+            if (pair) costs.add(1, x, t_dims[pde2asset[i]] - 1, leaves(opts[pde2asset[i]], q));
             kv[i] = {((1ull << 50) - 1) - (uint64_t)x * (uint64_t)(t_dims[pde2asset[i]] - 1), (uint32_t)i};
             x_max = std::max(x_max, x);
             x_min = std::min(x_min, x);
@@ -219,8 +226,11 @@ int price_buckets(kwg_ctx* ctx, const kwg_option* opts, const int32_t* x_dims, c
         const cudaStream_t st = ctx->profiling ? ctx->stream : bk.stream;
         KWG_CUDA(ctx, cudaMemcpyAsync(io, h, L.in_bytes, cudaMemcpyHostToDevice, st));
         const kwg::SolveEvents* ev = ctx->next_events();
+        const bool fp64_steps = pair && costs.any_left() && costs.on_chip_ns() < costs.pair_ns();
         const int r =
-            pair ? kwg::fd1d_pair64_launch(b, a, sh, v, (int32_t*)(v + nodes), d_pde_status, d_counters, d_prices,
+            fp64_steps ? kwg::fd1d_pcr64_half_launch(b, a, sh, v, d_pde_status, d_counters, d_prices, d_status,
+                                                     ctx->device, st, ev)
+            : pair ? kwg::fd1d_pair64_launch(b, a, sh, v, (int32_t*)(v + nodes), d_pde_status, d_counters, d_prices,
                                            d_status, ctx->device, st, ev)
             : q.precision == KWG_FP32 ? kwg::fd1d_fp32_launch(b, a, sh, v, d_pde_status, d_counters, d_prices,
                                                               d_status, ctx->device, st, ev)
@@ -277,14 +287,6 @@ int check_strict(kwg_ctx* ctx, const int32_t* status, size_t n)
     return KWG_OK;
 }
 
-// The FP64 solver of an uneven batch at theta = 1/2, every option a PDE of its own.
-kwg::Fp64Route uneven_route(const int32_t* x_dims, const int32_t* t_dims, size_t n, const kwg_fd1d_params& q)
-{
-    kwg::Fp64Batch b(std::isinf(q.density));
-    for (size_t i = 0; i < n; ++i) b.add(1, x_dims[i], t_dims[i] - 1);
-    return b.best();
-}
-
 uint64_t mix(uint64_t h, uint64_t v)
 {
     h ^= v + 0x9e3779b97f4a7c15ull + (h << 6) + (h >> 2);
@@ -323,14 +325,25 @@ extern "C" int kwg_fd1d_price_uneven(kwg_ctx* ctx, const kwg_option* opts, const
     // launch choices: the explicit ones, else what kwg_autotune_uneven recorded for
     // uneven batches of this precision and size, else the on-chip solvers with warps by the
     // bucket's size, or (theta != 1/2, more than 2048 nodes, and where the cost model of fp64_route.h
-    // says so) Thomas with one warp per block
+    // says so) Thomas.  PDEs left over by pair arithmetic bring the model in where that is recorded too.
     kwg_ctx::Tuned tn;
     {
         const auto it = ctx->tuned.find(tune_key(q.precision, 0, 0, (long long)n));
-        if (it != ctx->tuned.end())
-            tn = it->second;
-        else if (q.solver == KWG_SOLVER_AUTO && pair64_ok(&q) && uneven_route(x_dims, t_dims, n, q) != kwg::Fp64Route::kStream)
+        const bool recorded = it != ctx->tuned.end();
+        if (recorded) tn = it->second;
+        if (q.solver == KWG_SOLVER_AUTO && pair64_ok(&q) && !(recorded && tn.solver == KWG_SOLVER_THOMAS)) {
+            // every option a PDE of its own
+            kwg::Fp64Batch b(std::isinf(q.density));
+            for (size_t i = 0; i < n; ++i) b.add(1, x_dims[i], t_dims[i] - 1, leaves(opts[i], q));
             tn.solver = KWG_SOLVER_PCR;
+            if ((!recorded || b.any_left()) && b.best() == kwg::Fp64Route::kStream) {
+                tn.solver = KWG_SOLVER_THOMAS;
+                if (b.few_long_chains()) {
+                    tn.block_warps = 4;
+                    tn.sm_blocks = 1;
+                }
+            }
+        }
         if (q.precision == KWG_FP64 && q.solver == KWG_SOLVER_AUTO &&
             (tn.solver != KWG_SOLVER_PCR || pair64_ok(&q) || kwg::fd1d_pcr64_nodes_per_lane(x_max) > 0))
             q.solver = tn.solver;

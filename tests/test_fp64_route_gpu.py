@@ -1,6 +1,7 @@
 """Which FP64 solver KWG_SOLVER_AUTO takes at theta = 1/2: many PDEs of few nodes and few steps on ragged
-uniform grids stream, all else runs on chip, in the uniform and the uneven call alike.  The routes are
-told apart by their bits: streaming lanes and on-chip PDEs do not depend on their neighbours."""
+uniform grids stream, all else runs on chip, in the uniform and the uneven call alike; batches with
+many PDEs that pair arithmetic leaves over are stepped in FP64.  The routes are told apart by their bits (streaming
+lanes and on-chip PDEs do not depend on their neighbours) and launches (pair arithmetic 3, FP64 on chip 2)."""
 import math
 
 import numpy as np
@@ -55,5 +56,65 @@ def test_uneven_auto_takes_the_faster_solver(built, n, nodes, levels, streams):
             assert rc == kwg.KWG_OK, c.last_error()
         assert not np.array_equal(got[1], got[2], equal_nan=True)
         assert np.array_equal(got[0], got[1] if streams else got[2], equal_nan=True)
+    finally:
+        c.close()
+
+
+def drifting(n, share, seed=4):
+    """`share` of the options with a drift of more than 0.3 half-widths of a grid at scale 5."""
+    import portfolio
+
+    o = portfolio.american_portfolio(n, seed=seed)
+    k = portfolio.uniforms(seed, 40, n) < share
+    o["z"][k], o["r"][k], o["q"][k], o["t"][k] = 0.03, 0.08, 0.0, 1.5
+    o["t"][k] += np.arange(k.sum()) * 1e-4  # PDEs of their own
+    o["s"] = o["k"]
+    return o
+
+
+@pytest.mark.parametrize("n,x_dim,t_dim,share,route", [
+    (20000, 65, 40, 1.0, "stream"), (12000, 300, 12, 0.9, "stream"), (300, 512, 40, 0.1, "fp64"), (60, 1500, 20, 0.2, "fp64"),
+    (2000, 256, 40, 1.0, "fp64"), (6000, 512, 60, 0.05, "pair")])
+@pytest.mark.parametrize("entry", ["host", "bs"])
+def test_batches_crossed_by_their_drift(built, entry, n, x_dim, t_dim, share, route):
+    import kwg
+
+    c = kwg.Context(0)
+    try:
+        o = drifting(n // 2 if entry == "bs" else n, share)
+        call = c.fd1d_bs_price if entry == "bs" else c.fd1d_price
+        kw = dict(t_dim=t_dim, x_dim=x_dim, scale=5.0, density=math.inf)
+        rc, p, st = call(o, kwg.params(**kw))
+        assert rc == kwg.KWG_OK, c.last_error()
+        launches = c.launch_count() - (entry == "bs")
+        rc, want, wst = call(o, kwg.params(solver=kwg.SOLVER_THOMAS, **kw))
+        assert rc == kwg.KWG_OK and np.array_equal(st, wst)
+        ok = st == 0
+        assert ok.all()
+        assert np.max(np.abs(p - want) / np.maximum(1e-10 * np.abs(want), 1e-13 * o["k"])) <= 1.0
+        if route == "stream":
+            assert np.array_equal(p, want)
+        else:
+            assert not np.array_equal(p, want) and launches == (2 if route == "fp64" else 3)
+    finally:
+        c.close()
+
+
+@pytest.mark.parametrize("n,share,streams", [(30000, 1.0, True), (30000, 0.02, False)])
+def test_uneven_batches_crossed_by_their_drift(built, n, share, streams):
+    import kwg
+
+    c = kwg.Context(0)
+    try:
+        rng = np.random.default_rng(n)
+        o = drifting(n, share)
+        x, t = (rng.integers(*r, n).astype(np.int32) for r in ((90, 140), (20, 50)))
+        got = {}
+        for s in (kwg.SOLVER_AUTO, kwg.SOLVER_THOMAS, kwg.SOLVER_PCR):
+            rc, got[s], _ = c.fd1d_price_uneven(o, x, t, kwg.params(scale=5.0, density=math.inf, solver=s))
+            assert rc == kwg.KWG_OK, c.last_error()
+        assert not np.array_equal(got[1], got[2])
+        assert np.array_equal(got[0], got[1] if streams else got[2])
+        assert np.max(np.abs(got[0] - got[1]) / np.maximum(1e-10 * np.abs(got[1]), 1e-13 * o["k"])) <= 1.0
     finally:
         c.close()
