@@ -31,7 +31,7 @@ __global__ void fd1d_interp_rows(const PdeBatch b, const AssetBatch a, Fd1dShape
                                  int32_t* __restrict__ status)
 {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= a.n) return;
+    if (i >= a.n || (sh.left_streams && many_left(sh))) return;
     const int slot = a.pde[i];
     const int N = shape_x(sh, slot);
     const double s = a.s[i], k = a.k[i];

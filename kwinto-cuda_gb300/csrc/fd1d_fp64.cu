@@ -322,7 +322,7 @@ __global__ void __launch_bounds__(128) fd1d_setup_fp64(const PdeBatch b, Fd1dSha
                                                        int32_t* __restrict__ pde_status)
 {
     const int slot = blockIdx.x * blockDim.x + threadIdx.x;
-    if (slot >= b.m_pad) return;  // whole warps: m_pad is a multiple of the tile
+    if (slot >= b.m_pad || (sh.left && !many_left(sh))) return;  // whole warps: m_pad is a multiple of the tile
     const int src = slot < b.m ? slot : b.m - 1;  // padding lanes replicate the last PDE
     const int tile = slot / kTile, lane = slot % kTile;
     int N;
@@ -744,6 +744,7 @@ __global__ void __launch_bounds__(32 * kMaxBlockWarps)
     fd1d_solve_fp64(const PdeBatch b, Fd1dShape sh, double* __restrict__ base, int* __restrict__ tile_counter)
 {
     using G = Geo<kBig>;
+    if (sh.left && !many_left(sh)) return;
     extern __shared__ __align__(128) unsigned char smem[];
     Ring ring;
     ring.stage = smem + (size_t)(threadIdx.x >> 5) * G::kSolveSmem;
@@ -835,7 +836,7 @@ __global__ void fd1d_interp_fp64(const PdeBatch b, const AssetBatch a, Fd1dShape
                                  double* __restrict__ prices, int32_t* __restrict__ status)
 {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= a.n) return;
+    if (i >= a.n || (sh.left && !many_left(sh))) return;
     const int slot = a.pde[i];
     int N;
     long long toff;

@@ -68,7 +68,15 @@ struct Fd1dShape {
     // each -- an American PDE in the even lane, its European copy (same t, r, q, z, w)
     // in the odd lane -- which read one shared record of coefficients and payoff
     int twin_tiles = 0;
+    // device calls at theta = 1/2: the number of PDEs that pair arithmetic leaves over, which only the
+    // device knows.  The batch is launched for both of its solvers (fp64_route.h): below left_from pair
+    // arithmetic runs and the other launch ends at once; from there on the other way round.
+    const int* left = nullptr;
+    int left_from = 0;
+    bool left_streams = false;  // the other is the streaming solver (else the warp-per-PDE FP64 kernel)
 };
+
+__device__ inline bool many_left(const Fd1dShape& sh) { return sh.left && *sh.left >= sh.left_from; }
 
 __host__ __device__ inline int shape_x(const Fd1dShape& sh, int pde) { return sh.pde_x ? sh.pde_x[pde] : sh.x_dim; }
 __host__ __device__ inline int shape_t(const Fd1dShape& sh, int pde) { return sh.pde_t ? sh.pde_t[pde] : sh.t_dim; }
@@ -141,11 +149,13 @@ int fd1d_pair64_launch(const PdeBatch& b, const AssetBatch& a, const Fd1dShape& 
 // class (European puts, European calls, American puts, American calls) so that the
 // streaming FP64 solver's tiles are homogeneous; the slot order inside a class is
 // arrival order.  counts: 8 ints (per-class counts, cursors), zeroed here on
-// `stream`.  Two launches; returns the first CUDA error.
+// `stream`.  left: counts + 8, the number of PDEs for which pair64_leaves holds at `scale`, or nullptr.
+// Two launches; returns the first CUDA error.
 cudaError_t unpack_by_class(const void* d_opts, int n, int* counts, double* t, double* z, double* r, double* q,
-                            double* s, double* k, int32_t* pde, int8_t* w, uint8_t* e, cudaStream_t stream);
+                            double* s, double* k, int32_t* pde, int8_t* w, uint8_t* e, int* left, double scale,
+                            cudaStream_t stream);
 
-// Interpolation over a [m][x_dim] array of final values (FP32 and PCR paths).
+// Interpolation over a [m][x_dim] array of final values (the on-chip solvers).
 __global__ void fd1d_interp_rows(const PdeBatch b, const AssetBatch a, Fd1dShape sh, const double* __restrict__ vrow,
                                  const int32_t* __restrict__ pde_status, double* __restrict__ prices,
                                  int32_t* __restrict__ status);

@@ -312,6 +312,8 @@ __global__ void __launch_bounds__(32 * W, budget(M, W, kUni, kPair).warps / W)
     // row of slot kk in the coefficient tables (uniform grids of full lanes keep slots 0, P-1)
     auto crow = [](int kk) { return kUni ? (kk == 0 ? 0 : Y::S - 1) : kk; };
 
+    if (kPair && many_left(sh)) return;
+
     for (;;) {
         int pde = 0;
         if constexpr (W == 1) {

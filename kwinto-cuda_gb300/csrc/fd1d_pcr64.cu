@@ -53,6 +53,10 @@ __global__ void __launch_bounds__(32) fd1d_solve_fp64_pcr(const PdeBatch b, Fd1d
                                                           int32_t* __restrict__ pde_status,
                                                           int* __restrict__ counters, const int32_t* __restrict__ list)
 {
+    if (many_left(sh)) {  // pair arithmetic has not run: all PDEs are this kernel's, or the streaming solver's
+        if (sh.left_streams) return;
+        list = nullptr;
+    }
     extern __shared__ double qtab[];  // [M][kP64Fields][32], or (kShared) [M][32] + [M][5][2]
     const int k = threadIdx.x & 31;
     // this lane's copy of the shared factors: +1 for lane 31 only (arithmetic, so

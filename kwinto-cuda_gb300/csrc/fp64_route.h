@@ -79,9 +79,9 @@ struct Fp64Batch {
     // the warp-per-PDE FP64 kernel
     void add_fp64(Cost& c, const Kind& d, int k) const
     {
+        constexpr double kStep[kSizes] = {1.45, 2., 3.4, 6., 14.5, 59.};  // 2048 nodes: 64 per lane, spills
         const double n = 64 << k;
-        c.sum += 0.16 * n * (double)d.n +
-                 (uniform ? 1. : 1.12) * (n > 1024. ? 0.029 * n : 0.5 + 0.0135 * n) * (double)d.steps;
+        c.sum += 0.16 * n * (double)d.n + (uniform ? 1. : 1.12) * kStep[k] * (double)d.steps;
         c.longest = std::max(c.longest, d.longest * (1200. + 8.8 * n) * (d.n > 304 ? 1.25 : 1.));
     }
     double pair_ns() const
@@ -139,5 +139,26 @@ struct Fp64Batch {
         return stream_ns() < p ? Fp64Route::kStream : Fp64Route::kPair;
     }
 };
+
+// A batch of m PDEs of x nodes and s steps on the device, where the number left over is known later: from how
+// many of them on another solver takes it (m + 1: none), and which.  The cost of pair arithmetic
+// grows with that number, the others' do not depend on it.
+inline long long pair64_limit(long long m, int x, int s, bool uniform, bool may_stream, Fp64Route* instead)
+{
+    auto route = [&](long long left) {
+        Fp64Batch b(uniform);
+        b.add(m, x, s, left);
+        if (may_stream) return b.best();
+        return left > 0 && b.on_chip_ns() < b.pair_ns() ? Fp64Route::kOnChip : Fp64Route::kPair;
+    };
+    long long lo = 1, hi = m + 1;
+    while (lo < hi) {
+        const long long mid = (lo + hi) / 2;
+        if (route(mid) != Fp64Route::kPair) hi = mid;
+        else lo = mid + 1;
+    }
+    *instead = lo <= m ? route(lo) : Fp64Route::kPair;
+    return lo;
+}
 
 }  // namespace kwg

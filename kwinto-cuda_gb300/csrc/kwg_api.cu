@@ -96,13 +96,25 @@ __global__ void bs_control_variate(int n, const double* __restrict__ s, const do
 // where it is zero for every lane (kernels are indifferent to the PDE order).
 __host__ __device__ inline int pde_class(uint8_t e, int8_t w) { return (e ? 2 : 0) + (w < 0 ? 0 : 1); }
 
-// Device path, pass 1: PDEs per class (warp-aggregated atomics).
-__global__ void count_classes(const kwg_option* __restrict__ o, int n, int* __restrict__ counts)
+// PDEs per class, and those that pair arithmetic leaves over (warp-aggregated atomics; every lane
+// of the warp calls, c < 0 for none).
+__device__ void count_pde(const kwg_option* __restrict__ o, int i, int c, int* __restrict__ counts, int* __restrict__ left,
+                          double scale)
 {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    const int c = i < n ? pde_class(o[i].e, o[i].w) : -1;
     const unsigned peers = __match_any_sync(0xffffffffu, c);
     if (c >= 0 && (threadIdx.x & 31) == __ffs(peers) - 1) atomicAdd(&counts[c], __popc(peers));
+    if (!left) return;
+    const unsigned l =
+        __ballot_sync(0xffffffffu, c >= 0 && kwg::pair64_leaves(o[i].t, o[i].z, o[i].r, o[i].q, o[i].w, scale));
+    if (l && (threadIdx.x & 31) == 0) atomicAdd(left, __popc(l));
+}
+
+// Device path, pass 1.
+__global__ void count_classes(const kwg_option* __restrict__ o, int n, int* __restrict__ counts, int* __restrict__ left,
+                              double scale)
+{
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    count_pde(o, i, i < n ? pde_class(o[i].e, o[i].w) : -1, counts, left, scale);
 }
 
 // Device path, pass 2: AoS options -> the SoA arrays of one packed buffer, each PDE
@@ -177,12 +189,10 @@ __global__ void dedup_insert(const kwg_option* __restrict__ o, int n, unsigned* 
 
 // Owners per class, like count_classes.
 __global__ void dedup_count(const kwg_option* __restrict__ o, int n, const int* __restrict__ owner,
-                            int* __restrict__ counts)
+                            int* __restrict__ counts, int* __restrict__ left, double scale)
 {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    const int c = (i < n && owner[i] == i) ? pde_class(o[i].e, o[i].w) : -1;
-    const unsigned peers = __match_any_sync(0xffffffffu, c);
-    if (c >= 0 && (threadIdx.x & 31) == __ffs(peers) - 1) atomicAdd(&counts[c], __popc(peers));
+    count_pde(o, i, (i < n && owner[i] == i) ? pde_class(o[i].e, o[i].w) : -1, counts, left, scale);
 }
 
 // Owners become PDEs at class offset + arrival slot; every option keeps its s, k.
@@ -278,8 +288,9 @@ kwg_ctx::Tuned choose(kwg_ctx* ctx, const kwg_fd1d_params* p, int m, int left)
     return t;
 }
 
+// left: PDEs that pair arithmetic would leave over; d_left: their number is there, on the device.
 int run_batch(kwg_ctx* ctx, char* io, const IoLayout& L, int m, int n, const kwg_fd1d_params* p,
-              double* prices, int32_t* status, cudaStream_t stream, int twin_tiles = 0, int left = 0)
+              double* prices, int32_t* status, cudaStream_t stream, int twin_tiles, int left, const int* d_left)
 {
     const int m_pad = (m + kwg::kTile - 1) / kwg::kTile * kwg::kTile;
     kwg::PdeBatch b;
@@ -305,15 +316,39 @@ int run_batch(kwg_ctx* ctx, char* io, const IoLayout& L, int m, int n, const kwg
     sh.sm_blocks = tn.sm_blocks;
     if (solver == KWG_SOLVER_PCR && pair64_ok(p)) {
         const long long nodes = (long long)m * sh.x_dim;
-        if (int rc = ensure_device(ctx, &ctx->d_work, &ctx->work_bytes, kwg::fd1d_pair64_work_bytes(m, nodes))) return rc;
+        const size_t bytes = kwg::fd1d_pair64_work_bytes(m, nodes), stream_bytes = kwg::fd1d_fp64_work_bytes(m_pad, sh.x_dim);
+        if (d_left) {
+            kwg::Fp64Route other;
+            const long long from =
+                kwg::pair64_limit(m, sh.x_dim, sh.t_dim - 1, sh.uniform, p->solver == KWG_SOLVER_AUTO, &other);
+            if (from <= m) {
+                sh.left = d_left;
+                sh.left_from = (int)from;
+                sh.left_streams = other == kwg::Fp64Route::kStream;
+            }
+        }
+        // a device without room for the streaming solver's work arrays keeps to pair arithmetic
+        if (sh.left_streams && ensure_device(ctx, &ctx->d_work, &ctx->work_bytes, std::max(bytes, stream_bytes))) {
+            ctx->err.clear();
+            cudaGetLastError();
+            sh.left = nullptr;
+            sh.left_streams = false;
+        }
+        if (int rc = ensure_device(ctx, &ctx->d_work, &ctx->work_bytes, bytes)) return rc;
         double* v = (double*)ctx->d_work;
         int32_t* const pde_status = (int32_t*)(io + L.pde_status);
-        const int n_launch =
+        const kwg::SolveEvents* ev = ctx->next_events();
+        int n_launch =
             tn.fp64_steps ? kwg::fd1d_pcr64_half_launch(b, a, sh, v, pde_status, ctx->d_counter, prices, status,
-                                                        ctx->device, stream, ctx->next_events())
+                                                        ctx->device, stream, ev)
                           : kwg::fd1d_pair64_launch(b, a, sh, v, (int32_t*)(v + nodes), pde_status, ctx->d_counter, prices,
-                                                    status, ctx->device, stream, ctx->next_events());
+                                                    status, ctx->device, stream, ev);
         if (n_launch < 0) return set_err(ctx, KWG_ERR_INVALID, "kwg: the on-chip FP64 solver supports x_dim <= 2048");
+        if (sh.left_streams) {
+            const int blocks = kwg::fd1d_fp64_solve_blocks(m_pad / kwg::kTile, ctx->device, sh.block_warps, sh.sm_blocks);
+            n_launch += kwg::fd1d_fp64_launch(b, a, sh, v, pde_status, ctx->d_counter, prices, status, blocks, stream, nullptr);
+            if (ev) cudaEventRecord(ev->stop, stream);
+        }
         ctx->launches += n_launch;
     } else if (p->precision == KWG_FP64 && solver == KWG_SOLVER_PCR) {
         const size_t wbytes = kwg::fd1d_fp32_work_bytes(m, sh.x_dim);
@@ -451,7 +486,7 @@ int price_host(kwg_ctx* ctx, const kwg_option* user_opts, size_t n_user, const k
     // 3. kernels
     char* dio = (char*)ctx->d_io;
     if (int rc = run_batch(ctx, dio, L, (int)m, (int)n, p, (double*)(dio + L.prices), (int32_t*)(dio + L.status),
-                           ctx->stream, twin_tiles, left))
+                           ctx->stream, twin_tiles, left, nullptr))
         return rc;
     if (control_variate) {
         bs_control_variate<<<(unsigned)((n_user + 255) / 256), 256, 0, ctx->stream>>>(
@@ -495,18 +530,18 @@ int price_device_dedup(kwg_ctx* ctx, const kwg_option* d_opts, size_t n, size_t 
     const IoLayout L = io_layout(n, n_pad, n);
     unsigned cap = 64;
     while (cap < 2 * n) cap <<= 1;
-    const size_t extra = 8 * sizeof(int) + (size_t)cap * sizeof(unsigned) + 2 * n * sizeof(int);
+    const size_t extra = 12 * sizeof(int) + (size_t)cap * sizeof(unsigned) + 2 * n * sizeof(int);
     if (int rc = ensure_device(ctx, &ctx->d_io, &ctx->io_bytes, L.total + extra)) return rc;
     if (int rc = ensure_host(ctx, &ctx->h_io, &ctx->h_io_bytes, 64)) return rc;
     char* io = (char*)ctx->d_io;
-    int* counts = (int*)(io + L.total);  // [4] per-class counts, [4] cursors
-    unsigned* table = (unsigned*)(counts + 8);
+    int* counts = (int*)(io + L.total);  // [4] per-class counts, [4] cursors, PDEs left over by pair arithmetic
+    unsigned* table = (unsigned*)(counts + 12);
     int* owner = (int*)(table + cap);
     int* slot_of = owner + n;
-    KWG_CUDA(ctx, cudaMemsetAsync(counts, 0, 8 * sizeof(int) + (size_t)cap * sizeof(unsigned), stream));
+    KWG_CUDA(ctx, cudaMemsetAsync(counts, 0, 12 * sizeof(int) + (size_t)cap * sizeof(unsigned), stream));
     const unsigned nb = (unsigned)((n + 255) / 256);
     dedup_insert<<<nb, 256, 0, stream>>>(d_opts, (int)n, table, cap - 1, owner);
-    dedup_count<<<nb, 256, 0, stream>>>(d_opts, (int)n, owner, counts);
+    dedup_count<<<nb, 256, 0, stream>>>(d_opts, (int)n, owner, counts, counts + 8, p->scale);
     dedup_unpack<<<nb, 256, 0, stream>>>(d_opts, (int)n, owner, counts, counts + 4, slot_of, (double*)(io + L.t),
                                          (double*)(io + L.z), (double*)(io + L.r), (double*)(io + L.q),
                                          (double*)(io + L.s), (double*)(io + L.k), (int8_t*)(io + L.w),
@@ -514,10 +549,10 @@ int price_device_dedup(kwg_ctx* ctx, const kwg_option* d_opts, size_t n, size_t 
     dedup_map<<<nb, 256, 0, stream>>>((int)n, owner, slot_of, (int32_t*)(io + L.pde));
     ctx->launches += 4;
     int* hc = (int*)ctx->h_io;
-    KWG_CUDA(ctx, cudaMemcpyAsync(hc, counts, 4 * sizeof(int), cudaMemcpyDeviceToHost, stream));
+    KWG_CUDA(ctx, cudaMemcpyAsync(hc, counts, 9 * sizeof(int), cudaMemcpyDeviceToHost, stream));
     KWG_CUDA(ctx, cudaStreamSynchronize(stream));
     const int m = hc[0] + hc[1] + hc[2] + hc[3];
-    return run_batch(ctx, io, L, m, (int)n, p, d_prices, d_status, stream);
+    return run_batch(ctx, io, L, m, (int)n, p, d_prices, d_status, stream, 0, hc[8], nullptr);
 }
 
 // Synthetic batch of m options for the autotuner: puts and calls, strikes 80..120,
@@ -537,12 +572,13 @@ std::vector<kwg_option> tuning_batch(size_t m)
 }  // namespace
 
 cudaError_t kwg::unpack_by_class(const void* d_opts, int n, int* counts, double* t, double* z, double* r, double* q,
-                                 double* s, double* k, int32_t* pde, int8_t* w, uint8_t* e, cudaStream_t stream)
+                                 double* s, double* k, int32_t* pde, int8_t* w, uint8_t* e, int* left, double scale,
+                                 cudaStream_t stream)
 {
-    if (cudaError_t ce = cudaMemsetAsync(counts, 0, 8 * sizeof(int), stream); ce != cudaSuccess) return ce;
+    if (cudaError_t ce = cudaMemsetAsync(counts, 0, (left ? 9 : 8) * sizeof(int), stream); ce != cudaSuccess) return ce;
     const kwg_option* o = (const kwg_option*)d_opts;
     const unsigned nb = (unsigned)((n + 255) / 256);
-    count_classes<<<nb, 256, 0, stream>>>(o, n, counts);
+    count_classes<<<nb, 256, 0, stream>>>(o, n, counts, left, scale);
     unpack_options<<<nb, 256, 0, stream>>>(o, n, counts, counts + 4, t, z, r, q, s, k, pde, w, e);
     return cudaGetLastError();
 }
@@ -742,15 +778,15 @@ int kwg_fd1d_price_device(kwg_ctx* ctx, const kwg_option* d_opts, size_t n, cons
     if (p->device_dedup) return price_device_dedup(ctx, d_opts, n, n_pad, p, d_prices, d_status, stream);
     const size_t m = n, m_pad = n_pad;
     const IoLayout L = io_layout(m, m_pad, n);
-    if (int rc = ensure_device(ctx, &ctx->d_io, &ctx->io_bytes, L.total + 8 * sizeof(int))) return rc;
+    if (int rc = ensure_device(ctx, &ctx->d_io, &ctx->io_bytes, L.total + 12 * sizeof(int))) return rc;
     char* io = (char*)ctx->d_io;
-    int* counts = (int*)(io + L.total);  // [4] per-class counts, [4] cursors
+    int* counts = (int*)(io + L.total);  // [4] per-class counts, [4] cursors, PDEs left over by pair arithmetic
     KWG_CUDA(ctx, kwg::unpack_by_class(d_opts, (int)n, counts, (double*)(io + L.t), (double*)(io + L.z),
                                        (double*)(io + L.r), (double*)(io + L.q), (double*)(io + L.s),
                                        (double*)(io + L.k), (int32_t*)(io + L.pde), (int8_t*)(io + L.w),
-                                       (uint8_t*)(io + L.e), stream));
+                                       (uint8_t*)(io + L.e), counts + 8, p->scale, stream));
     ctx->launches += 2;
-    return run_batch(ctx, io, L, (int)m, (int)n, p, d_prices, d_status, stream);
+    return run_batch(ctx, io, L, (int)m, (int)n, p, d_prices, d_status, stream, 0, 0, counts + 8);
 }
 
 }  // extern "C"

@@ -179,7 +179,7 @@ extern "C" int kwg_fd1d_price_device_static(const kwg_option* d_opts, size_t n, 
     cudaStream_t st = (cudaStream_t)stream;
     int dev = 0;
     cudaGetDevice(&dev);
-    if (cudaError_t ce = kwg::unpack_by_class(d_opts, (int)n, classes, t, z, r, q, sp, k, pde, w, e, st);
+    if (cudaError_t ce = kwg::unpack_by_class(d_opts, (int)n, classes, t, z, r, q, sp, k, pde, w, e, nullptr, p->scale, st);
         ce != cudaSuccess) {
         put(err, errlen, cudaGetErrorString(ce));
         return KWG_ERR_CUDA;

@@ -118,3 +118,31 @@ def test_uneven_batches_crossed_by_their_drift(built, n, share, streams):
         assert np.max(np.abs(got[0] - got[1]) / np.maximum(1e-10 * np.abs(got[1]), 1e-13 * o["k"])) <= 1.0
     finally:
         c.close()
+
+
+@pytest.mark.parametrize("n,x_dim,t_dim,share", [(20000, 65, 40, 1.0), (12000, 300, 12, 0.9), (300, 512, 40, 0.1),
+                                                 (60, 1500, 20, 0.2), (6000, 512, 60, 0.05), (20000, 65, 40, 0.01)])
+@pytest.mark.parametrize("dedup", [0, 1])
+def test_device_calls_choose_as_host_calls(built, n, x_dim, t_dim, share, dedup):
+    """Bit for bit, also when the next batch on the same buffers takes the other route."""
+    import kwg
+    import torch
+
+    c = kwg.Context(0)
+    try:
+        prm = kwg.params(t_dim=t_dim, x_dim=x_dim, scale=5.0, density=math.inf)
+        prm.device_dedup = dedup
+        price = torch.empty(n, dtype=torch.float64, device="cuda")
+        status = torch.empty(n, dtype=torch.int32, device="cuda")
+        for s in (share, 0.0, share):
+            o = drifting(n, s)
+            rc, want, wst = c.fd1d_price(o, kwg.params(t_dim=t_dim, x_dim=x_dim, scale=5.0, density=math.inf))
+            assert rc == kwg.KWG_OK
+            d = torch.from_numpy(o.view(np.uint8).copy()).cuda()
+            torch.cuda.synchronize()
+            rc = c.fd1d_price_device(d.data_ptr(), n, prm, price.data_ptr(), status.data_ptr(), 0)
+            assert rc == kwg.KWG_OK, c.last_error()
+            torch.cuda.synchronize()
+            assert np.array_equal(price.cpu().numpy(), want) and np.array_equal(status.cpu().numpy(), wst)
+    finally:
+        c.close()
