@@ -140,6 +140,14 @@ struct Fp64Batch {
     }
 };
 
+// FD1D-BS on small grids with few time levels is stepped in FP64: its American and European solve round alike there,
+// and the errors cancel to 1e-15 to 6e-15 of the price; pair arithmetic's, which do not, are 3e-15 to 8e-15.  Beyond these
+// lines (64 options at scale 5 and 50, 48 to 2048 nodes, 40 to 2048 levels) pair arithmetic is the nearer one.
+inline bool bs_in_fp64(int x, int t_dim, bool uniform)
+{
+    return uniform ? x < 100 && t_dim <= 150 : (x <= 160 && t_dim <= 700) || (x <= 600 && t_dim <= 400);
+}
+
 // A batch of m PDEs of x nodes and s steps on the device, where the number left over is known later: from how
 // many of them on another solver takes it (m + 1: none), and which.  The cost of pair arithmetic
 // grows with that number, the others' do not depend on it.

@@ -255,7 +255,7 @@ __global__ void selftest_waits(int32_t* __restrict__ out, uint32_t limit)
 // recorded (the tuner's batch has none).  Other schemes: the thread-per-option kernel runs m/32 warps, the
 // warp-per-option FP64 kernel m warps at twice the FP64 work per node-step, so the latter wins
 // while m/32 warps cannot fill the GPU.
-kwg_ctx::Tuned choose(kwg_ctx* ctx, const kwg_fd1d_params* p, int m, int left)
+kwg_ctx::Tuned choose(kwg_ctx* ctx, const kwg_fd1d_params* p, int m, int left, bool control_variate)
 {
     kwg_ctx::Tuned t;
     auto it = ctx->tuned.find(tune_key(p->precision, p->x_dim, p->t_dim, m));
@@ -275,8 +275,11 @@ kwg_ctx::Tuned choose(kwg_ctx* ctx, const kwg_fd1d_params* p, int m, int left)
         kwg::Fp64Batch b(std::isinf(p->density));
         b.add(m, p->x_dim, p->t_dim - 1, left);
         const bool open = p->solver == KWG_SOLVER_AUTO && (!recorded || (left > 0 && t.solver == KWG_SOLVER_PCR));
-        if (open) t.solver = b.best() == kwg::Fp64Route::kStream ? KWG_SOLVER_THOMAS : KWG_SOLVER_PCR;
-        t.fp64_steps = t.solver == KWG_SOLVER_PCR && left > 0 && b.on_chip_ns() < b.pair_ns();
+        const bool fp64 = control_variate && p->solver == KWG_SOLVER_AUTO &&
+                          kwg::bs_in_fp64(p->x_dim, p->t_dim, std::isinf(p->density));
+        if (open || (fp64 && t.solver == KWG_SOLVER_PCR))
+            t.solver = (fp64 ? b.fp64() : b.best()) == kwg::Fp64Route::kStream ? KWG_SOLVER_THOMAS : KWG_SOLVER_PCR;
+        t.fp64_steps = t.solver == KWG_SOLVER_PCR && (fp64 || (left > 0 && b.on_chip_ns() < b.pair_ns()));
     }
     // an explicit block size or residency replaces the recorded pair (the tuner timed
     // every block size at full residency)
@@ -290,7 +293,7 @@ kwg_ctx::Tuned choose(kwg_ctx* ctx, const kwg_fd1d_params* p, int m, int left)
 
 // left: PDEs that pair arithmetic would leave over; d_left: their number is there, on the device.
 int run_batch(kwg_ctx* ctx, char* io, const IoLayout& L, int m, int n, const kwg_fd1d_params* p,
-              double* prices, int32_t* status, cudaStream_t stream, int twin_tiles, int left, const int* d_left)
+              double* prices, int32_t* status, cudaStream_t stream, int twin_tiles, int left, const int* d_left, bool control_variate)
 {
     const int m_pad = (m + kwg::kTile - 1) / kwg::kTile * kwg::kTile;
     kwg::PdeBatch b;
@@ -309,7 +312,7 @@ int run_batch(kwg_ctx* ctx, char* io, const IoLayout& L, int m, int n, const kwg
     a.n = n;
     kwg::Fd1dShape sh = make_shape(p);
     sh.twin_tiles = twin_tiles;
-    const kwg_ctx::Tuned tn = choose(ctx, p, m, left);
+    const kwg_ctx::Tuned tn = choose(ctx, p, m, left, control_variate);
     const int solver = tn.solver;
     sh.block_warps = tn.block_warps;
     sh.option_warps = tn.option_warps;
@@ -486,7 +489,7 @@ int price_host(kwg_ctx* ctx, const kwg_option* user_opts, size_t n_user, const k
     // 3. kernels
     char* dio = (char*)ctx->d_io;
     if (int rc = run_batch(ctx, dio, L, (int)m, (int)n, p, (double*)(dio + L.prices), (int32_t*)(dio + L.status),
-                           ctx->stream, twin_tiles, left, nullptr))
+                           ctx->stream, twin_tiles, left, nullptr, control_variate))
         return rc;
     if (control_variate) {
         bs_control_variate<<<(unsigned)((n_user + 255) / 256), 256, 0, ctx->stream>>>(
@@ -552,7 +555,7 @@ int price_device_dedup(kwg_ctx* ctx, const kwg_option* d_opts, size_t n, size_t 
     KWG_CUDA(ctx, cudaMemcpyAsync(hc, counts, 9 * sizeof(int), cudaMemcpyDeviceToHost, stream));
     KWG_CUDA(ctx, cudaStreamSynchronize(stream));
     const int m = hc[0] + hc[1] + hc[2] + hc[3];
-    return run_batch(ctx, io, L, m, (int)n, p, d_prices, d_status, stream, 0, hc[8], nullptr);
+    return run_batch(ctx, io, L, m, (int)n, p, d_prices, d_status, stream, 0, hc[8], nullptr, false);
 }
 
 // Synthetic batch of m options for the autotuner: puts and calls, strikes 80..120,
@@ -786,7 +789,7 @@ int kwg_fd1d_price_device(kwg_ctx* ctx, const kwg_option* d_opts, size_t n, cons
                                        (double*)(io + L.k), (int32_t*)(io + L.pde), (int8_t*)(io + L.w),
                                        (uint8_t*)(io + L.e), counts + 8, p->scale, stream));
     ctx->launches += 2;
-    return run_batch(ctx, io, L, (int)m, (int)n, p, d_prices, d_status, stream, 0, 0, counts + 8);
+    return run_batch(ctx, io, L, (int)m, (int)n, p, d_prices, d_status, stream, 0, 0, counts + 8, false);
 }
 
 }  // extern "C"

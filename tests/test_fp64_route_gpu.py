@@ -146,3 +146,27 @@ def test_device_calls_choose_as_host_calls(built, n, x_dim, t_dim, share, dedup)
             assert np.array_equal(price.cpu().numpy(), want) and np.array_equal(status.cpu().numpy(), wst)
     finally:
         c.close()
+
+
+@pytest.mark.parametrize("n,x_dim,t_dim,density,fp64", [(40, 300, 100, 0.25, True), (40, 64, 40, math.inf, True),
+                                                        (40, 128, 600, 0.25, True), (40, 300, 600, 0.25, False),
+                                                        (40, 700, 40, 0.25, False), (40, 128, 40, math.inf, False)])
+def test_small_control_variates_step_in_fp64(built, n, x_dim, t_dim, density, fp64):
+    """Where the two solves' errors cancel better than pair arithmetic resolves (launches: FP64 on chip 2,
+    pair arithmetic 3, and the control variate)."""
+    import kwg
+    import portfolio
+
+    c = kwg.Context(0)
+    try:
+        o = portfolio.american_portfolio(n, seed=x_dim)
+        got = {}
+        for s in (kwg.SOLVER_AUTO, kwg.SOLVER_THOMAS):
+            rc, got[s], st = c.fd1d_bs_price(o, kwg.params(t_dim=t_dim, x_dim=x_dim, scale=50.0 if density < 1 else 5.0,
+                                                           density=density, solver=s))
+            assert rc == kwg.KWG_OK and (st == 0).all()
+            if s == kwg.SOLVER_AUTO:
+                assert c.launch_count() == (3 if fp64 else 4)
+        assert np.max(np.abs(got[0] - got[1]) / np.maximum(1e-10 * np.abs(got[1]), 1e-13 * o["k"])) <= 1.0
+    finally:
+        c.close()
