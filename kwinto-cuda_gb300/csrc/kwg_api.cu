@@ -258,17 +258,11 @@ __global__ void selftest_waits(int32_t* __restrict__ out, uint32_t limit)
 kwg_ctx::Tuned choose(kwg_ctx* ctx, const kwg_fd1d_params* p, int m, int left, bool control_variate)
 {
     kwg_ctx::Tuned t;
-    auto it = ctx->tuned.find(tune_key(p->precision, p->x_dim, p->t_dim, m));
+    auto it = ctx->tuned.find(tune_key(p, p->x_dim, p->t_dim, m));
     const bool pcr_ok = kwg::fd1d_pcr64_nodes_per_lane(p->x_dim) > 0;
     const bool recorded = it != ctx->tuned.end();
-    if (recorded) {
-        t = it->second;
-        // recorded for theta = 1/2, which the key does not hold
-        if (p->precision == KWG_FP64 && t.solver == KWG_SOLVER_PCR && !pair64_ok(p) && !pcr_ok)
-            t.solver = KWG_SOLVER_THOMAS;
-    } else {
-        t.solver = pcr_ok && m < 8192 ? KWG_SOLVER_PCR : KWG_SOLVER_THOMAS;
-    }
+    if (recorded) t = it->second;
+    else t.solver = pcr_ok && m < 8192 ? KWG_SOLVER_PCR : KWG_SOLVER_THOMAS;
     if (p->precision == KWG_FP32) t.solver = KWG_SOLVER_PCR;
     else if (p->solver != KWG_SOLVER_AUTO) t.solver = p->solver;
     if (pair64_ok(p)) {
@@ -732,7 +726,7 @@ int kwg_autotune_ex(kwg_ctx* ctx, const kwg_fd1d_params* p, size_t m, kwg_tuning
     const std::vector<kwg_option> opts = tuning_batch(m);
     std::vector<double> prices(m);
     const bool pcr_ok = kwg::fd1d_pcr64_nodes_per_lane(p->x_dim) > 0;
-    const uint64_t key = tune_key(p->precision, p->x_dim, p->t_dim, (int)m);
+    const uint64_t key = tune_key(p, p->x_dim, p->t_dim, (int)m);
     ctx->tuned[key] = kwg_ctx::Tuned();
     ctx->tuned[key].solver = KWG_SOLVER_PCR;
     const kwg_ctx::Tuned best = tune(ctx, p, pcr_ok, pair64_ok(p), [&](const kwg_fd1d_params& q) {

@@ -155,14 +155,14 @@ inline bool pair64_ok(const kwg_fd1d_params* p)
     return p->precision == KWG_FP64 && p->theta == 0.5 && kwg::fd1d_fp32_nodes_per_lane(p->x_dim) > 0;
 }
 
-// Autotuner key: precision, grid and the batch size rounded up to a power of two.
-// Uneven batches use x_dim = t_dim = 0.
-inline uint64_t tune_key(int precision, int x_dim, int t_dim, long long m)
+// Autotuner key: precision, theta = 1/2 or not and the kind of grid, which choose the kernel, the
+// grid size and the batch size rounded up to a power of two.  Uneven batches use x_dim = t_dim = 0.
+inline uint64_t tune_key(const kwg_fd1d_params* p, int x_dim, int t_dim, long long m)
 {
     int mb = 0;
     while ((1ll << mb) < m && mb < 40) ++mb;
-    return ((uint64_t)precision << 60) | ((uint64_t)(x_dim & 0xfffff) << 40) | ((uint64_t)(t_dim & 0xfffff) << 20) |
-           (uint64_t)mb;
+    const uint64_t kind = (uint64_t)p->precision | (p->theta == 0.5 ? 2 : 0) | (std::isinf(p->density) ? 4 : 0);
+    return (kind << 60) | ((uint64_t)(x_dim & 0xfffff) << 40) | ((uint64_t)(t_dim & 0xfffff) << 20) | (uint64_t)mb;
 }
 
 // Solve-kernel milliseconds of one call (after a warm-up call), or -1 on error.

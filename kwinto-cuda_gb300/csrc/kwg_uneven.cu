@@ -328,7 +328,7 @@ extern "C" int kwg_fd1d_price_uneven(kwg_ctx* ctx, const kwg_option* opts, const
     // says so) Thomas.  PDEs left over by pair arithmetic bring the model in where that is recorded too.
     kwg_ctx::Tuned tn;
     {
-        const auto it = ctx->tuned.find(tune_key(q.precision, 0, 0, (long long)n));
+        const auto it = ctx->tuned.find(tune_key(&q, 0, 0, (long long)n));
         const bool recorded = it != ctx->tuned.end();
         if (recorded) tn = it->second;
         if (q.solver == KWG_SOLVER_AUTO && pair64_ok(&q) && !(recorded && tn.solver == KWG_SOLVER_THOMAS)) {
@@ -540,7 +540,7 @@ extern "C" int kwg_autotune_uneven(kwg_ctx* ctx, const kwg_option* opts, const i
     for (size_t i = 0; i < n; ++i) x_max = std::max(x_max, (int)x_dims[i]);
     std::vector<double> prices(n);
     const bool pcr_ok = kwg::fd1d_pcr64_nodes_per_lane(x_max) > 0;
-    const uint64_t key = tune_key(p->precision, 0, 0, (long long)n);
+    const uint64_t key = tune_key(p, 0, 0, (long long)n);
     ctx->tuned[key] = kwg_ctx::Tuned();
     ctx->tuned[key].solver = KWG_SOLVER_PCR;
     kwg_fd1d_params widest = *p;
