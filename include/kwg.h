@@ -206,7 +206,8 @@ typedef struct kwg_tuning {
     double thomas_ms[3];  /* streaming FP64 solver with 1, 2, 4 warps per block */
     double pcr_ms;        /* FP64 on-chip solver (KWG_SOLVER_PCR) */
     double fp32_ms[3];    /* FP32 solver with 1, 2, 4 warps per option (the launch may use
-                             another count: option_warps of kwg_fd1d_params) */
+                             another count: option_warps of kwg_fd1d_params; counts that come to
+                             the same launch are timed once) */
     double spread_ms;     /* streaming FP64 solver, 4 warps per block, one block per SM */
     double fp32_8w_ms;    /* FP32 solver with 8 warps per option (same caveat) */
 } kwg_tuning;

@@ -112,6 +112,14 @@ int fd1d_fp32_nodes_per_lane(int x_dim)
     return m <= 64 ? m : -1;
 }
 
+int fd1d_fp32_warps(int x_dim, int option_warps)
+{
+    const int m1 = fd1d_fp32_nodes_per_lane(x_dim);
+    if (m1 < 8) return 1;
+    const int w = option_warps > 4 ? 4 : option_warps;
+    return m1 == 64 && w < 2 ? 2 : w;
+}
+
 size_t fd1d_fp32_work_bytes(int m, int x_dim) { return (size_t)m * x_dim * sizeof(double); }
 
 int fd1d_fp32_launch(const PdeBatch& b, const AssetBatch& a, const Fd1dShape& sh, double* vout, int32_t* pde_status,
@@ -125,9 +133,7 @@ int fd1d_fp32_launch(const PdeBatch& b, const AssetBatch& a, const Fd1dShape& sh
     const int m1 = fd1d_fp32_nodes_per_lane(sh.x_dim);
     if (m1 < 0) return -1;
     const bool uni = sh.uniform && (sh.pde_x ? sh.full_lanes : sh.x_dim == 32 * m1);
-    int W = sh.option_warps > 0 ? (sh.option_warps > 4 ? 4 : sh.option_warps) : fp32_warps(m1, uni, b.m, sms);
-    if (m1 < 8) W = 1;
-    if (m1 == 64 && W < 2) W = 2;
+    const int W = fd1d_fp32_warps(sh.x_dim, sh.option_warps > 0 ? sh.option_warps : fp32_warps(m1, uni, b.m, sms));
     const int M = m1 / W;
     cudaMemsetAsync(counters, 0, 4 * sizeof(int), stream);
     if (ev) cudaEventRecord(ev->start, stream);

@@ -108,6 +108,8 @@ int fd1d_fp64_launch(const PdeBatch& b, const AssetBatch& a, const Fd1dShape& sh
 // with decoupled identity rows; W warps take M/W each); -1 if x_dim > 2048.  The work buffer
 // holds the final V of every PDE, [m][x_dim] doubles.
 int fd1d_fp32_nodes_per_lane(int x_dim);
+// The warps per PDE that a choice of `option_warps` (1, 2, 4, 8) comes to on x_dim nodes.
+int fd1d_fp32_warps(int x_dim, int option_warps);
 size_t fd1d_fp32_work_bytes(int m, int x_dim);
 int fd1d_fp32_launch(const PdeBatch& b, const AssetBatch& a, const Fd1dShape& sh, double* vout, int32_t* pde_status,
                      int* counters, double* prices, int32_t* status, int device, cudaStream_t stream,

@@ -729,7 +729,7 @@ int kwg_autotune_ex(kwg_ctx* ctx, const kwg_fd1d_params* p, size_t m, kwg_tuning
     const uint64_t key = tune_key(p, p->x_dim, p->t_dim, (int)m);
     ctx->tuned[key] = kwg_ctx::Tuned();
     ctx->tuned[key].solver = KWG_SOLVER_PCR;
-    const kwg_ctx::Tuned best = tune(ctx, p, pcr_ok, pair64_ok(p), [&](const kwg_fd1d_params& q) {
+    const kwg_ctx::Tuned best = tune(ctx, p, p->x_dim, pcr_ok, pair64_ok(p), [&](const kwg_fd1d_params& q) {
         return kwg_fd1d_price(ctx, opts.data(), m, &q, prices.data(), nullptr);
     }, out);
     ctx->tuned[key] = best;

@@ -2,6 +2,7 @@
 // translation units of libkwg.so (not part of the public interface).
 #pragma once
 
+#include <algorithm>
 #include <cmath>
 #include <cstdint>
 #include <map>
@@ -183,12 +184,13 @@ inline double time_solve(kwg_ctx* ctx, F&& call)
 // Times every candidate launch shape on fn(params) and returns the fastest: FP64 --
 // the streaming solver with 1, 2, 4 warps per block (as many blocks per SM as fit),
 // with one 4-warp block per SM (one warp per scheduler), and the warp-per-PDE solver
-// (when pcr_ok); FP32 -- 1, 2, 4 and 8 warps per option.  auto_on_chip: a call with AUTO and
+// (when pcr_ok); FP32 -- 1, 2, 4 and 8 warps per option, the distinct ones of them on x_dim nodes (0:
+// an uneven batch), whose times stand for the others.  auto_on_chip: a call with AUTO and
 // no record takes the on-chip FP64 solver although KWG_SOLVER_PCR is refused (grids of 1025
 // to 2048 nodes); it is then timed through AUTO, and reported as KWG_SOLVER_AUTO.  The
 // caller has set the shape's record to the on-chip solver, so that AUTO takes it.
 template <typename F>
-inline kwg_ctx::Tuned tune(kwg_ctx* ctx, const kwg_fd1d_params* p, bool pcr_ok, bool auto_on_chip, F&& fn,
+inline kwg_ctx::Tuned tune(kwg_ctx* ctx, const kwg_fd1d_params* p, int x_dim, bool pcr_ok, bool auto_on_chip, F&& fn,
                            kwg_tuning* out)
 {
     kwg_tuning r = {};
@@ -237,11 +239,18 @@ inline kwg_ctx::Tuned tune(kwg_ctx* ctx, const kwg_fd1d_params* p, bool pcr_ok, 
         }
     } else {
         const int ws[4] = {1, 2, 4, 8};
+        double* const ms[4] = {&r.fp32_ms[0], &r.fp32_ms[1], &r.fp32_ms[2], &r.fp32_8w_ms};
+        auto runs = [&](int w) { return x_dim > 0 ? kwg::fd1d_fp32_warps(x_dim, w) : std::min(w, 4); };
         for (int i = 0; i < 4; ++i) {
+            int same = 0;
+            while (runs(ws[same]) != runs(ws[i])) ++same;
+            if (same < i) {
+                *ms[i] = *ms[same];
+                continue;
+            }
             q.option_warps = ws[i];
-            double& ms = i < 3 ? r.fp32_ms[i] : r.fp32_8w_ms;
-            ms = time_solve(ctx, [&] { return fn(q); });
-            consider(ms, KWG_SOLVER_PCR, 1, ws[i], 0);
+            *ms[i] = time_solve(ctx, [&] { return fn(q); });
+            consider(*ms[i], KWG_SOLVER_PCR, 1, ws[i], 0);
         }
     }
     r.solver = best.solver == KWG_SOLVER_PCR && auto_on_chip && !pcr_ok ? KWG_SOLVER_AUTO : best.solver;

@@ -548,7 +548,7 @@ extern "C" int kwg_autotune_uneven(kwg_ctx* ctx, const kwg_option* opts, const i
     auto call = [&](const kwg_fd1d_params& q) {
         return kwg_fd1d_price_uneven(ctx, opts, x_dims, t_dims, n, &q, prices.data(), nullptr);
     };
-    kwg_ctx::Tuned best = tune(ctx, p, pcr_ok, pair64_ok(&widest), call, out);
+    kwg_ctx::Tuned best = tune(ctx, p, 0, pcr_ok, pair64_ok(&widest), call, out);
     if (p->precision == KWG_FP32) {
         // One number of warps for all buckets against each bucket's own by its size.  Whole calls
         // decide: the candidates' solves were timed one after the other, and buckets that run side

@@ -58,3 +58,18 @@ def test_an_uneven_record_binds_its_own_scheme(built):
     finally:
         tuned.close()
         fresh.close()
+
+
+@pytest.mark.parametrize("x_dim,same", [(100, [0, 1, 2, 3]), (256, [2, 3]), (1500, [0, 1]), (1500, [2, 3])])
+def test_fp32_choices_that_run_alike_share_one_time(built, x_dim, same):
+    """Up to 128 nodes one warp, at least two above 1024, never more than four."""
+    import kwg
+
+    c = kwg.Context(0)
+    try:
+        t = c.autotune_ex(kwg.params(t_dim=30, x_dim=x_dim, scale=5.0, density=math.inf, precision=kwg.FP32), 300)
+        ms = [*t.fp32_ms, t.fp32_8w_ms]
+        assert min(ms) > 0 and len({ms[i] for i in same}) == 1
+        assert ms[(1, 2, 4, 8).index(t.option_warps)] == min(ms) and t.option_warps != 8
+    finally:
+        c.close()
