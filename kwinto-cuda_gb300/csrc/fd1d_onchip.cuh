@@ -160,9 +160,9 @@ __device__ __forceinline__ void floor_to(float2 ph, float2 pl, float2& h, float2
     }
 }
 
-// 1 / d by Newton's method in its cubic form, r (1 + e + e^2) with e = 1 - d r, from the
-// hardware's 20-bit estimate: the error left is e^3 ~ 2^-60, then rounding.  Zero and
-// non-finite d give a non-finite result.
+// 1 / d by one step of Chebyshev's third-order iteration (Newton's with the next term of the series),
+// r (1 + e + e^2) with e = 1 - d r, from the hardware's 20-bit estimate: e^3 ~ 2^-60 is left, then
+// rounding: within an ulp for d from 2^-1000 to 2^1000.  Zero and non-finite d give a non-finite result.
 __device__ __forceinline__ double rcp(double d)
 {
     double r;

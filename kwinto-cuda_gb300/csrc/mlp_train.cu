@@ -55,13 +55,6 @@ __device__ __forceinline__ uint32_t act_offset(int row, int ch)
     return (uint32_t)(row >> 3) * kRow8 + (uint32_t)(ch >> 3) * kCore + (uint32_t)((row & 7) * 16 + (ch & 7) * 2);
 }
 
-__device__ __forceinline__ float dsilu_f(float z)
-{
-    // the reciprocal as in silu_f: no branch, corrected by its exact residual
-    const float d = 1.f + __expf(-z), r = rcp_approx(d), s = z < -87.f ? 0.f : fmaf(fmaf(-d, r, 1.f), r, r);
-    return s * (1.f + z * (1.f - s));
-}
-
 // Sums over the 32 lanes of 32 values: lane i returns the sum of v[i] (31 shuffles).
 __device__ __forceinline__ float lane_sums(float (&v)[32], int lane)
 {
