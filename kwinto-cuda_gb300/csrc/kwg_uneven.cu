@@ -123,26 +123,32 @@ int price_buckets(kwg_ctx* ctx, const kwg_option* opts, const int32_t* x_dims, c
     std::stable_sort(by_work, by_work + kBuckets, [&](int a, int b) { return part[a].work > part[b].work; });
     if (pair && n < 32768) std::reverse(by_work + 1, by_work + kBuckets);
 
-    // Buffers for all buckets before the first launch, at the size they have without duplicates:
-    // growing one later would wait for the solves in flight.  Batches beyond 2 GB of rows, and what
-    // does not fit, grow bucket by bucket to the size after dedup.
-    uint64_t rows = 0;
-    for (const Part& p : part) rows += p.nodes * sizeof(double);
-    for (int b = 0; b < kBuckets && rows <= 2000000000ull; ++b) {
-        const size_t nb = part[b].end - part[b].begin;
-        kwg_ctx::Bucket& bk = ctx->buckets[b];
-        if (nb == 0) continue;
-        const size_t io = uneven_layout(nb, nb, 0).total,
-                     work = pair ? kwg::fd1d_pair64_work_bytes((int)nb, (long long)part[b].nodes)
-                                 : (size_t)part[b].nodes * sizeof(double);
-        if (ensure_host(ctx, &bk.h_io, &bk.h_io_bytes, io) ||
-            ensure_device(ctx, &bk.d_io, &bk.io_bytes, align_up(io, 256) + 4 * sizeof(int)) ||
-            ensure_device(ctx, &bk.d_work, &bk.work_bytes, work)) {
-            ctx->err.clear();
-            cudaGetLastError();
-            break;
+    // Buffers of the later buckets before the first launch, as growing one later would wait for the solves in
+    // flight: at the size they have with the first bucket's share of distinct PDEs and a tenth.  Batches
+    // beyond 2 GB of rows, what does not fit, and buckets with a larger share grow one by one.
+    auto reserve = [&](int first, double distinct) {
+        size_t m[kBuckets], nodes[kBuckets], rows = 0;
+        for (int b = 0; b < kBuckets; ++b) {
+            const size_t nb = part[b].end - part[b].begin;
+            m[b] = std::min(nb, (size_t)(1.1 * distinct * (double)nb) + 32);
+            nodes[b] = std::min((size_t)part[b].nodes, (size_t)(1.1 * distinct * (double)part[b].nodes) + 32 * ((size_t)64 << b));
+            rows += nodes[b] * sizeof(double);
         }
-    }
+        for (int b = 0; b < kBuckets && rows <= 2000000000ull; ++b) {
+            const size_t nb = part[b].end - part[b].begin;
+            kwg_ctx::Bucket& bk = ctx->buckets[b];
+            if (nb == 0 || b == first) continue;
+            const size_t io = uneven_layout(m[b], nb, 0).total,
+                         work = pair ? kwg::fd1d_pair64_work_bytes((int)m[b], (long long)nodes[b]) : nodes[b] * sizeof(double);
+            if (ensure_host(ctx, &bk.h_io, &bk.h_io_bytes, io) ||
+                ensure_device(ctx, &bk.d_io, &bk.io_bytes, align_up(io, 256) + 4 * sizeof(int)) ||
+                ensure_device(ctx, &bk.d_work, &bk.work_bytes, work)) {
+                ctx->err.clear();
+                cudaGetLastError();
+                break;
+            }
+        }
+    };
 
     std::vector<int32_t> asset2pde, pde_slot;
     std::vector<uint32_t> pde2asset;
@@ -153,6 +159,7 @@ int price_buckets(kwg_ctx* ctx, const kwg_option* opts, const int32_t* x_dims, c
         const uint32_t* const idx = order.data() + p.begin;
         const size_t nb = p.end - p.begin;
         const size_t m = kwg::dedup_host(opts, nb, x_dims, t_dims, asset2pde, pde2asset, idx);
+        if (bi == by_work[0]) reserve(bi, (double)m / (double)nb);
         // node-steps descending (x_dim <= 2048 here, so node-steps < 2^43), ties by PDE number
         kv.resize(m);
         int x_max = 0, x_min = INT32_MAX;
