@@ -84,9 +84,10 @@ struct Fp64Batch {
         c.sum += 0.16 * n * (double)d.n + (uniform ? 1. : 1.12) * kStep[k] * (double)d.steps;
         c.longest = std::max(c.longest, d.longest * (1200. + 8.8 * n) * (d.n > 304 ? 1.25 : 1.));
     }
-    double pair_ns() const
+    // pair arithmetic; `rest`: of the PDEs it leaves over
+    Cost pair(Cost& rest) const
     {
-        Cost c, rest;
+        Cost c;
         long long n_plain = 0, n_all = 0;
         for (int k = 0; k < kSizes; ++k) {
             n_plain += plain[k].n;
@@ -102,16 +103,31 @@ struct Fp64Batch {
             rest.sum += setup_ns(k) * (double)left[k].n;
             add_fp64(rest, left[k], k);
         }
-        return c.ns() + rest.ns();
+        return c;
     }
-    double on_chip_ns() const
+    Cost on_chip() const
     {
         Cost c;
         for (int k = 0; k < kSizes; ++k) {
             add_fp64(c, plain[k], k);
             add_fp64(c, left[k], k);
         }
-        return c.ns();
+        return c;
+    }
+    double pair_ns() const
+    {
+        Cost rest;
+        const Cost c = pair(rest);
+        return c.ns() + rest.ns();
+    }
+    double on_chip_ns() const { return on_chip().ns(); }
+    // One of several batches that run side by side: others fill the time of a few PDEs' chains, so
+    // that work counts, not latency.
+    bool fp64_beside_others() const
+    {
+        Cost rest;
+        const Cost c = pair(rest);
+        return any_left() && on_chip().sum < c.sum + rest.sum;
     }
     Cost stream() const
     {

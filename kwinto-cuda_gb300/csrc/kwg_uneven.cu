@@ -233,7 +233,7 @@ int price_buckets(kwg_ctx* ctx, const kwg_option* opts, const int32_t* x_dims, c
         const cudaStream_t st = ctx->profiling ? ctx->stream : bk.stream;
         KWG_CUDA(ctx, cudaMemcpyAsync(io, h, L.in_bytes, cudaMemcpyHostToDevice, st));
         const kwg::SolveEvents* ev = ctx->next_events();
-        const bool fp64_steps = pair && costs.any_left() && costs.on_chip_ns() < costs.pair_ns();
+        const bool fp64_steps = pair && costs.fp64_beside_others();
         const int r =
             fp64_steps ? kwg::fd1d_pcr64_half_launch(b, a, sh, v, d_pde_status, d_counters, d_prices, d_status,
                                                      ctx->device, st, ev)

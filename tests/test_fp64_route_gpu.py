@@ -170,3 +170,23 @@ def test_small_control_variates_step_in_fp64(built, n, x_dim, t_dim, density, fp
         assert np.max(np.abs(got[0] - got[1]) / np.maximum(1e-10 * np.abs(got[1]), 1e-13 * o["k"])) <= 1.0
     finally:
         c.close()
+
+
+def test_a_bucket_with_few_left_over_keeps_pair_arithmetic(built):
+    """Buckets run side by side, so one PDE left over does not send a bucket of a thousand to FP64 stepping, as it would
+    send a batch of its own (launches of an on-chip bucket: pair arithmetic 3, FP64 2)."""
+    import kwg
+
+    c = kwg.Context(0)
+    try:
+        o = drifting(1000, 0.0)
+        o["z"][7], o["r"][7], o["q"][7], o["t"][7] = 0.03, 0.08, 0.0, 1.5
+        x, t = np.full(1000, 200, np.int32), np.full(1000, 60, np.int32)
+        prm = kwg.params(scale=5.0, density=math.inf)
+        rc, p, st = c.fd1d_price_uneven(o, x, t, prm)
+        assert rc == kwg.KWG_OK and (st == 0).all() and c.launch_count() == 3
+        o["z"], o["r"], o["q"], o["t"] = 0.03, 0.08, 0.0, 1.5 + 1e-4 * np.arange(1000)
+        rc, p, st = c.fd1d_price_uneven(o, x, t, kwg.params(scale=5.0, density=math.inf, solver=kwg.SOLVER_PCR))
+        assert rc == kwg.KWG_OK and (st == 0).all() and c.launch_count() == 2
+    finally:
+        c.close()
