@@ -18,6 +18,7 @@
 #pragma once
 
 #include <algorithm>
+#include <utility>
 
 #include "fd1d_kernels.h"
 
@@ -44,17 +45,20 @@ struct Fp64Batch {
         double ns() const { return std::max(sum, longest); }
     };
     static constexpr int kSizes = 6;
-    bool uniform;
+    bool uniform = false;
     Kind plain[kSizes], left[kSizes];
     bool ragged[kSizes] = {};  // a PDE that does not fill the lanes
     long long nodes = 0, node_steps = 0, most_nodes = 0, most_node_steps = 0;
 
+    Fp64Batch() = default;
     explicit Fp64Batch(bool uniform_grid) : uniform(uniform_grid) {}
+    // the size class of x nodes
+    static int size_of(int x) { return x <= 64 ? 0 : 26 - __builtin_clz((unsigned)x - 1u); }
 
     // `count` PDEs of x nodes (2048 at most) and s steps, `leaves` of them left over by pair arithmetic
     void add(long long count, int x, int s, long long leaves = 0)
     {
-        const int k = x <= 64 ? 0 : 26 - __builtin_clz((unsigned)x - 1u);
+        const int k = size_of(x);
         ragged[k] = ragged[k] || x != 64 << k;
         if (count > leaves) plain[k].add(count - leaves, s);
         if (leaves > 0) left[k].add(leaves, s);
@@ -63,6 +67,22 @@ struct Fp64Batch {
         node_steps += count * xs;
         most_nodes = std::max(most_nodes, (long long)x);
         most_node_steps = std::max(most_node_steps, xs);
+    }
+
+    void add(const Fp64Batch& o)
+    {
+        for (int k = 0; k < kSizes; ++k) {
+            for (auto [to, from] : {std::pair{&plain[k], &o.plain[k]}, std::pair{&left[k], &o.left[k]}}) {
+                to->n += from->n;
+                to->steps += from->steps;
+                to->longest = std::max(to->longest, from->longest);
+            }
+            ragged[k] = ragged[k] || o.ragged[k];
+        }
+        nodes += o.nodes;
+        node_steps += o.node_steps;
+        most_nodes = std::max(most_nodes, o.most_nodes);
+        most_node_steps = std::max(most_node_steps, o.most_node_steps);
     }
 
     bool any_left() const

@@ -72,10 +72,7 @@ UnevenLayout uneven_layout(size_t m, size_t n, size_t ntiles)
     return L;
 }
 
-bool leaves(const kwg_option& o, const kwg_fd1d_params& q)
-{
-    return kwg::pair64_leaves(o.t, o.z, o.r, o.q, o.w, q.scale);
-}
+constexpr int kBuckets = sizeof(kwg_ctx::buckets) / sizeof(kwg_ctx::Bucket);
 
 // Warp-per-PDE solvers.  Preparing a batch (dedup, sort by work, packing) takes the host ~85 ns per
 // option: 11 of the 52 ms of 131072 options in FP32 when the whole batch was prepared before
@@ -84,9 +81,9 @@ bool leaves(const kwg_option& o, const kwg_fd1d_params& q)
 // next one's start: 42.8 ms (FP64: 143.9 -> 129.9).  With profiling on all run on the context's stream, one after
 // the other.
 int price_buckets(kwg_ctx* ctx, const kwg_option* opts, const int32_t* x_dims, const int32_t* t_dims, size_t n,
-                  const kwg_fd1d_params& q, const kwg_ctx::Tuned& tn, bool pair, double* prices, int32_t* status)
+                  const kwg_fd1d_params& q, const kwg_ctx::Tuned& tn, bool pair, const kwg::Fp64Batch* costs,
+                  double* prices, int32_t* status)
 {
-    constexpr int kBuckets = sizeof(ctx->buckets) / sizeof(ctx->buckets[0]);
     auto mlane = [&](int x) {
         return q.precision == KWG_FP32 || pair ? kwg::fd1d_fp32_nodes_per_lane(x) : kwg::fd1d_pcr64_nodes_per_lane(x);
     };
@@ -164,10 +161,8 @@ int price_buckets(kwg_ctx* ctx, const kwg_option* opts, const int32_t* x_dims, c
         kv.resize(m);
         int x_max = 0, x_min = INT32_MAX;
         long long nodes = 0;
-        kwg::Fp64Batch costs(std::isinf(q.density));
         for (size_t i = 0; i < m; ++i) {
             const int x = x_dims[pde2asset[i]];
-            if (pair) costs.add(1, x, t_dims[pde2asset[i]] - 1, leaves(opts[pde2asset[i]], q));
             kv[i] = {((1ull << 50) - 1) - (uint64_t)x * (uint64_t)(t_dims[pde2asset[i]] - 1), (uint32_t)i};
             x_max = std::max(x_max, x);
             x_min = std::min(x_min, x);
@@ -233,7 +228,7 @@ int price_buckets(kwg_ctx* ctx, const kwg_option* opts, const int32_t* x_dims, c
         const cudaStream_t st = ctx->profiling ? ctx->stream : bk.stream;
         KWG_CUDA(ctx, cudaMemcpyAsync(io, h, L.in_bytes, cudaMemcpyHostToDevice, st));
         const kwg::SolveEvents* ev = ctx->next_events();
-        const bool fp64_steps = pair && costs.fp64_beside_others();
+        const bool fp64_steps = pair && costs[bi].fp64_beside_others();
         const int r =
             fp64_steps ? kwg::fd1d_pcr64_half_launch(b, a, sh, v, d_pde_status, d_counters, d_prices, d_status,
                                                      ctx->device, st, ev)
@@ -334,14 +329,22 @@ extern "C" int kwg_fd1d_price_uneven(kwg_ctx* ctx, const kwg_option* opts, const
     // bucket's size, or (theta != 1/2, more than 2048 nodes, and where the cost model of fp64_route.h
     // says so) Thomas.  PDEs left over by pair arithmetic bring the model in where that is recorded too.
     kwg_ctx::Tuned tn;
+    kwg::Fp64Batch costs[kBuckets];
+    for (kwg::Fp64Batch& c : costs) c.uniform = std::isinf(q.density);
     {
         const auto it = ctx->tuned.find(tune_key(&q, 0, 0, (long long)n));
         const bool recorded = it != ctx->tuned.end();
         if (recorded) tn = it->second;
-        if (q.solver == KWG_SOLVER_AUTO && pair64_ok(&q) && !(recorded && tn.solver == KWG_SOLVER_THOMAS)) {
-            // every option a PDE of its own
+        const bool may_pair = pair64_ok(&q) && q.solver != KWG_SOLVER_THOMAS &&
+                              !(q.solver == KWG_SOLVER_AUTO && recorded && tn.solver == KWG_SOLVER_THOMAS);
+        if (may_pair)  // every option a PDE of its own
+            for (size_t i = 0; i < n; ++i)
+                costs[kwg::Fp64Batch::size_of(x_dims[i])].add(
+                    1, x_dims[i], t_dims[i] - 1,
+                    kwg::pair64_leaves(opts[i].t, opts[i].z, opts[i].r, opts[i].q, opts[i].w, q.scale));
+        if (may_pair && q.solver == KWG_SOLVER_AUTO) {
             kwg::Fp64Batch b(std::isinf(q.density));
-            for (size_t i = 0; i < n; ++i) b.add(1, x_dims[i], t_dims[i] - 1, leaves(opts[i], q));
+            for (const kwg::Fp64Batch& c : costs) b.add(c);
             tn.solver = KWG_SOLVER_PCR;
             if ((!recorded || b.any_left()) && b.best() == kwg::Fp64Route::kStream) {
                 tn.solver = KWG_SOLVER_THOMAS;
@@ -369,7 +372,7 @@ extern "C" int kwg_fd1d_price_uneven(kwg_ctx* ctx, const kwg_option* opts, const
             own.resize(n);
             status = own.data();
         }
-        const int rc = price_buckets(ctx, opts, x_dims, t_dims, n, q, tn, pair, prices, status);
+        const int rc = price_buckets(ctx, opts, x_dims, t_dims, n, q, tn, pair, costs, prices, status);
         return rc == KWG_OK && p->strict ? check_strict(ctx, status, n) : rc;
     }
 
