@@ -68,9 +68,9 @@ def node_steps(n, x_dim=None, t_dim=None):
 FP64_FLOPS_PER_NODE_STEP = 6  # 3 FMA per node-step at theta = 1/2
 # The on-chip kernel in pair arithmetic: FP32 operations (an add, a multiply or an FMA each) per
 # node and step, counted in csrc/fd1d_onchip.cuh: two tridiagonal solves of 5, the first
-# residual 6, W = V + u 7, its differences 8, the residual in pairs 30, the update 12, the
+# residual 6, W = V + u 7, its differences 11, the residual in pairs 30, the update 12, the
 # floor 3.  It reads 34 bytes and writes 8 N per PDE.
-PAIR_OPS_PER_NODE_STEP = 76
+PAIR_OPS_PER_NODE_STEP = 79
 FP32_LANES_PER_SM = 128
 ALGO_BYTES_PER_NODE_STEP = 32  # FP64 streaming scheme: V read + write, sweep value write + read
 

@@ -75,11 +75,11 @@ namespace {
 // 1024-node grids with tables per node and on 2048-node uniform ones, four on 2048-node grids
 // with tables per node; twice as many while every warp still has a scheduler to itself, and
 // from 1024 nodes (512 with tables per node) while they fit 12 to an SM.  Measured, ms with
-// 1/2/4 warps: 256 steps, uniform grids of 512 nodes, 150 PDEs 0.141/0.115/0.104, 300 of them
-// 0.141/0.115/0.130, 600 of them 0.145/0.149/0.196; of 1024 nodes, 300 of them 0.242/0.186/0.166, 600 of
-// them 0.258/0.245/0.270, 900 of them 0.344/0.331/0.393, 1200 of them 0.370/0.422/0.487; 512 nodes at
-// density 0.25, 600 of them 0.206/0.190/0.299; 512 steps, 8192 PDEs of 1024 nodes, density 0.25,
-// 6.81/5.71/6.77, uniform 3.86/4.42/5.8; 4096 PDEs of 2048 nodes -/8.48/6.58, uniform -/4.17/5.48.
+// 1/2/4 warps: 256 steps, uniform grids of 512 nodes, 150 PDEs 0.130/0.114/0.104, 300 of them
+// 0.130/0.116/0.129, 600 of them 0.135/0.149/0.194; of 1024 nodes, 300 of them 0.237/0.170/0.163, 900 of them
+// 0.344/0.311/0.395, 1200 of them 0.364/0.436/0.528; 512 nodes at density 0.25, 600 of them 0.206/0.192/0.296; 511
+// steps, 8192 PDEs of 1024 nodes, density 0.25, 5.86/5.25/6.59, uniform 3.77/4.41/5.82; 4096 PDEs of 2048 nodes
+// -/6.22/5.87, uniform -/4.17/5.37.
 int fp32_warps(int m1, bool uni, int m, int sms)
 {
     int w = m1 == 64 ? (uni ? 2 : 4) : m1 == 32 && !uni ? 2 : 1;

@@ -185,24 +185,16 @@ __device__ __forceinline__ Split split(double v)
 // A variant's share of the registers: the warps per SM that must fit, phase edges, and how
 // many of the factor tables stay in registers for the whole PDE (the spikes; also 1/d and u;
 // also l -- shared memory otherwise returns them every step, 40 of 56 bytes per slot and lane in
-// FP32 stepping, where it was the busiest unit, 71 %).  Best of 1 to 5 settings each, ms before
-// the tables moved -> now (8192 PDEs of 512 and 1024 nodes, 16384 of 256 and 128, 4096 of 2048;
-// 512 steps, FP32 at 2048 nodes 1024):
-//                          FP32 stepping       pair arithmetic (255 steps at 1024 and 2048 nodes)
-//   M = 32 uniform         4.57 -> 3.78        6.79 -> 5.61   (12 warps at 168 registers, 8 at 236)
-//   M = 16 uniform, W = 1  2.41 -> 1.95        5.84 -> 5.54
-//   M = 16 uniform, W = 4                      6.65 -> 6.15
-//   M = 16, W = 1          2.94 -> 2.51        6.57 -> 6.41
-//   M = 16, W = 2          7.33 -> 5.71        7.60 -> 7.47
-//   M = 16, W = 4          18.3 -> 12.5        8.74 -> 7.96
-//   M = 8 uniform          2.43 -> 1.94        6.16 -> 5.78
-//   M = 8                  2.89 -> 2.26        6.49 -> 6.12
-//   M = 4 uniform          1.54 -> 1.12        3.60 -> 3.46
-//   M = 4                  1.33 -> 1.32        3.66 -> 3.51
+// FP32 stepping, where it was the busiest unit, 71 %).  Best of 1 to 40 settings each; the tables in registers
+// took 2 to 30 % off.  Kernel ms now (511 steps; pair arithmetic at 1024 and 2048 nodes 255), FP32 | pair:
+//   M = 32 uniform   8192 x 1024   3.77 | 5.85       M = 8 uniform  16384 x 256   1.94 | 5.85
+//   M = 16 uniform   8192 x 512    1.95 | 5.78       M = 8          16384 x 256   2.29 | 6.41
+//   M = 16           8192 x 512    2.38 | 6.59       M = 4 uniform  16384 x 128   1.12 | 3.54
+//   M = 16, W = 2    8192 x 1024   5.25 | 7.06       M = 4          16384 x 128   1.32 | 3.78
+//   M = 16, W = 4    4096 x 2048   5.87 | 7.94       M = 2 uniform  16384 x 64    0.75 | 2.22
 // Variants that only small batches take (more warps per PDE than a large batch would) need
-// registers, not resident warps: 26 PDEs of 567 nodes (500 steps) 0.652 -> 0.520 pair, 0.267 -> 0.256
-// FP32; 150 of 1024 uniform nodes (256 steps) 0.318 -> 0.267 pair; 300 of 2048 uniform nodes 0.267 -> 0.239
-// FP32.
+// registers, not resident warps: 150 PDEs of 1024 uniform nodes (256 steps) 0.318 -> 0.267 pair; 300 of 2048
+// uniform nodes 0.267 -> 0.239 FP32.
 struct Budget {
     int warps, tables;
     bool edges;
@@ -253,8 +245,8 @@ struct Lay {
     static constexpr int oEdge = oX, oVec = oEdge + 4 * W, oInv = oVec + 2 * (nv + 1), oSp = oInv + nv * n,
                          oInt = oSp + 2 * W;
     static constexpr int kEx = W == 1 ? 0 : 4 * W + 2 * (nv + 1) + nv * n + 2 * W + W + 2;
-    // setup exchange in doubles, over the payoff table's space is not possible (in use):
-    // [3][W] boundary couplings, [2][W] neighbour spikes
+    // setup exchange in doubles (the payoff table's space is in use): [2][W] spike ends of each warp's
+    // last node, [5][W] responses at the warp boundaries
     static constexpr int oDbl = (oX + kEx + 1) / 2 * 2;
     static constexpr int kDbl = W == 1 ? 0 : 2 * 7 * W;
     static constexpr size_t kBytes = (size_t)(oDbl + kDbl) * sizeof(float);

@@ -4,14 +4,14 @@
 //
 // Why.  A warp-wide FP64 instruction holds its scheduler's FP64 unit for 64 cycles, a
 // warp-wide FP32 one for 1.  The streaming kernel's three FP64 multiply-adds per node-step
-// (fd1d_fp64.cu) therefore cost 6 scheduler cycles per node; the ~76 FP32 operations here
-// cost 2.4, and their latency is 4 cycles instead of 64.
+// (fd1d_fp64.cu) therefore cost 6 scheduler cycles per node; the ~79 FP32 operations here
+// cost 2.5, and their latency is 4 cycles instead of 64.
 //
 // Bound by the FP32 pipe (75 % busy at 1024 uniform nodes) and, for few PDEs, by the
 // latency of the two separator solves per step.  Measured against the FP64 solvers that took
-// these shapes before (whole calls): 32768 PDEs, 1024 x 1024 uniform, 192 -> 84 ms; 8192 PDEs,
-// 1024 x 1024, density 0.25, 186 -> 26 ms; 777 PDEs, 1000 x 731, 12.4 -> 2.4 ms; 600 PDEs,
-// 512 x 512, 2.50 -> 0.77 ms; 12 PDEs 2.35 -> 0.44 ms; 131072 uneven PDEs 340 -> 129 ms.
+// these shapes before (whole calls): 32768 PDEs, 1024 x 1024 uniform, 192 -> 87 ms; 8192 PDEs,
+// 1024 x 1024, density 0.25, 186 -> 27 ms; 777 PDEs, 1000 x 731, 12.4 -> 2.5 ms; 600 PDEs,
+// 512 x 512, 2.50 -> 0.78 ms; 12 PDEs 2.35 -> 0.45 ms; 131072 uneven PDEs 340 -> 133 ms.
 //
 // Numerics.  The reference step B V' = E V (src/Math/kwFd1d.cpp:61-132) is taken in
 // increments.  With A' = theta dt A and u = theta (V' - V) it reads
@@ -27,15 +27,16 @@
 //      (~49 significant bits, renormalised every step).
 // An FP32 solve has a relative error of ~1e-7, so u0 + e has one of ~1e-14 V.  Rounding a
 // tridiagonal row in FP64 perturbs V by ~1e-15 per step, always the same way; the
-// difference form has no such drift.  On the 1024 x 1024 uniform grid the largest error
-// against the scheme in exact arithmetic is 3e-13 relative where the FP64 sweeps have
-// 2e-12 (CPU emulation over random options, |x| < 0.75).
+// difference form has no such drift.  Against stepping in 64-bit increments (48 to 2048 nodes, 40 to 2048 time levels,
+// uniform and density 0.25, 64 to 32768 options): 3e-15 to 8e-13 where the FP64 solvers have 3e-15 to 6e-12, and
+// nowhere more than they (1.05 times at 3.5e-15 at most).
 //
 // What it does not take: theta != 1/2, more than 2048 nodes, and -- PDE by PDE, found in
 // the setup or at the end -- values beyond FP32's range, and grids that a drift crosses
 // (|r - q - z^2/2| T above kMaxDrift half-widths), where the one-sided boundary rows of the
 // scheme amplify whatever stands at the boundary by orders of magnitude.  Those PDEs go
-// to a list that the FP64 kernel of fd1d_pcr64.cu works off in a launch of its own.
+// to a list that the FP64 kernel of fd1d_pcr64.cu works off in a launch of its own; a batch with many of
+// them is not given to this solver (fp64_route.h).
 #include "fd1d_onchip.cuh"
 
 namespace kwg {
@@ -48,10 +49,10 @@ namespace {
 // four beyond.  Fewer PDEs: twice the warps while every warp still has a scheduler to
 // itself, from 1024 nodes while they fit 12 to an SM, up to four (at eight, or below two nodes
 // per lane, the exchange costs more than the shorter chains save).  Measured, ms with 1/2/4
-// warps (256 steps): density 0.25, 150 PDEs of 512 nodes 0.355/0.271/0.228, 300 of them
-// 0.356/0.278/0.293, 450 of them 0.359/0.383/0.377; uniform, 300 of 1024 nodes 0.623/0.424/0.409, 450 of
-// them 0.629/0.568/0.533, 600 of them 0.648/0.582/0.672, 900 of them 0.936/0.793/0.958, 1200 of them
-// 0.963/1.015/1.287; 8192 of 1024 nodes, density 0.25 (512 steps) -/15.0/17.1.
+// warps (256 steps): density 0.25, 150 PDEs of 512 nodes 0.359/0.277/0.226, 300 of them
+// 0.361/0.281/0.295, 450 of them 0.361/0.392/0.383; uniform, 300 of 1024 nodes 0.645/0.418/0.393, 450 of
+// them 0.655/0.578/0.524, 600 of them 0.672/0.596/0.684, 900 of them 0.967/0.809/1.000, 1200 of them
+// 1.008/1.030/1.270; 8192 of 1024 nodes, density 0.25 (511 steps) -/13.7/16.1.
 int pair64_warps(int m1, bool uni, int m, int sms)
 {
     int w = m1 == 64 ? 4 : m1 == 32 && !uni ? 2 : 1;

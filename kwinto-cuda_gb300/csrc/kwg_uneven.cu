@@ -113,8 +113,9 @@ int price_buckets(kwg_ctx* ctx, const kwg_option* opts, const int32_t* x_dims, c
     for (size_t i = 0; i < n; ++i) order[part[id[i]].at++] = (uint32_t)i;
     // The heaviest bucket first.  The others by work as well, but in pair arithmetic upwards: a
     // bucket's rescue launch (fd1d_pair64.cu), one PDE's FP64 latency however short its list, then runs
-    // beside the next bucket (4000 options 6.8 -> 5.4 ms; in FP32, which has none, 1.86 -> 1.97).  In
-    // large batches the heavy buckets' own tails weigh more (131072 options 129.9 -> 132.1).
+    // beside the next bucket (in FP32, which has none, 1.86 -> 1.97 ms for 4000 options).  In large batches the
+    // heavy buckets' own tails weigh as much: downwards / upwards 8000 options 15.2 / 12.3 ms, 16000 22.8 / 18.9, 32000
+    // 34.0 / 33.5, 48000 49.7 / 51.7, 131072 132.9 / 132.9.
     int by_work[kBuckets];
     std::iota(by_work, by_work + kBuckets, 0);
     std::stable_sort(by_work, by_work + kBuckets, [&](int a, int b) { return part[a].work > part[b].work; });
