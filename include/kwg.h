@@ -78,8 +78,13 @@ typedef struct kwg_fd1d_params {
                           thread per PDE; _PCR: the on-chip solver, one to four warps per
                           PDE, x_dim <= 1024.  AUTO takes the on-chip one at theta = 1/2 up
                           to x_dim 2048 (the streaming one where many PDEs of few nodes or
-                          few steps run faster there) unless the autotuner recorded another
-                          choice */
+                          few steps run faster there, and FP64 stepping where many PDEs are
+                          not for pair arithmetic, or for an FD1D-BS on a small grid) unless
+                          the autotuner recorded another choice.  AUTO's choice and the
+                          warps per PDE of the on-chip solvers follow the batch, so a price
+                          depends on it within its error (FP64 in the last digits, FP32 by a
+                          few 1e-8 of the strike); _THOMAS, and in FP32 uniform calls an
+                          explicit option_warps, give prices that do not */
     int32_t strict;    /* blocking host calls (kwg_fd1d_price, kwg_fd1d_bs_price,
                           kwg_fd1d_price_uneven): 1 returns an error for the first
                           bad option, like the reference

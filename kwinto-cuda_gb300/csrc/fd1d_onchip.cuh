@@ -97,7 +97,7 @@ __device__ __forceinline__ PP2 pair_diff(const PP2& a, const PP2& b)
 // 2^-24 of the values the loss is that of pair_diff).  The low parts of neighbouring values do not
 // cancel as the values do: as they come, a difference's is up to 2^-24 of the values, and a step's
 // residual rounds it times alpha.  2 % of a call; errors against 64-bit stepping before -> after, FD1D-BS at density
-// 0.25: 1024 x 1024 1.9e-13 -> 1.4e-14, 1024 x 40 8.4e-13 -> 1.2e-14, 512 x 40 3.4e-13 -> 1.1e-14.
+// 0.25: 1024 x 1024 1.9e-13 -> 1.0e-14, 1024 x 40 8.4e-13 -> 1.2e-14, 512 x 40 3.4e-13 -> 1.1e-14.
 __device__ __forceinline__ PP2 pair_diff_norm(const PP2& a, const PP2& b)
 {
     const PP2 d = pair_diff(a, b);
