@@ -306,14 +306,22 @@ int run_batch(kwg_ctx* ctx, char* io, const IoLayout& L, int m, int n, const kwg
     a.n = n;
     kwg::Fd1dShape sh = make_shape(p);
     sh.twin_tiles = twin_tiles;
-    const kwg_ctx::Tuned tn = choose(ctx, p, m, left, control_variate);
+    kwg_ctx::Tuned tn = choose(ctx, p, m, left, control_variate);
+    const size_t stream_bytes = kwg::fd1d_fp64_work_bytes(m_pad, sh.x_dim);
+    if (tn.solver == KWG_SOLVER_THOMAS && p->solver == KWG_SOLVER_AUTO && pair64_ok(p) &&
+        ensure_device(ctx, &ctx->d_work, &ctx->work_bytes, stream_bytes)) {
+        // no room for the streaming solver's 72 bytes per node: on chip it is a ninth
+        ctx->err.clear();
+        cudaGetLastError();
+        tn.solver = KWG_SOLVER_PCR;
+    }
     const int solver = tn.solver;
     sh.block_warps = tn.block_warps;
     sh.option_warps = tn.option_warps;
     sh.sm_blocks = tn.sm_blocks;
     if (solver == KWG_SOLVER_PCR && pair64_ok(p)) {
         const long long nodes = (long long)m * sh.x_dim;
-        const size_t bytes = kwg::fd1d_pair64_work_bytes(m, nodes), stream_bytes = kwg::fd1d_fp64_work_bytes(m_pad, sh.x_dim);
+        const size_t bytes = kwg::fd1d_pair64_work_bytes(m, nodes);
         if (d_left) {
             kwg::Fp64Route other;
             const long long from =
@@ -324,7 +332,7 @@ int run_batch(kwg_ctx* ctx, char* io, const IoLayout& L, int m, int n, const kwg
                 sh.left_streams = other == kwg::Fp64Route::kStream;
             }
         }
-        // a device without room for the streaming solver's work arrays keeps to pair arithmetic
+        // without room for the streaming solver's work arrays: pair arithmetic, whatever the number
         if (sh.left_streams && ensure_device(ctx, &ctx->d_work, &ctx->work_bytes, std::max(bytes, stream_bytes))) {
             ctx->err.clear();
             cudaGetLastError();
@@ -364,8 +372,7 @@ int run_batch(kwg_ctx* ctx, char* io, const IoLayout& L, int m, int n, const kwg
         if (n_launch < 0) return set_err(ctx, KWG_ERR_INVALID, "kwg: FP32 stepping supports x_dim <= 2048");
         ctx->launches += n_launch;
     } else {
-        const size_t wbytes = kwg::fd1d_fp64_work_bytes(m_pad, sh.x_dim);
-        if (int rc = ensure_device(ctx, &ctx->d_work, &ctx->work_bytes, wbytes)) return rc;
+        if (int rc = ensure_device(ctx, &ctx->d_work, &ctx->work_bytes, stream_bytes)) return rc;
         const int blocks = kwg::fd1d_fp64_solve_blocks(m_pad / kwg::kTile, ctx->device, sh.block_warps, sh.sm_blocks);
         ctx->launches += kwg::fd1d_fp64_launch(b, a, sh, (double*)ctx->d_work, (int32_t*)(io + L.pde_status),
                                                ctx->d_counter, prices, status, blocks, stream, ctx->next_events());

@@ -367,15 +367,16 @@ extern "C" int kwg_fd1d_price_uneven(kwg_ctx* ctx, const kwg_option* opts, const
     const bool pcr = q.precision == KWG_FP32 || q.solver == KWG_SOLVER_PCR;
     const bool pair = q.solver == KWG_SOLVER_PCR && pair64_ok(&q);
     KWG_CUDA(ctx, cudaSetDevice(ctx->device));
-    if (pcr) {
+    auto on_chip = [&](bool in_pairs) {
         std::vector<int32_t> own;
         if (!status) {
             own.resize(n);
             status = own.data();
         }
-        const int rc = price_buckets(ctx, opts, x_dims, t_dims, n, q, tn, pair, costs, prices, status);
+        const int rc = price_buckets(ctx, opts, x_dims, t_dims, n, q, tn, in_pairs, costs, prices, status);
         return rc == KWG_OK && p->strict ? check_strict(ctx, status, n) : rc;
-    }
+    };
+    if (pcr) return on_chip(pair);
 
     // 1. dedup by (t, r, q, z, e, w, x_dim, t_dim)
     std::vector<int32_t> asset2pde;
@@ -430,8 +431,14 @@ extern "C" int kwg_fd1d_price_uneven(kwg_ctx* ctx, const kwg_option* opts, const
 
     // 3. pack inputs into pinned memory
     const UnevenLayout L = uneven_layout(ms, n, tiles.size());
-    if (int rc = ensure_host(ctx, &ctx->h_io, &ctx->h_io_bytes, L.total)) return rc;
     const size_t wbytes = kwg::fd1d_fp64_work_bytes_nl((int)ms, node_lanes);
+    if (p->solver == KWG_SOLVER_AUTO && pair64_ok(&q) && ensure_device(ctx, &ctx->d_work, &ctx->work_bytes, wbytes)) {
+        // no room for the streaming solver's 72 bytes per node: on chip it is a ninth
+        ctx->err.clear();
+        cudaGetLastError();
+        return on_chip(true);
+    }
+    if (int rc = ensure_host(ctx, &ctx->h_io, &ctx->h_io_bytes, L.total)) return rc;
     // the graph bakes in device addresses: grow buffers before deciding on replay
     if (int rc = ensure_device(ctx, &ctx->d_io, &ctx->io_bytes, L.total)) return rc;
     if (int rc = ensure_device(ctx, &ctx->d_work, &ctx->work_bytes, wbytes)) return rc;

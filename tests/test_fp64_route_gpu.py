@@ -190,3 +190,39 @@ def test_a_bucket_with_few_left_over_keeps_pair_arithmetic(built):
         assert rc == kwg.KWG_OK and (st == 0).all() and c.launch_count() == 2
     finally:
         c.close()
+
+
+@pytest.mark.parametrize("entry", ["host", "uneven", "device"])
+def test_without_room_for_streaming_it_stays_on_chip(built, entry):
+    """2.1 million PDEs of 2048 nodes: 310 GB for the streaming solver, which the cost model names, 34 GB on chip."""
+    import kwg
+    import torch
+
+    n, x_dim = 2100000, 2048
+    o = drifting(3000, 1.0)[np.arange(n) % 3000]
+    o["t"] += 1e-9 * np.arange(n)  # PDEs of their own
+    torch.cuda.empty_cache()
+    total = torch.cuda.mem_get_info()[1]
+    if not 40 * 10**9 < total < 305 * 10**9:
+        pytest.skip("sized for a device of 298 GB")
+    c = kwg.Context(0)
+    try:
+        kw = dict(scale=5.0, density=math.inf)
+        if entry == "uneven":
+            rc, p, st = c.fd1d_price_uneven(o, np.full(n, x_dim), np.full(n, 3), kwg.params(**kw))
+        elif entry == "host":
+            rc, p, st = c.fd1d_price(o, kwg.params(t_dim=3, x_dim=x_dim, **kw))
+        else:
+            d = torch.from_numpy(o.view(np.uint8).copy()).cuda()
+            price, status = torch.empty(n, dtype=torch.float64, device="cuda"), torch.empty(n, dtype=torch.int32, device="cuda")
+            rc = c.fd1d_price_device(d.data_ptr(), n, kwg.params(t_dim=3, x_dim=x_dim, **kw), price.data_ptr(),
+                                     status.data_ptr(), 0)
+            torch.cuda.synchronize()
+            p, st = price.cpu().numpy(), status.cpu().numpy()
+        assert rc == kwg.KWG_OK, c.last_error()
+        assert (st == 0).all()
+        pick = np.arange(0, n, 6007)
+        rc, want, _ = c.fd1d_price(o[pick], kwg.params(t_dim=3, x_dim=x_dim, solver=kwg.SOLVER_THOMAS, **kw))
+        assert rc == kwg.KWG_OK and np.max(np.abs(p[pick] - want) / np.maximum(1e-10 * np.abs(want), 1e-13 * o["k"][pick])) <= 1.0
+    finally:
+        c.close()
